@@ -481,8 +481,8 @@ rrhd_status rrhd_rad_source(const rrhd_emission *em, const double *W, const doub
  * (illum_utils.cpp:377-433), area-weighted face mean (plain mean for the last
  * cell).  The upwind order (the reference's sorted_graph, made offline by its
  * graph/ and make_trace/ tools) is built on the device at setup as levels of
- * cells whose upwind neighbours are all done; one level is one kernel launch,
- * all launches of a sweep are one CUDA graph. */
+ * cells whose upwind neighbours are all done; a sweep is one kernel, one CTA per
+ * direction, that walks the levels of its direction. */
 #define RRHD_RAD_FP64 0  /* sweep arithmetic and storage in double */
 #define RRHD_RAD_FP32 1  /* in float (input of the tensor-core scattering) */
 #define RRHD_RAD_MIXED 2 /* the sweep in double (geometry, records, face values, arithmetic)
@@ -498,18 +498,16 @@ rrhd_status rrhd_rad_source(const rrhd_emission *em, const double *W, const doub
 typedef struct {
   int32_t groups;         /* frequency groups G >= 1 (grey copies, rows cell * G + g)           */
   int32_t precision;      /* RRHD_RAD_FP64, RRHD_RAD_FP32 or RRHD_RAD_MIXED                     */
-  int32_t dirs_per_batch; /* directions swept together (face values [dirs_per_batch][F][groups] are
-                             kept for them): power of two <= 256; 0 = min(64, M)                */
+  int32_t dirs_per_batch; /* directions whose levels rrhd_rad_plan_info counts together: power of two <= 256;
+                             0 = min(64, M).  All directions are swept in one launch        */
   double boundary_value;  /* intensity entering through boundary faces (illum::BoundaryConditions
                              returns 0 for free, lock and outer boundaries, illum_utils.cpp:52-65) */
-  int32_t item_geometry;  /* 1: precompute at setup, per (cell, direction) item in sweep order, which
-                             faces are in- and out-faces, the in-face each interpolation node is
-                             traced to and the in-face distances H_f / -cos_f (16 bytes per item,
-                             cells x directions x 16 bytes of device memory); the sweep then reads
-                             that stream in order instead of each item's cell normals and heights.
-                             RRHD_RAD_FP32 and RRHD_RAD_MIXED only: the distances are stored as
-                             float (FP32: the same values; MIXED: the double distance rounded
-                             once, every choice made in double).  0: off                         */
+  int32_t item_geometry;  /* 0 or 1 (1: RRHD_RAD_FP32 and RRHD_RAD_MIXED only).  The sweep order keeps, per
+                             (cell, direction) item, which faces are in- and out-faces, the traced
+                             distances and the face weights (16 bytes and five values of the
+                             arithmetic's precision) whatever this says, where device memory holds
+                             them beside three arrays of the intensity's size; else it forms the
+                             distances and weights again from the cells' records               */
 } rrhd_rad_opts;
 /* Builds the sweep geometry and plan for ctx's mesh and the direction set (which
  * must outlive the context's radiation use).  RRHD_ERR_STATE if the mesh has a

@@ -50,45 +50,37 @@ struct rrhd_dirs;
 struct rrhd_scatter_tc;
 
 namespace rrhd {
-// Pointers a sweep reads and writes, kept in device memory so that one captured
-// graph of level launches serves every call.
-struct SweepIO {
-  const void *S;          // scattering integral
-  void *I;                // intensity
-  const int32_t *row_of;  // layout 0: context cell -> caller cell
-  int32_t layout;         // 0: rows (cell * G + g) x M in caller numbering; 1: [N][M][G], context numbering
-};
-
 // Radiation part of a context: the transport sweep and the coupled step.
 struct RadState {
   bool ready = false;
   const rrhd_dirs *dirs = nullptr;  // not owned
-  int M = 0, G = 1, DB = 64, shift = 6, nbatch = 0;
-  int prec = 0;  // RRHD_RAD_FP64 or RRHD_RAD_FP32: storage and arithmetic of the sweep
-  int RW = 0;    // stride (values) of the per-cell record
-  int GS = 0;    // stride (values) of one face-value slot: G rounded up to a 32-byte sector
+  int M = 0, G = 1;
+  int DB = 64;   // directions per batch of the level counts rrhd_rad_plan_info gives
+  int prec = 0;  // RRHD_RAD_FP64, RRHD_RAD_FP32 or RRHD_RAD_MIXED
+  int SW = 0;    // stride (values) of the per-cell source record
   double bc = 0.0;
-  int64_t last_cell = 0;  // context index of the caller's last cell (plain-mean quirk)
   void *d_w = nullptr;    // [M][3] directions in the sweep precision
-  // per-cell record (context numbering, RW values): outward normals n_j (12), heights
-  // H_j = 3 V / A_j (4), face-value slots of the faces (4 x int32) and neighbours (4 x int32,
-  // context numbering or -1), then the step's source record {k, betta/k, alpha Q_g/k}
-  void *d_rec = nullptr;
-  void *d_area = nullptr;  // [N][4] face areas
-  uint32_t *d_plan = nullptr;               // all batches: items (d << shift | cell) in level order
-  bool item_geometry = false;
-  uint4 *d_geo = nullptr;                   // item_geometry: per plan item {code, in-face distances}
-  std::vector<std::vector<int64_t>> lvl;    // per batch: level offsets into d_plan
+  void *d_rec = nullptr;  // [N] geometry records (normals, heights, neighbours); freed once d_dist stands
+  void *d_wt = nullptr;   // [N][4] face weights of the cell value
+  void *d_src = nullptr;  // [N][SW] source records {k, betta/k, alpha Q_g/k}
+  // the plan: per direction its N items in level order and the level offsets
+  uint4 *d_ord = nullptr;     // [M][N] {cell, code word, own and upwind slots (16 bits each)}
+  uint2 *d_ord_hi = nullptr;  // [M][N] upper halves of the slots, where 16 bits do not hold them
+  // geometry stream, where memory allows: [M][N][2] distances, [M][N][2] and [M][N] in-face weights
+  void *d_dist = nullptr, *d_wgt = nullptr, *d_wgt3 = nullptr;
+  int32_t *d_lvl = nullptr, *d_depth = nullptr;  // level offsets of all directions; levels per direction
+  int64_t *d_lvl_base = nullptr;                 // first entry of a direction in d_lvl
+  std::vector<int32_t> depth;
+  std::vector<int64_t> lvl_base;
   int64_t levels = 0, max_level = 0;
-  cudaGraphExec_t graph = nullptr;          // every level launch of one sweep
-  SweepIO *d_io = nullptr;
-  SweepIO h_io{};       // last pointers uploaded to d_io
-  bool io_valid = false;
+  int64_t nlow = 0, nhigh = 0;  // most slots a direction has in shared (slot 0: the boundary value) and global memory
+  void *d_slots = nullptr;      // [M][nhigh][G]
+  void *d_x = nullptr;          // S and I in the sweep's layout, [xdirs][N][G]
+  int xdirs = 0;
   // phase marks of the last coupled step: 0 start, 1 hydro done, 2 sweep done, 3 source
   // start and 4 source done (side stream), 5 join, 6 scattering done
   cudaEvent_t ev[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   cudaStream_t side = nullptr;  // the coupled step's source term runs here, beside the sweep
-  void *d_fv = nullptr;  // [DB][F][GS] face values, direction-major
   // coupled step (context numbering, [N][M][G])
   void *d_I = nullptr, *d_S = nullptr;
   double *d_G4 = nullptr;                                    // [N][4] radiation 4-force of the last step

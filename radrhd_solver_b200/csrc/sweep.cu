@@ -4,22 +4,36 @@
 // graph (sorted_graph: (cell, out-face) pairs) with precomputed node distances
 // (vec_x0), solvers/illum/src/mpi/multi_gpu/illum_multi_gpu_face_calc.cpp:91-190.
 // Here the order is built on the device once per mesh and direction set as
-// levels: level 0 holds the (cell, direction) pairs whose in-faces are all on
-// the boundary, level L+1 those whose last upwind neighbour is in level L.  All
-// pairs of a level are independent, so one level is one kernel launch with one
-// thread per pair, and a sweep is one CUDA graph of all level launches.  A batch
-// of DB directions is swept together, so the face values of one batch,
-// [DB][F][G] (direction-major), are the only scratch.
+// levels per direction: level 0 holds the cells whose in-faces are all on the
+// boundary, level L+1 those whose last upwind neighbour is in level L.  A sweep
+// is one kernel with one CTA per direction that walks its direction's levels,
+// one thread per cell and a CTA barrier between levels.
 //
-// Per pair the kernel classifies the four faces by the sign of n_j . w, traces
-// the three nodes of each out-face back to the in-face they came through (the
-// smallest t_h = lam_h H_h / -cos_h, H_h the height of the cell over face h and
-// lam_h the node's barycentric weight of the vertex opposite h: no vertex data
-// is needed), evaluates GetIllum per group with one set of exponentials shared by
-// all groups (the opacity k = alpha + betta does not depend on the group), and
-// folds the four face values into the cell value (ReCalcIllumOpt) in the same
-// thread, so face values are read once.  Compiled with --fmad=false: in double
-// precision every value is the oracle's operation for operation, exp aside.
+// One value per cell.  The reference gives every out-face the mean over its three
+// interpolation nodes of the intensity traced back from the node to the in-face it
+// came through: the in-face h with the smallest t_h = lam_h r_h (r_h = H_h / -cos_h,
+// H_h the height of the cell over face h, lam_h the node's barycentric weight of the
+// vertex opposite h: 2/3 at the node's own vertex, 1/6 at the others).  Let b1 be the
+// in-face with the smallest r / 6 and b2 the next.  A node of a vertex v other than b1's
+// sees t = r_b1 / 6 at b1 and at least min(2/3 r_v, r / 6) >= r_b1 / 6 elsewhere, so it is
+// traced to b1; only the node at b1's own vertex compares 2/3 r_b1 with r_b2 / 6.  A face j
+// holds the nodes of the three vertices other than j, and an out-face is not b1, so every
+// out-face holds the special node and two ordinary ones: all out-faces of a cell carry the
+// SAME value, (A + A + B) / 3.  The sweep therefore keeps one outgoing value per (cell,
+// direction), two attenuations at most, and forms the cell value (ReCalcIllumOpt, an
+// area-weighted face mean) in the same thread from the in-face values and that one value.
+//
+// A cell's outgoing value lives from its level to the last level of its downwind
+// neighbours; the plan gives it a slot for that time (a free list per direction), so a
+// direction needs about as many slots as its front is wide (9,400 on the 48^3 x 6 mesh)
+// and no face-value array exists.  Slots sit in shared memory when they fit, else in a
+// per-direction array that stays in L2.
+//
+// What a thread reads of its item comes in sweep order: a 16-byte record (cell, face
+// choice, slots) and the two distances; by cell index it reads the source record of the
+// step and the scattering integral.
+// Compiled with --fmad=false: in double precision every value is the oracle's operation
+// for operation, but for exp, exp(-4x) = exp(-x)^4 and the order of the face sums.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,28 +55,23 @@ using namespace rrhd;
 
 namespace {
 
-constexpr int kSweepThreads = 128;
-
-// Per-cell record (RW words): 0-11 outward normals n_j, 12-15 heights H_j, then the
-// face-value slots as int32 (4: 2 doubles or 4 floats; bit 31 set where the face has no
-// neighbour), then the source record {k, betta/k, alpha Q_g/k} of the step, and in the
-// last 16 bytes the neighbours (int32, -1 on the boundary), which only the plan reads.
-// RW makes a record a whole number of 128-byte lines (G = 4: 256 B in double, 128 B in
-// float); what one level item reads of its cell is 6 sectors (double) or 4 (float).
+// Per-cell geometry record (RW words), read by the plan and, in a sweep without the
+// distance stream, by every item: 0-11 outward normals n_j, 12-15 heights H_j, then the
+// neighbours (4 x int32, -1 on the boundary).
 template <class T>
 struct Rec {
-  static constexpr int IDS = 16;                       // word offset of the face-value slots
-  static constexpr int DYN = sizeof(T) == 8 ? 18 : 20;  // word offset of the source record
-  static constexpr int NBRW = 16 / (int)sizeof(T);      // words of the neighbours, at the record's end
-  static constexpr int LINE = 128 / (int)sizeof(T);     // words per 128-byte line
+  static constexpr int NBR = 16;                        // word offset of the neighbours
+  static constexpr int RW = 16 + 16 / (int)sizeof(T);  // words: 144 B in double, 80 B in float
 };
-constexpr int32_t kNoNeighbour = INT32_MIN;  // bit 31 of a face-value slot id
+// Per-cell source record (SW words): {k, betta/k, alpha Q_g/k}, one Q for all groups where
+// they share it (the coupled step).
+constexpr int kSrcQ = 2;
 
-// normals, heights and face-value slot ids (negative: a face without a neighbour)
 template <class T>
-__device__ __forceinline__ void load_rec(const T *r, T *g, int *fid) {
+__device__ __forceinline__ void load_vec(const T *r, T *g, int n) {
+  constexpr int V = 16 / (int)sizeof(T);
 #pragma unroll
-  for (int q = 0; q < 16; q += 16 / (int)sizeof(T)) {
+  for (int q = 0; q < n; q += V) {
     if constexpr (sizeof(T) == 8) {
       const double2 v = __ldg(reinterpret_cast<const double2 *>(r) + q / 2);
       g[q] = v.x;
@@ -75,36 +84,12 @@ __device__ __forceinline__ void load_rec(const T *r, T *g, int *fid) {
       g[q + 3] = v.w;
     }
   }
-  const int4 f = __ldg(reinterpret_cast<const int4 *>(r + Rec<T>::IDS));
-  fid[0] = f.x, fid[1] = f.y, fid[2] = f.z, fid[3] = f.w;
 }
-// normals and neighbours only (the plan kernels); RW: record words
 template <class T>
-__device__ __forceinline__ void load_normals(const T *r, int RW, T *g, int *nbr) {
-#pragma unroll
-  for (int q = 0; q < 12; q++) g[q] = __ldg(r + q);
-  const int4 n = __ldg(reinterpret_cast<const int4 *>(r + RW - Rec<T>::NBRW));
+__device__ __forceinline__ void load_nbr(const T *r, int *nbr) {
+  const int4 n = __ldg(reinterpret_cast<const int4 *>(r + Rec<T>::NBR));
   nbr[0] = n.x, nbr[1] = n.y, nbr[2] = n.z, nbr[3] = n.w;
 }
-__device__ __forceinline__ int64_t slot_of(int fid) { return (int64_t)(fid & 0x7fffffff); }
-
-// T: geometry and source records (directions, per-cell records, face areas); TV: face
-// values and the transport arithmetic.
-template <class T, class TV>
-struct SweepArgs {
-  const SweepIO *io;
-  const uint32_t *items;
-  int64_t n;  // items of this level
-  int shift, DB, d0, M, G, RW, GS, nbd;  // item = direction << shift | cell
-  int64_t NF;                            // face-value slots
-  const T *w;     // [M][3]
-  const T *rec;   // [N][RW]
-  const T *area;  // [N][4] face areas (cell values)
-  TV *fv;         // [DB][NF][GS] face values, direction-major (GS >= G, full 32-byte sectors)
-  const uint4 *geo;  // per item of the level (items[i] <-> geo[i]): its geometry, or null
-  TV bc;
-  int64_t last;
-};
 
 __device__ __forceinline__ double ex(double x) { return exp(x); }
 __device__ __forceinline__ float ex(float x) { return __expf(x); }
@@ -117,68 +102,84 @@ __device__ __forceinline__ void face_cos(const T *g, T wx, T wy, T wz, T *cosf) 
   for (int j = 0; j < 4; j++) cosf[j] = (g[3 * j] * wx + g[3 * j + 1] * wy) + g[3 * j + 2] * wz;
 }
 
-// Geometry of one (cell, direction) item from the cell's normals and heights g[16]:
-// r[f] = H_f / -cos_f for the in-faces (cos_f < 0), 0 for the others, and the code word
-//   bits 0-3   in-faces (cos_f < 0)
-//   bits 4-7   out-faces (cos_f > 0)
-//   bits 8-23  per vertex v (4 bits at 8 + 4v) the in-face its node is traced to: face
-//              index, bit 2 lam = 2/3 (the face opposite v), bit 3 no in-face.
-// Node selection: the restatement takes, for each node, the in-face with the smallest
-// (t, face index); t = t4 = 2r/3 for the face opposite the node's own vertex, t1 = r/6 for
-// the others.  So only the two smallest in-faces by (t1, index) are needed: the node's
-// candidate among the other faces is the best unless that is its own opposite face.  The
-// choice depends on the node's vertex only, not on the out-face the node belongs to.
+// Code word of an item:
+//   bits 0-1, 2-3, 4-5  the in-faces (cos < 0) b1, b2 and the third, as far as there are
+//   bits 6-7            their number (at most three: the four outward normals weighted by
+//                       the face areas sum to zero)
+//   bits 8-11           out-faces (cos > 0)
+//   bit 12              the node at b1's vertex is traced to b2 (else to b1, lam = 2/3)
+constexpr uint32_t kCodeB2 = 1u << 12;
+
+// Code word and distances of one (cell, direction) from the cell's normals and heights
+// g[16]: tA = r_b1 / 6, tB = r_b2 / 6 (bit 12; else 0).  b1, b2: the smallest by (t, face
+// index), as the restatement compares them; an equal 2/3 r_b1 = r_b2 / 6 goes to the lower
+// face index.
 template <class T>
-__device__ __forceinline__ uint32_t item_geometry(const T *g, T wx, T wy, T wz, T (&r)[4]) {
-  T cosf[4], t1[4], t4[4];
-  face_cos(g, wx, wy, wz, cosf);
-  uint32_t code = 0;
+__device__ __forceinline__ uint32_t item_geometry(const T *g, const T *cosf, T &tA, T &tB) {
+  uint32_t out = 0;
+  int b1 = -1, b2 = -1, n = 0, sum = 0;
+  T tb1 = 0, tb2 = 0, rb1 = 0;
 #pragma unroll
   for (int f = 0; f < 4; f++) {
-    r[f] = t1[f] = t4[f] = (T)0;
     if (cosf[f] < 0) {
-      r[f] = dv(g[12 + f], -cosf[f]);
-      t1[f] = (T)(1.0 / 6.0) * r[f];
-      t4[f] = (T)(2.0 / 3.0) * r[f];
-      code |= 1u << f;
+      const T r = dv(g[12 + f], -cosf[f]);
+      const T t1 = (T)(1.0 / 6.0) * r;
+      n++;
+      sum += f;
+      if (b1 < 0 || t1 < tb1) {
+        b2 = b1;
+        tb2 = tb1;
+        b1 = f;
+        tb1 = t1;
+        rb1 = r;
+      } else if (b2 < 0 || t1 < tb2) {
+        b2 = f;
+        tb2 = t1;
+      }
     } else if (cosf[f] > 0) {
-      code |= 16u << f;
+      out |= 1u << f;
     }
   }
-  int b1 = -1, b2 = -1;
-  T tb1 = 0, tb2 = 0;
-#pragma unroll
-  for (int f = 0; f < 4; f++) {
-    if (!(cosf[f] < 0)) continue;
-    if (b1 < 0 || t1[f] < tb1) {
-      b2 = b1;
-      tb2 = tb1;
-      b1 = f;
-      tb1 = t1[f];
-    } else if (b2 < 0 || t1[f] < tb2) {
-      b2 = f;
-      tb2 = t1[f];
+  n = min(n, 3);  // four only on a mesh whose cells do not close
+  tA = tb1;
+  tB = (T)0;
+  uint32_t code = out << 8 | (uint32_t)n << 6;
+  if (n >= 1) code |= (uint32_t)b1;
+  if (n >= 2) {
+    code |= (uint32_t)b2 << 2;
+    const T t4 = (T)(2.0 / 3.0) * rb1;
+    if (!(t4 < tb2 || (t4 == tb2 && b1 < b2))) {
+      code |= kCodeB2;
+      tB = tb2;
     }
   }
-#pragma unroll
-  for (int v = 0; v < 4; v++) {
-    const int B = b1 != v ? b1 : b2;
-    const T tB = b1 != v ? tb1 : tb2;
-    uint32_t cv;
-    if (cosf[v] < 0 && (B < 0 || t4[v] < tB || (t4[v] == tB && v < B)))
-      cv = (uint32_t)v | 4u;
-    else
-      cv = B < 0 ? 8u : (uint32_t)B;
-    code |= cv << (8 + 4 * v);
-  }
+  if (n >= 3) code |= (uint32_t)((sum - b1 - b2) & 3) << 4;
   return code;
 }
 
+// weights (area_j / sum of the areas) of the in-faces b1, b2 and the third, 0 where there is none
+template <class T>
+__device__ __forceinline__ void in_weights(const T *wt, uint32_t code, T (&w)[3]) {
+  const int nin = (int)(code >> 6) & 3;
+#pragma unroll
+  for (int q = 0; q < 3; q++) w[q] = q < nin ? wt[(code >> (2 * q)) & 3] : (T)0;
+}
 
-// G values at p (contiguous), vectorised for 2 and 4 groups
-template <class T, int G>
+// 32 bytes of global memory in one access (32-byte aligned)
+__device__ __forceinline__ void ld_32(const double *p, double &a, double &b, double &c, double &d) {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_32(double *p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+// G values at p (contiguous), vectorised for 2 and 4 groups; GMEM: p is in global memory,
+// 32-byte aligned when the values are 32 bytes
+template <bool GMEM, class T, int G>
 __device__ __forceinline__ void ld_groups(const T *p, T (&v)[G]) {
-  if constexpr (sizeof(T) == 8 && G % 2 == 0) {
+  if constexpr (GMEM && sizeof(T) == 8 && G == 4) {
+    ld_32(p, v[0], v[1], v[2], v[3]);
+  } else if constexpr (sizeof(T) == 8 && G % 2 == 0) {
 #pragma unroll
     for (int q = 0; q < G / 2; q++) {
       const double2 x = reinterpret_cast<const double2 *>(p)[q];
@@ -193,499 +194,510 @@ __device__ __forceinline__ void ld_groups(const T *p, T (&v)[G]) {
     for (int q = 0; q < G; q++) v[q] = p[q];
   }
 }
-// G values to a face-value slot of GS values; float slots of 4 groups are padded to 8 so
-// that every store fills a whole 32-byte sector
-template <class T, int G>
-__device__ __forceinline__ void st_slot(T *p, const T (&v)[G]) {
-  if constexpr (sizeof(T) == 8 && G % 2 == 0) {
+template <bool GMEM, class T, int G>
+__device__ __forceinline__ void st_groups(T *p, const T (&v)[G]) {
+  if constexpr (GMEM && sizeof(T) == 8 && G == 4) {
+    st_32(p, v[0], v[1], v[2], v[3]);
+  } else if constexpr (sizeof(T) == 8 && G % 2 == 0) {
 #pragma unroll
     for (int q = 0; q < G / 2; q++) reinterpret_cast<double2 *>(p)[q] = make_double2(v[2 * q], v[2 * q + 1]);
   } else if constexpr (sizeof(T) == 4 && G == 4) {
-    reinterpret_cast<float4 *>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4 *>(p)[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
   } else {
 #pragma unroll
     for (int q = 0; q < G; q++) p[q] = v[q];
   }
 }
 
-// One thread per (cell, direction) pair of a level: the out-face values of all
-// groups.  GT: compile-time group count (1, 2 or 4), 0 for any other (loop).
+// T: records, slots and the transport arithmetic; S and I come and go as TI.
+template <class T, class TI>
+struct SweepArgs {
+  int64_t N;
+  int d0, G, SW;
+  int qs;                   // 1: Q per group, 0: one for all
+  const uint4 *ord;         // [M][N] items in sweep order {cell, code, own | in0 << 16, in1 | in2 << 16}
+  const uint2 *ord_hi;      // [M][N] upper halves of the slots (WIDE)
+  const T *dist;            // [M][N][2] {tA, tB} (GEO)
+  const T *wgt, *wgt3;      // [M][N][2], [M][N] weights of the in-faces (GEO)
+  const T *rec, *w, *wt;    // geometry records and directions (not GEO), face weights [N][4]
+  const int32_t *lvl;       // level offsets of every direction
+  const int64_t *lvl_base;  // [M] first entry in lvl
+  const int32_t *depth;     // [M] levels
+  const T *src;             // [N][SW]
+  T *slots;                 // [directions of the launch][nhigh][G]: slots from `cap` on
+  uint32_t cap;             // slots in shared memory
+  int64_t nhigh;
+  const TI *S;              // S and I element (cell c, direction d0 + x, group g) at c * sc + x * sd + g
+  TI *I;
+  int64_t sc, sd;
+  T bc;
+};
+
+// One CTA per direction.  GT: compile-time group count (1, 2 or 4), 0 for any other.
+// HIGH: slots from a.cap on are in global memory (the others in shared memory).  GEO: distances and weights from the stream, else
+// from the cell's records.  Slot 0 holds the boundary value for the whole sweep; an item
+// whose own slot is 0 has no downwind neighbour and writes none.
 //
-// Node distances: node q of out-face j is traced to the in-face f with the
-// smallest t = lam r_f (r_f = H_f / -cos_f, lam = 2/3 when f is opposite the
-// node's own vertex, 1/6 otherwise), compared exactly as in the restatement.
-// The attenuations need only one exponential per in-face: E1_f = exp(-k r_f / 6)
-// and exp(-k 2 r_f / 3) = E1_f^4 (equal to a few ulp).
-template <class T, class TV, class TI, int GT, bool PRE>
-__global__ void __launch_bounds__(kSweepThreads) k_sweep_level(SweepArgs<T, TV> a) {
-  // Levels after the first of a batch are launched with programmatic stream
-  // serialisation: the next level may start while this one drains, and everything up to
-  // the first face-value read (item, cell record, source record, S, geometry,
-  // exponentials) overlaps the previous level; griddepcontrol.wait then waits for the
-  // previous level to complete and its writes to be visible.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  const uint32_t it = a.items[i];
-  uint4 gq = make_uint4(0u, 0u, 0u, 0u);
-  if constexpr (PRE) gq = __ldcs(a.geo + i);  // read once per sweep, in item order
-  const int64_t c = it & ((1u << a.shift) - 1u);
-  const int dl = (int)(it >> a.shift);
-  const int d = a.d0 + dl;
-  int fid[4];
-  T r[4];
-  uint32_t code;
-  const T *rc = a.rec + (int64_t)a.RW * c;
-  if constexpr (PRE) {
-    // the item's geometry from the stream (item_geometry at setup, the in-face distances
-    // in face order, k_plan_geometry's format); of the cell record only the face-value
-    // slots and the source record are read
-    const int4 f = __ldg(reinterpret_cast<const int4 *>(rc + Rec<T>::IDS));
-    fid[0] = f.x, fid[1] = f.y, fid[2] = f.z, fid[3] = f.w;
-    code = gq.x;
-    int m = 0;
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int f = 0; f < 4; f++) {
-        r[f] = (T)0;
-        if ((code >> f) & 1u) {
-          r[f] = __uint_as_float(m == 0 ? gq.y : m == 1 ? gq.z : gq.w);
-          m++;
-        }
-      }
-    } else {
-      // 2^(e-32), exact: e in [-127, 127]
-      const double down = __hiloint2double((int)((code >> 24) - 128u - 32u + 1023u) << 20, 0);
-#pragma unroll
-      for (int f = 0; f < 4; f++) {
-        r[f] = (T)0;
-        if ((code >> f) & 1u) {
-          r[f] = (T)((double)(m == 0 ? gq.y : m == 1 ? gq.z : gq.w) * down);
-          m++;
-        }
-      }
-    }
-  } else {
-    T g[16];
-    load_rec<T>(rc, g, fid);
-    code = item_geometry<T>(g, a.w[3 * d], a.w[3 * d + 1], a.w[3 * d + 2], r);
-  }
-  const T *dy = rc + Rec<T>::DYN;
-  const T k = dy[0], bk = dy[1];
-  const SweepIO io = *a.io;
-  const TI *Sv = (const TI *)io.S;
-  // S element (group gg) of this cell and direction: base + gg * gs
-  int64_t base, gs;
-  if (io.layout) {
-    base = (c * a.M + d) * a.G;
-    gs = 1;
-  } else {
-    base = (int64_t)io.row_of[c] * a.G * a.M + d;
-    gs = a.M;
-  }
-  TV E1[4], E4[4];
-#pragma unroll
-  for (int f = 0; f < 4; f++) {
-    E1[f] = E4[f] = (TV)1;
-    if ((code >> f) & 1u) {
-      const T t1 = (T)(1.0 / 6.0) * r[f];
-      E1[f] = ex((TV)(-k * t1));
-      const TV e2 = E1[f] * E1[f];
-      E4[f] = e2 * e2;
-    }
-  }
-  // 4 bits per (out-face, node) from the node's vertex code; out-faces compacted into
-  // slots (2 bits each in jo)
-  uint64_t sel = 0;
-  uint32_t jo = 0;
-  int nout = 0;
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    if (!((code >> (4 + j)) & 1u)) continue;
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      const int vq = (j + 1 + q) & 3;
-      sel |= (uint64_t)((code >> (8 + 4 * vq)) & 15u) << (12 * nout + 4 * q);
-    }
-    jo |= (uint32_t)j << (2 * nout);
-    nout++;
-  }
-  if constexpr (GT > 0) {
-    // separate per-face arrays (not one [4][GT] array), selected by comparisons, so that
-    // no selection turns into an indexed local-memory access
-    TV rhs[GT], f0[GT], f1[GT], f2[GT], f3[GT];
-    TI sv[GT];
-    if (io.layout) {
-      ld_groups<TI, GT>(Sv + base, sv);
-    } else {
-#pragma unroll
-      for (int q = 0; q < GT; q++) sv[q] = Sv[base + q * gs];
-    }
-#pragma unroll
-    for (int q = 0; q < GT; q++) rhs[q] = (TV)dy[2 + q] + (TV)bk * (TV)sv[q];
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    auto in_face = [&](int j, TV (&fj)[GT]) {
-      if (((code >> j) & 1u) && fid[j] >= 0) {
-        ld_groups<TV, GT>(a.fv + ((int64_t)dl * a.NF + fid[j]) * a.GS, fj);
+// Each item has three uncoalesced accesses, each one access of up to 32 bytes: its source
+// record, S and I; the slots are in shared memory as far as they fit.  Only the slot values
+// depend on the levels before, so a thread loads the record of its item after the next, and
+// the source and S of its next one, while it works on one item.  Measured (whole sweep with
+// its copies, before: one launch per level of all directions, face values in HBM): 48^3 x 6
+// cells x 256 directions FP64, one group, 28.1 -> 5.2 ms; 12^3 x 6 x 64, 269 -> 87 us; the
+// mixed sweep of 4 groups at 48^3 x 256, 37.0 -> 13 ms.  What bounds it: issue slots and the
+// latency of those accesses at 16 warps an SM (about 400 instructions an item of a warp).
+template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB>
+__global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
+  extern __shared__ __align__(16) uint8_t sweep_smem[];
+  constexpr int GR = GT > 0 ? GT : 1;
+  const int x = blockIdx.x, d = a.d0 + x;
+  const int G = GT > 0 ? GT : a.G;
+  T *const low = reinterpret_cast<T *>(sweep_smem);
+  T *const high = HIGH ? a.slots + (int64_t)x * a.nhigh * G : nullptr;
+  auto get_slot = [&](uint32_t q, T (&v)[GR]) {
+    if (HIGH && q >= a.cap)
+      ld_groups<true>(high + (int64_t)(q - a.cap) * GR, v);
+    else
+      ld_groups<false>(low + q * GR, v);
+  };
+  auto slot = [&](uint32_t q) {
+    if (HIGH && q >= a.cap) return high + (int64_t)(q - a.cap) * G;
+    return low + q * (uint32_t)G;
+  };
+  const int64_t at = (int64_t)d * a.N;
+  const uint4 *ord = a.ord + at;
+  const int32_t *lvl = a.lvl + a.lvl_base[d];
+  const int depth = a.depth[d];
+  const TI *S = a.S + x * a.sd;
+  TI *I = a.I + x * a.sd;
+  const int N = (int)a.N;
+  T wx = 0, wy = 0, wz = 0;
+  if (!GEO) wx = a.w[3 * d], wy = a.w[3 * d + 1], wz = a.w[3 * d + 2];
+  for (int g = threadIdx.x; g < G; g += NT) low[g] = a.bc;
+  __syncthreads();
+
+  struct Item {
+    uint4 o;
+    uint2 hi;
+    T tA, tB, w[3];
+    T k, bk, q[GR];
+    TI s[GR];
+  };
+  auto load_record = [&](int i, Item &it) {
+    it.o = __ldcs(ord + i);
+    if constexpr (WIDE) it.hi = __ldcs(a.ord_hi + at + i);
+    if constexpr (GEO) {
+      if constexpr (sizeof(T) == 8) {
+        const double2 t = __ldcs(reinterpret_cast<const double2 *>(a.dist) + at + i);
+        const double2 u = __ldcs(reinterpret_cast<const double2 *>(a.wgt) + at + i);
+        it.tA = t.x, it.tB = t.y, it.w[0] = u.x, it.w[1] = u.y;
       } else {
-#pragma unroll
-        for (int q = 0; q < GT; q++) fj[q] = a.bc;
+        const float2 t = __ldcs(reinterpret_cast<const float2 *>(a.dist) + at + i);
+        const float2 u = __ldcs(reinterpret_cast<const float2 *>(a.wgt) + at + i);
+        it.tA = t.x, it.tB = t.y, it.w[0] = u.x, it.w[1] = u.y;
       }
-    };
-    in_face(0, f0);
-    in_face(1, f1);
-    in_face(2, f2);
-    in_face(3, f3);
-    const TV E1_0 = E1[0], E1_1 = E1[1], E1_2 = E1[2], E1_3 = E1[3];
-    const TV E4_0 = E4[0], E4_1 = E4[1], E4_2 = E4[2], E4_3 = E4[3];
-    const int64_t fid0 = slot_of(fid[0]), fid1 = slot_of(fid[1]), fid2 = slot_of(fid[2]), fid3 = slot_of(fid[3]);
-    // the (at most three) out-faces, one slot after another
-    for (int o = 0; o < nout; o++) {
-      const int j = (jo >> (2 * o)) & 3;
-      TV e[3];
-      int h[3];
-#pragma unroll
-      for (int n = 0; n < 3; n++) {
-        const uint32_t code = (uint32_t)(sel >> (12 * o + 4 * n)) & 15u;
-        h[n] = code & 8u ? -1 : (int)(code & 3u);
-        const bool four = code & 4u;
-        e[n] = h[n] == 0 ? (four ? E4_0 : E1_0)
-             : h[n] == 1 ? (four ? E4_1 : E1_1)
-             : h[n] == 2 ? (four ? E4_2 : E1_2)
-             : h[n] == 3 ? (four ? E4_3 : E1_3) : (TV)1;
-      }
-      TV out[GT];
-#pragma unroll
-      for (int q = 0; q < GT; q++) {
-        TV I0[3];
-#pragma unroll
-        for (int n = 0; n < 3; n++)
-          I0[n] = h[n] == 0 ? f0[q] : h[n] == 1 ? f1[q] : h[n] == 2 ? f2[q] : h[n] == 3 ? f3[q] : a.bc;
-        TV Icur = e[0] * (I0[0] - rhs[q]) + rhs[q];
-        Icur += (e[1] * (I0[1] - rhs[q]) + rhs[q]);
-        Icur += (e[2] * (I0[2] - rhs[q]) + rhs[q]);
-        out[q] = Icur * (TV)0.3333333333333333;
-      }
-      const int64_t fj = j == 0 ? fid0 : j == 1 ? fid1 : j == 2 ? fid2 : fid3;
-      st_slot<TV, GT>(a.fv + ((int64_t)dl * a.NF + fj) * a.GS, out);
+      it.w[2] = __ldcs(a.wgt3 + at + i);
     }
-  } else {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int gg = 0; gg < a.G; gg++) {
-      const TV rhs = (TV)dy[2 + gg] + (TV)bk * (TV)Sv[base + gg * gs];
-      TV fvals[4];
+  };
+  auto load_cell = [&](Item &it) {
+    const int64_t c = it.o.x;
+    const T *sr = a.src + c * a.SW;
+    T q0, q1;
+    if constexpr (sizeof(T) == 8) {
+      ld_32(sr, it.k, it.bk, q0, q1);
+    } else {
+      const float4 t = __ldg(reinterpret_cast<const float4 *>(sr));
+      it.k = t.x, it.bk = t.y, q0 = t.z, q1 = t.w;
+    }
+    if constexpr (GT > 0) {
+      ld_groups<true>(S + c * a.sc, it.s);
 #pragma unroll
-      for (int j = 0; j < 4; j++)
-        fvals[j] = (((code >> j) & 1u) && fid[j] >= 0) ? a.fv[((int64_t)dl * a.NF + fid[j]) * a.GS + gg] : a.bc;
-      for (int o = 0; o < nout; o++) {
-        const int j = (jo >> (2 * o)) & 3;
-        TV I0[3], e[3];
+      for (int g = 0; g < GT; g++) it.q[g] = q0;
+      if constexpr (GT > 1) {
+        if (a.qs) {
+          it.q[1] = q1;
 #pragma unroll
-        for (int n = 0; n < 3; n++) {
-          const uint32_t code = (uint32_t)(sel >> (12 * o + 4 * n)) & 15u;
-          const int h = code & 8u ? -1 : (int)(code & 3u);
-          I0[n] = a.bc;
-          e[n] = (TV)1;
-#pragma unroll
-          for (int f = 0; f < 4; f++)
-            if (h == f) {
-              I0[n] = fvals[f];
-              e[n] = code & 4u ? E4[f] : E1[f];
-            }
+          for (int g = 2; g < GT; g++) it.q[g] = __ldg(sr + kSrcQ + g);
         }
-        TV Icur = e[0] * (I0[0] - rhs) + rhs;
-        Icur += (e[1] * (I0[1] - rhs) + rhs);
-        Icur += (e[2] * (I0[2] - rhs) + rhs);
-        a.fv[((int64_t)dl * a.NF + slot_of(fid[j])) * a.GS + gg] = Icur * (TV)0.3333333333333333;
       }
     }
+  };
+
+  // this thread's items in order, two ahead of the one in work: position p in the level that
+  // ends at p_hi (the next one at p_hi2); N when there are none left
+  int p = (int)threadIdx.x, p_lvl = 0, p_hi = lvl[1], p_hi2 = lvl[min(2, depth)];
+  auto settle = [&]() {
+    while (p >= p_hi && p_hi < N) {
+      p = p_hi + (int)threadIdx.x;
+      p_lvl++;
+      p_hi = p_hi2;
+      p_hi2 = lvl[min(p_lvl + 2, depth)];
+    }
+  };
+  Item it, next;
+  settle();
+  int i = p;
+  if (p < N) {
+    load_record(p, it);
+    load_cell(it);
+    p += NT;
+    settle();
+    if (p < N) load_record(p, next);
+  }
+  int hi = lvl[1], hi2 = lvl[min(2, depth)];
+  for (int L = 0; L < depth; L++) {
+    while (i < hi) {
+      const Item now = it;
+      i = p;
+      it = next;
+      if (p < N) {
+        load_cell(it);
+        p += NT;
+        settle();
+        if (p < N) load_record(p, next);
+      }
+      const int64_t c = now.o.x;
+      const uint32_t code = now.o.y;
+      uint32_t own = now.o.z & 0xffffu, s0 = now.o.z >> 16, s1 = now.o.w & 0xffffu, s2 = now.o.w >> 16;
+      if constexpr (WIDE) {
+        own |= now.hi.x << 16;
+        s0 |= now.hi.x & 0xffff0000u;
+        s1 |= now.hi.y << 16;
+        s2 |= now.hi.y & 0xffff0000u;
+      }
+      T tA, tB, w[3];
+      if constexpr (GEO) {
+        tA = now.tA, tB = now.tB, w[0] = now.w[0], w[1] = now.w[1], w[2] = now.w[2];
+      } else {
+        T g[16], cosf[4];
+        load_vec<T>(a.rec + c * Rec<T>::RW, g, 16);
+        face_cos(g, wx, wy, wz, cosf);
+        (void)item_geometry<T>(g, cosf, tA, tB);  // the code word is the plan's
+        in_weights(a.wt + 4 * c, code, w);
+      }
+      const T k = now.k, bk = now.bk;
+      const int nin = (int)(code >> 6) & 3;
+      const bool two = (code & kCodeB2) != 0;
+      const T EA = ex(-k * tA);
+      T EB = EA * EA;
+      EB = EB * EB;
+      if (two) EB = ex(-k * tB);
+      T wo = ((T)1 - w[0]) - (w[1] + w[2]);  // all out-faces together
+      T par = (T)0;                          // a face parallel to the direction holds the boundary value
+      if (nin + __popc((code >> 8) & 15u) != 4) {
+        uint32_t seen = (code >> 8) & 15u;
+        if (nin > 0) seen |= 1u << (code & 3);
+        if (nin > 1) seen |= 1u << ((code >> 2) & 3);
+        if (nin > 2) seen |= 1u << ((code >> 4) & 3);
+        wo = (T)0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const T wj = a.wt[4 * c + j];
+          if ((code >> (8 + j)) & 1u) wo += wj;
+          if (!((seen >> j) & 1u)) par += wj * a.bc;
+        }
+      }
+      auto value = [&](T v0, T v1, T v2, T rhs, T &cell) {
+        const T A = EA * (v0 - rhs) + rhs;
+        const T B = EB * ((two ? v1 : v0) - rhs) + rhs;
+        const T o = ((A + A) + B) * (T)0.3333333333333333;
+        cell = (v0 * w[0] + v1 * w[1]) + (v2 * w[2] + o * wo) + par;
+        return o;
+      };
+      TI *Ic = I + c * a.sc;
+      if constexpr (GT > 0) {
+        TI iv[GT];
+        T v0[GT], v1[GT], v2[GT], o[GT];
+        get_slot(s0, v0);
+#pragma unroll
+        for (int g = 0; g < GT; g++) v1[g] = v2[g] = (T)0;
+        if (nin > 1) get_slot(s1, v1);
+        if (nin > 2) get_slot(s2, v2);
+#pragma unroll
+        for (int g = 0; g < GT; g++) {
+          T cell;
+          o[g] = value(v0[g], v1[g], v2[g], now.q[g] + bk * (T)now.s[g], cell);
+          iv[g] = (TI)cell;
+        }
+        if (HIGH && own >= a.cap)
+          st_groups<true>(high + (int64_t)(own - a.cap) * GR, o);
+        else if (own)
+          st_groups<false>(low + own * GR, o);
+        st_groups<true>(Ic, iv);
+      } else {
+        const T *sr = a.src + c * a.SW + kSrcQ;
+        const TI *Sc = S + c * a.sc;
+        for (int g = 0; g < G; g++) {
+          const T v0 = slot(s0)[g];
+          const T v1 = nin > 1 ? slot(s1)[g] : (T)0;
+          const T v2 = nin > 2 ? slot(s2)[g] : (T)0;
+          T cell;
+          const T o = value(v0, v1, v2, sr[g * a.qs] + bk * (T)Sc[g], cell);
+          if (own) slot(own)[g] = o;
+          Ic[g] = (TI)cell;
+        }
+      }
+    }
+    hi = hi2;
+    hi2 = lvl[min(L + 3, depth)];
+    __syncthreads();
   }
 }
 
-// Cell values of one direction batch from its face values: ReCalcIllumOpt
-// (illum_utils.cpp:377-433), the area-weighted face mean, a plain mean for the caller's
-// last cell.  Faces nobody wrote for a direction (inflow boundary, parallel to it) hold
-// the boundary value.  A CTA takes 32 cells (lane = cell) x 32 directions of the batch (four
-// per warp): the face values of one direction are stored direction-major, so a warp's reads
-// of 32 neighbouring cells' face slots fall close together (a face shared by two of them is
-// read from L1 the second time), and each cell's record is read once per CTA.  The cell
-// values go through a shared-memory tile [direction][cell + 1 pad] and each warp writes four
-// cells' rows, lane = direction, so the stores of a cell's 32 directions are contiguous.
-constexpr int kRcCells = 32, kRcDirs = 32;
-template <class T, class TV, class TI, int GT>
-__global__ void __launch_bounds__(256) k_recalc(SweepArgs<T, TV> a, int64_t N) {
-  constexpr int GQ = GT > 0 ? GT : 1;
-  __shared__ __align__(16) TI tile[kRcDirs][kRcCells + 1][GQ];
-  // the tile's cells: outward normals, face areas and face-value slots, read once per CTA
-  __shared__ T s_n[kRcCells][12];
-  __shared__ T s_area[kRcCells][4];
-  __shared__ int s_fid[kRcCells][4];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t c = (int64_t)blockIdx.x * kRcCells + lane;
-  const int dl0 = (int)blockIdx.y * kRcDirs;
-  const bool cell_ok = c < N;
-  if (warp == 0 && cell_ok) {
-    T g[16];
-    int f[4];
-    load_rec<T>(a.rec + (int64_t)a.RW * c, g, f);
+// The sweep's own layout is [direction][cell * G + g] in context numbering (V = TI), so that
+// the cells of a front, close together in Morton order, lie close together in memory.  These
+// tiles of 32 x 32 values of type V bring an array there and back through shared memory,
+// whole lines on both sides, directions d0 .. d0 + nd - 1:
+//   rows [rows][M] in caller numbering (perm; row = cell * G + g, V = TI), or
+//   [cells][M][G] in context numbering (perm null; V = the G values of a cell and direction).
+template <class V, bool IMPORT>
+__global__ void __launch_bounds__(256) k_tile(int64_t rows, int G, int M, int d0, int nd, const int32_t *perm,
+                                              const V *in, V *out) {
+  __shared__ V tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t r0 = (int64_t)blockIdx.x * 32;
+  const int x0 = blockIdx.y * 32;
+  auto row = [&](int64_t r) { return (perm ? (int64_t)perm[r / G] * G + r % G : r) * M + d0 + x0 + tx; };
 #pragma unroll
-    for (int q = 0; q < 12; q++) s_n[lane][q] = g[q];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      s_area[lane][j] = __ldg(a.area + 4 * c + j);
-      s_fid[lane][j] = f[j];
+  for (int k = 0; k < 4; k++) {
+    const int y = ty + 8 * k;
+    if (IMPORT) {
+      if (r0 + y < rows && x0 + tx < nd) tile[y][tx] = in[row(r0 + y)];
+    } else {
+      if (r0 + tx < rows && x0 + y < nd) tile[y][tx] = in[(int64_t)(x0 + y) * rows + r0 + tx];
     }
   }
   __syncthreads();
-  const SweepIO io = *a.io;
-  TI *I = (TI *)io.I;
-  const bool last = c == a.last;
-  auto cell_value = [&](const TV *fv) {
-    TV curI = 0;
-    if (!last) {
-      TV Ssum = 0;
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        curI += fv[j] * (TV)s_area[lane][j];
-        Ssum += (TV)s_area[lane][j];
-      }
-      curI /= Ssum;
+  for (int k = 0; k < 4; k++) {
+    const int y = ty + 8 * k;
+    if (IMPORT) {
+      if (r0 + tx < rows && x0 + y < nd) out[(int64_t)(x0 + y) * rows + r0 + tx] = tile[tx][y];
     } else {
-#pragma unroll
-      for (int j = 0; j < 4; j++) curI += fv[j];
-      curI /= (TV)4;
-    }
-    return curI;
-  };
-#pragma unroll 1
-  for (int k = 0; k < kRcDirs / 8; k++) {
-    const int dd = warp * (kRcDirs / 8) + k;  // direction within the tile
-    const int dl = dl0 + dd;
-    if (!cell_ok || dl >= a.nbd) continue;
-    const int d = a.d0 + dl;
-    T cosf[4];
-    face_cos(s_n[lane], a.w[3 * d], a.w[3 * d + 1], a.w[3 * d + 2], cosf);
-    int fid[4];
-    bool have[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      fid[j] = s_fid[lane][j];
-      have[j] = cosf[j] > 0 || (cosf[j] < 0 && fid[j] >= 0);
-    }
-    const TV *fvd = a.fv + (int64_t)dl * a.NF * a.GS;
-    if constexpr (GT > 0) {
-      // all four face slots in flight at once, vector loads
-      TV f0[GT], f1[GT], f2[GT], f3[GT];
-      auto slot = [&](int j, TV (&fj)[GT]) {
-        if (have[j]) {
-          ld_groups<TV, GT>(fvd + slot_of(fid[j]) * a.GS, fj);
-        } else {
-#pragma unroll
-          for (int q = 0; q < GT; q++) fj[q] = a.bc;
-        }
-      };
-      slot(0, f0);
-      slot(1, f1);
-      slot(2, f2);
-      slot(3, f3);
-#pragma unroll
-      for (int q = 0; q < GT; q++) {
-        const TV fv[4] = {f0[q], f1[q], f2[q], f3[q]};
-        tile[dd][lane][q] = (TI)cell_value(fv);  // the cell values as stored (float in the mixed form)
-      }
-    } else {
-      int64_t base, gs;
-      if (io.layout) {
-        base = (c * a.M + d) * a.G;
-        gs = 1;
-      } else {
-        base = (int64_t)io.row_of[c] * a.G * a.M + d;
-        gs = a.M;
-      }
-      for (int gg = 0; gg < a.G; gg++) {
-        TV fv[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) fv[j] = have[j] ? fvd[slot_of(fid[j]) * a.GS + gg] : a.bc;
-        I[base + gg * gs] = (TI)cell_value(fv);
-      }
-    }
-  }
-  if constexpr (GT > 0) {
-    __syncthreads();
-    const int dl = dl0 + lane;
-    if (dl < a.nbd) {
-      const int d = a.d0 + dl;
-#pragma unroll 1
-      for (int k = 0; k < kRcCells / 8; k++) {
-        const int cl = warp * (kRcCells / 8) + k;
-        const int64_t cc = (int64_t)blockIdx.x * kRcCells + cl;
-        if (cc >= N) break;
-        const TI *v = tile[lane][cl];
-        if (io.layout) {
-          TI *o = I + (cc * a.M + d) * a.G;
-          if constexpr (sizeof(TI) == 8 && GT % 2 == 0) {
-#pragma unroll
-            for (int q = 0; q < GT / 2; q++) reinterpret_cast<double2 *>(o)[q] = make_double2(v[2 * q], v[2 * q + 1]);
-          } else if constexpr (sizeof(TI) == 4 && GT == 4) {
-            *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
-          } else {
-#pragma unroll
-            for (int q = 0; q < GT; q++) o[q] = v[q];
-          }
-        } else {
-          const int64_t base = (int64_t)io.row_of[cc] * a.G * a.M + d;
-#pragma unroll
-          for (int q = 0; q < GT; q++) I[base + (int64_t)q * a.M] = v[q];
-        }
-      }
+      if (r0 + y < rows && x0 + tx < nd) out[row(r0 + y)] = tile[tx][y];
     }
   }
 }
 
 // ---------------------------------------------------------------- plan
-template <class T>
-__global__ void k_plan_init(int64_t N, int nbd, int shift, int d0, const T *w, const T *rec, int RW, uint32_t *indeg,
-                            uint32_t *plan, unsigned long long *tail) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= N * nbd) return;
-  const int64_t c = i / nbd;
-  const int dl = (int)(i - c * nbd);
-  const int d = d0 + dl;
-  T g[12];
-  int nbr[4];
-  load_normals<T>(rec + (int64_t)RW * c, RW, g, nbr);
-  T cosf[4];
-  face_cos(g, w[3 * d], w[3 * d + 1], w[3 * d + 2], cosf);
-  uint32_t cnt = 0;
-#pragma unroll
-  for (int j = 0; j < 4; j++) cnt += (cosf[j] < 0 && nbr[j] >= 0) ? 1u : 0u;
-  indeg[i] = cnt;
-  if (cnt == 0) plan[atomicAdd(tail, 1ull)] = ((uint32_t)dl << shift) | (uint32_t)c;
-}
+constexpr int kPlanThreads = 1024;
 
+// Levels of every cell for one direction per CTA (breadth first: a cell joins the queue
+// when its last upwind neighbour has been taken).  level [nd][N]; indeg, queue [nd][N]
+// scratch; depth, count [nd]: levels and cells reached (fewer than N: a cycle).
 template <class T>
-__global__ void k_plan_expand(const uint32_t *cur, int64_t n, int nbd, int shift, int d0, const T *w, const T *rec,
-                              int RW, uint32_t *indeg, uint32_t *plan, unsigned long long *tail) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t it = cur[i];
-  const int64_t c = it & ((1u << shift) - 1u);
-  const int dl = (int)(it >> shift);
-  const int d = d0 + dl;
-  T g[12];
-  int nbr[4];
-  load_normals<T>(rec + (int64_t)RW * c, RW, g, nbr);
-  T cosf[4];
-  face_cos(g, w[3 * d], w[3 * d + 1], w[3 * d + 2], cosf);
+__global__ void __launch_bounds__(kPlanThreads) k_plan_levels(int64_t N, int d0, const T *w, const T *rec,
+                                                              uint32_t *indeg_all, uint32_t *queue_all,
+                                                              uint32_t *level_all, int32_t *depth, int32_t *count) {
+  __shared__ int tail;
+  const int x = blockIdx.x, d = d0 + x;
+  uint32_t *indeg = indeg_all + x * N, *queue = queue_all + x * N, *level = level_all + x * N;
+  const T wx = w[3 * d], wy = w[3 * d + 1], wz = w[3 * d + 2];
+  if (threadIdx.x == 0) tail = 0;
+  __syncthreads();
+  auto faces = [&](int64_t c, T *cosf, int *nbr) {
+    T g[12];
+    load_vec<T>(rec + c * Rec<T>::RW, g, 12);
+    load_nbr<T>(rec + c * Rec<T>::RW, nbr);
+    face_cos(g, wx, wy, wz, cosf);
+  };
+  for (int64_t c = threadIdx.x; c < N; c += kPlanThreads) {
+    T cosf[4];
+    int nbr[4];
+    faces(c, cosf, nbr);
+    uint32_t n = 0;
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    if (!(cosf[j] > 0) || nbr[j] < 0) continue;
-    const int64_t q = (int64_t)nbr[j] * nbd + dl;
-    if (atomicSub(indeg + q, 1u) == 1u) plan[atomicAdd(tail, 1ull)] = ((uint32_t)dl << shift) | (uint32_t)nbr[j];
+    for (int j = 0; j < 4; j++) n += (cosf[j] < 0 && nbr[j] >= 0) ? 1u : 0u;
+    indeg[c] = n;
+    if (n == 0) {
+      level[c] = 0;
+      queue[atomicAdd(&tail, 1)] = (uint32_t)c;
+    }
+  }
+  __syncthreads();
+  int lo = 0, hi = tail, L = 0;
+  __syncthreads();  // every thread has read tail before it moves on
+  while (lo < hi) {
+    L++;
+    for (int i = lo + (int)threadIdx.x; i < hi; i += kPlanThreads) {
+      T cosf[4];
+      int nbr[4];
+      faces(queue[i], cosf, nbr);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (cosf[j] > 0 && nbr[j] >= 0 && atomicSub(indeg + nbr[j], 1u) == 1u) {
+          level[nbr[j]] = (uint32_t)L;
+          queue[atomicAdd(&tail, 1)] = (uint32_t)nbr[j];
+        }
+    }
+    __syncthreads();
+    lo = hi;
+    hi = tail;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    depth[d] = L;
+    count[d] = lo;
   }
 }
 
-// The geometry stream: per plan item (in plan order) item_geometry's code word and the
-// distances r_f of the in-faces, in face order (at most three in-faces: the four outward
-// normals weighted by the face areas sum to zero).
-//   T = float: the distances as float, the values the sweep computes anyway.
-//   T = double: block floating point.  Only in-faces that some node of an out-face is traced
-//   to matter (the others are never read), and for those t = lam r_f is the distance from
-//   the node back to where its characteristic enters the cell, so r_f is at most six cell
-//   diameters.  With 2^(e-1) <= max r_f < 2^e over those faces, each is stored as
-//   round(r_f 2^(32-e)) in 32 bits and e in bits 24-31 of the code word (biased by 128):
-//   the error of every used distance is at most max r_f 2^-33, so an attenuation
-//   exp(-k t) moves by at most k (6 diameters) 2^-33 relative.
-template <class T>
-__global__ void k_plan_geometry(const uint32_t *items, int64_t n, int shift, int DB, int d0, const T *w,
-                                const T *rec, int RW, uint4 *geo) {
+// sort keys (direction << lbits | level) and cells of nd directions
+__global__ void k_plan_keys(int64_t N, int64_t total, int lbits, const uint32_t *level, uint32_t *key,
+                            uint32_t *cell) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t it = items[i];
-  const int64_t c = it & ((1u << shift) - 1u);
-  const int d = d0 + (int)(it >> shift);
-  T g[16];
-  int fid[4];
-  load_rec<T>(rec + (int64_t)RW * c, g, fid);
-  T r[4];
-  uint32_t code = item_geometry<T>(g, w[3 * d], w[3 * d + 1], w[3 * d + 2], r);
-  uint32_t q[3] = {0u, 0u, 0u};
-  if constexpr (sizeof(T) == 4) {
-    int m = 0;
+  if (i >= total) return;
+  const uint32_t x = (uint32_t)(i / N);
+  key[i] = x << lbits | level[i];
+  cell[i] = (uint32_t)(i - x * N);
+}
+
+// level offsets from the sorted keys of directions d0 .. (every level holds a cell)
+__global__ void k_plan_offsets(int64_t N, int64_t total, int lbits, int d0, const uint32_t *key,
+                               const int64_t *lvl_base, int32_t *lvl) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const int64_t x = i / N, k = i - x * N;
+  int32_t *o = lvl + lvl_base[d0 + x];
+  const uint32_t mask = (1u << lbits) - 1u, L = key[i] & mask;
+  if (k == 0 || (key[i - 1] & mask) != L) o[L] = (int32_t)k;
+  if (k == N - 1) o[L + 1] = (int32_t)N;
+}
+
+// Items of one direction per CTA in sweep order: face choice, distances and slots.  Within a
+// level the cells' own slots are taken first (from the free list, or a new one), then the
+// slots whose last reader sits in this level go back, so a slot is never written in a level
+// that reads it.  Slots below `cap` (those in shared memory) are preferred: the free list of
+// the low slots grows from the front of `freed`, that of the high ones from its end.  order [nd][N] cells in sweep order; slot_of, readers, freed [nd][N] scratch.
+template <class T>
+__global__ void __launch_bounds__(kPlanThreads)
+    k_plan_items(int64_t N, int d0, const T *w, const T *rec, const int32_t *lvl_all, const int64_t *lvl_base,
+                 const int32_t *depth, const uint32_t *order_all, uint32_t *slot_all, uint32_t *readers_all,
+                 uint32_t *freed_all, uint4 *ord_all, uint2 *hi_all, const T *wt, T *dist_all, T *wgt_all, T *wgt3_all,
+                 uint32_t cap, unsigned int *max_slots) {
+  __shared__ int top, next, htop, hnext;
+  const int x = blockIdx.x, d = d0 + x;
+  const uint32_t *order = order_all + x * N;
+  uint32_t *slot_of = slot_all + x * N, *readers = readers_all + x * N, *freed = freed_all + x * N;
+  uint4 *ord = ord_all + (int64_t)d * N;
+  uint2 *hi16 = hi_all ? hi_all + (int64_t)d * N : nullptr;
+  const int64_t at = (int64_t)d * N;
+  const int32_t *lvl = lvl_all + lvl_base[d];
+  const T wx = w[3 * d], wy = w[3 * d + 1], wz = w[3 * d + 2];
+  if (threadIdx.x == 0) top = htop = 0, next = 1, hnext = (int)cap;  // slot 0 is the boundary value
+  __syncthreads();
+  int lo = 0;
+  for (int L = 0; L < depth[d]; L++) {
+    const int hi = lvl[L + 1];
+    for (int i = lo + (int)threadIdx.x; i < hi; i += kPlanThreads) {
+      const int64_t c = order[i];
+      T g[16], cosf[4], tA, tB;
+      int nbr[4];
+      load_vec<T>(rec + c * Rec<T>::RW, g, 16);
+      load_nbr<T>(rec + c * Rec<T>::RW, nbr);
+      face_cos(g, wx, wy, wz, cosf);
+      const uint32_t code = item_geometry<T>(g, cosf, tA, tB);
+      uint32_t n = 0;
 #pragma unroll
-    for (int f = 0; f < 4; f++)
-      if ((code >> f) & 1u) {
-        const uint32_t v = __float_as_uint(r[f]);
-        if (m == 0) q[0] = v;
-        else if (m == 1) q[1] = v;
-        else q[2] = v;
-        m++;
+      for (int j = 0; j < 4; j++) n += (cosf[j] > 0 && nbr[j] >= 0) ? 1u : 0u;
+      uint32_t own = 0;
+      if (n) {
+        const int q = atomicSub(&top, 1) - 1;
+        if (q >= 0) {
+          own = freed[q];
+        } else {
+          own = (uint32_t)atomicAdd(&next, 1);
+          if (own >= cap) {
+            const int h = atomicSub(&htop, 1) - 1;
+            own = h >= 0 ? freed[N - 1 - h] : (uint32_t)atomicAdd(&hnext, 1);
+          }
+        }
+        slot_of[c] = own;
+        readers[c] = n;
       }
-  } else {
-    uint32_t used = 0;  // in-faces some node of an out-face is traced to
+      const int nin = (int)(code >> 6) & 3;
+      uint32_t s[3] = {0u, 0u, 0u};
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      if (!((code >> (4 + j)) & 1u)) continue;
-#pragma unroll
-      for (int qq = 0; qq < 3; qq++) {
-        const uint32_t cv = (code >> (8 + 4 * (((j + 1 + qq) & 3)))) & 15u;
-        if (!(cv & 8u)) used |= 1u << (cv & 3u);
+      for (int q = 0; q < 3; q++) {
+        const int f = (int)(code >> (2 * q)) & 3;
+        const int b = f == 0 ? nbr[0] : f == 1 ? nbr[1] : f == 2 ? nbr[2] : nbr[3];
+        if (q < nin && b >= 0) s[q] = slot_of[b];
+      }
+      ord[i] = make_uint4((uint32_t)c, code, (own & 0xffffu) | s[0] << 16, (s[1] & 0xffffu) | s[2] << 16);
+      if (hi16) hi16[i] = make_uint2(own >> 16 | (s[0] & 0xffff0000u), s[1] >> 16 | (s[2] & 0xffff0000u));
+      if (dist_all) {
+        T wq[3];
+        in_weights(wt + 4 * c, code, wq);
+        dist_all[2 * (at + i)] = tA;
+        dist_all[2 * (at + i) + 1] = tB;
+        wgt_all[2 * (at + i)] = wq[0];
+        wgt_all[2 * (at + i) + 1] = wq[1];
+        wgt3_all[at + i] = wq[2];
       }
     }
-    double rmax = 0.0;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      top = max(top, 0);
+      htop = max(htop, 0);
+      next = min(next, (int)cap);
+    }
+    __syncthreads();
+    for (int i = lo + (int)threadIdx.x; i < hi; i += kPlanThreads) {
+      const int64_t c = order[i];
+      T g[12], cosf[4];
+      int nbr[4];
+      load_vec<T>(rec + c * Rec<T>::RW, g, 12);
+      load_nbr<T>(rec + c * Rec<T>::RW, nbr);
+      face_cos(g, wx, wy, wz, cosf);
 #pragma unroll
-    for (int f = 0; f < 4; f++)
-      if ((used >> f) & 1u) rmax = fmax(rmax, (double)r[f]);
-    const int e = rmax > 0.0 ? max(-127, min(127, ilogb(rmax) + 1)) : 0;
-    const double up = ldexp(1.0, 32 - e);
-    int m = 0;
-#pragma unroll
-    for (int f = 0; f < 4; f++)
-      if ((code >> f) & 1u) {
-        const uint32_t v = ((used >> f) & 1u) ? (uint32_t)fmin(rint((double)r[f] * up), 4294967295.0) : 0u;
-        if (m == 0) q[0] = v;
-        else if (m == 1) q[1] = v;
-        else q[2] = v;
-        m++;
-      }
-    code |= (uint32_t)(e + 128) << 24;
+      for (int j = 0; j < 4; j++)
+        if (cosf[j] < 0 && nbr[j] >= 0 && atomicSub(readers + nbr[j], 1u) == 1u) {
+          const uint32_t q = slot_of[nbr[j]];
+          if (q < cap)
+            freed[atomicAdd(&top, 1)] = q;
+          else
+            freed[N - 1 - atomicAdd(&htop, 1)] = q;
+        }
+    }
+    lo = hi;
+    __syncthreads();
   }
-  geo[i] = make_uint4(code, q[0], q[1], q[2]);
+  if (threadIdx.x == 0) {
+    atomicMax(max_slots, (unsigned int)next);
+    atomicMax(max_slots + 1, (unsigned int)hnext);
+  }
 }
 
 // Source record {k = alpha + betta, betta / k, alpha Q_g / k} of each context cell
 // (rhs_g = alpha Q_g / k + (betta / k) S_g, GetRhsOpt with the division by k
 // distributed) from caller arrays (caller numbering) ...
 template <class T, class TA>
-__global__ void k_dyn_from_arrays(int64_t N, int G, int RW, const int32_t *perm, const TA *alpha, const TA *betta,
-                                  const TA *Q, T *rec) {
+__global__ void k_dyn_from_arrays(int64_t N, int G, int SW, const int32_t *perm, const TA *alpha, const TA *betta,
+                                  const TA *Q, T *src) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= N) return;
   const int64_t p = perm[c];
   const T al = (T)alpha[p], be = (T)betta[p];
-  T *o = rec + (int64_t)RW * c + Rec<T>::DYN;
+  T *o = src + (int64_t)SW * c;
   const T k = al + be;
   o[0] = k;
   o[1] = be / k;
-  for (int g = 0; g < G; g++) o[2 + g] = (al * (T)Q[p * G + g]) / k;
+  for (int g = 0; g < G; g++) o[kSrcQ + g] = (al * (T)Q[p * G + g]) / k;
 }
 
 // ... or from the solver state: alpha = a rho, betta = b rho, Q_g = B(T) / kRadiation / G.
 template <class T>
-__global__ void k_dyn_from_state(int64_t N, int G, int RW, const double *state, double a_coef, double b_coef,
-                                 Emission em, T *rec) {
+__global__ void k_dyn_from_state(int64_t N, int G, int SW, const double *state, double a_coef, double b_coef,
+                                 Emission em, T *src) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= N) return;
   const double rho = state[10 * c + 5], prs = state[10 * c + 9];
   const T al = (T)(a_coef * rho), be = (T)(b_coef * rho);
   const T q = (T)(planck_B(em, rho, prs) / em.rad_unit / (double)G);
-  T *o = rec + (int64_t)RW * c + Rec<T>::DYN;
+  T *o = src + (int64_t)SW * c;
   const T k = al + be;
   o[0] = k;
   o[1] = be / k;
-  const T aq = (al * q) / k;
-  for (int g = 0; g < G; g++) o[2 + g] = aq;
+  o[kSrcQ] = (al * q) / k;
 }
 
 // ---------------------------------------------------------------- coupled step
@@ -790,173 +802,305 @@ Eos eos_of(const rrhd_ctx *c) {
   return e;
 }
 
-template <class T>
-rrhd_status build_plan(rrhd_ctx *c) {
+// ---------------------------------------------------------------- launches
+// Shared memory of a sweep's CTA: two CTAs of 256 threads per SM while the slots of every
+// direction fit half an SM (the one works while the other waits at its level's barrier), else
+// one of 512 threads, with the slots beyond its shared memory in global memory.
+constexpr int kSweepSMs = 148, kSmemTwo = 112 * 1024, kSmemOne = 226 * 1024;
+
+uint32_t slot_cap(const RadState &R) {  // slots a CTA's shared memory can hold
+  const size_t tv = R.prec == RRHD_RAD_FP32 ? sizeof(float) : sizeof(double);
+  return (uint32_t)(kSmemOne / (tv * R.G));
+}
+
+template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB>
+cudaError_t launch_sweep_kernel(const SweepArgs<T, TI> &a, int nd, size_t smem, cudaStream_t st) {
+  auto *k = k_sweep<T, TI, GT, HIGH, WIDE, GEO, NT, NB>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k<<<nd, NT, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <class T, class TI, int GT, bool HIGH, bool WIDE, int NT, int NB>
+cudaError_t launch_sweep_geo(const SweepArgs<T, TI> &a, int nd, size_t smem, cudaStream_t st) {
+  return a.dist ? launch_sweep_kernel<T, TI, GT, HIGH, WIDE, true, NT, NB>(a, nd, smem, st)
+                : launch_sweep_kernel<T, TI, GT, HIGH, WIDE, false, NT, NB>(a, nd, smem, st);
+}
+
+template <class T, class TI, int GT>
+cudaError_t launch_sweep_groups(const SweepArgs<T, TI> &a, int64_t low, bool two, int nd, cudaStream_t st) {
+  const size_t smem = sizeof(T) * (size_t)low * a.G;
+  if (two && !a.nhigh && smem <= kSmemTwo) return launch_sweep_geo<T, TI, GT, false, false, 256, 2>(a, nd, smem, st);
+  if (a.ord_hi) return launch_sweep_geo<T, TI, GT, true, true, 512, 1>(a, nd, smem, st);
+  if (a.nhigh) return launch_sweep_geo<T, TI, GT, true, false, 512, 1>(a, nd, smem, st);
+  return launch_sweep_geo<T, TI, GT, false, false, 512, 1>(a, nd, smem, st);
+}
+
+// directions d0 .. d0 + nd - 1; S and I: element (cell, d0 + x, group) at cell * sc + x * sd + group
+template <class T, class TI>
+rrhd_status launch_sweep(rrhd_ctx *c, int d0, int nd, const void *S, void *I, int64_t sc, int64_t sd, bool one_q) {
   RadState &R = c->rad;
-  const int64_t N = c->N;
-  const int64_t total = N * (int64_t)R.M;
-  cudaStream_t st = c->stream;
-  uint32_t *indeg = nullptr, *tmp = nullptr;
-  unsigned long long *d_tail = nullptr;
-  void *sort_tmp = nullptr;
-  size_t sort_bytes = 0;
-  auto cleanup = [&]() {
-    cudaFree(indeg);
-    cudaFree(tmp);
-    cudaFree(d_tail);
-    cudaFree(sort_tmp);
-  };
-  const int64_t bmax = N * (int64_t)R.DB;
-  if (cudaMalloc(&R.d_plan, sizeof(uint32_t) * total) != cudaSuccess ||
-      cudaMalloc(&indeg, sizeof(uint32_t) * bmax) != cudaSuccess ||
-      cudaMalloc(&tmp, sizeof(uint32_t) * bmax) != cudaSuccess ||
-      cudaMalloc(&d_tail, sizeof(unsigned long long)) != cudaSuccess) {
-    cleanup();
-    return rrhd_fail(RRHD_ERR_OOM, "sweep plan allocation failed");
+  SweepArgs<T, TI> a;
+  a.N = c->N;
+  a.d0 = d0;
+  a.G = R.G;
+  a.ord = R.d_ord;
+  a.ord_hi = R.d_ord_hi;
+  a.dist = (const T *)R.d_dist;
+  a.wgt = (const T *)R.d_wgt;
+  a.wgt3 = (const T *)R.d_wgt3;
+  a.qs = one_q ? 0 : 1;
+  a.SW = one_q ? 4 : R.SW;
+  a.wt = (const T *)R.d_wt;
+  a.rec = (const T *)R.d_rec;
+  a.w = (const T *)R.d_w;
+  a.lvl = R.d_lvl;
+  a.lvl_base = R.d_lvl_base;
+  a.depth = R.d_depth;
+  a.src = (const T *)R.d_src;
+  a.slots = (T *)R.d_slots;
+  a.cap = slot_cap(R);
+  a.nhigh = R.nhigh;
+  a.S = (const TI *)S;
+  a.I = (TI *)I;
+  a.sc = sc;
+  a.sd = sd;
+  a.bc = (T)R.bc;
+  cudaError_t e;
+  switch (R.G) {
+    case 1: e = launch_sweep_groups<T, TI, 1>(a, R.nlow, R.M > kSweepSMs, nd, c->stream); break;
+    case 2: e = launch_sweep_groups<T, TI, 2>(a, R.nlow, R.M > kSweepSMs, nd, c->stream); break;
+    case 4: e = launch_sweep_groups<T, TI, 4>(a, R.nlow, R.M > kSweepSMs, nd, c->stream); break;
+    default: e = launch_sweep_groups<T, TI, 0>(a, R.nlow, R.M > kSweepSMs, nd, c->stream); break;
   }
-  int db_bits = 0;
-  while ((1 << db_bits) < R.DB) db_bits++;
-  const int end_bit = R.shift + db_bits;
-  cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, (const uint32_t *)nullptr, (uint32_t *)nullptr, bmax, 0,
-                                 end_bit, st);
-  if (cudaMalloc(&sort_tmp, sort_bytes) != cudaSuccess) {
-    cleanup();
-    return rrhd_fail(RRHD_ERR_OOM, "sweep plan allocation failed");
-  }
-  R.lvl.assign(R.nbatch, {});
-  R.levels = 0;
-  R.max_level = 0;
-  int64_t base = 0;
-  for (int b = 0; b < R.nbatch; b++) {
-    const int d0 = b * R.DB;
-    const int nbd = std::min(R.DB, R.M - d0);
-    uint32_t *plan = R.d_plan + base;
-    const unsigned long long zero = 0;
-    RRHD_CUDA(cudaMemcpyAsync(d_tail, &zero, sizeof zero, cudaMemcpyHostToDevice, st));
-    k_plan_init<T><<<grid_for(N * nbd, 256), 256, 0, st>>>(N, nbd, R.shift, d0, (const T *)R.d_w,
-                                                            (const T *)R.d_rec, R.RW, indeg, plan, d_tail);
-    RRHD_CUDA(cudaGetLastError());
-    std::vector<int64_t> &off = R.lvl[b];
-    off.assign(1, 0);
-    int64_t lo = 0;
-    for (;;) {
-      unsigned long long hi_u = 0;
-      RRHD_CUDA(cudaMemcpyAsync(&hi_u, d_tail, sizeof hi_u, cudaMemcpyDeviceToHost, st));
-      RRHD_CUDA(cudaStreamSynchronize(st));
-      const int64_t hi = (int64_t)hi_u;
-      if (hi == lo) break;
-      // items of a level in ascending (direction, cell) order: deterministic launches,
-      // and the items of one direction in cell order, so that neighbouring cells' face
-      // slots (direction-major) and records are read close together
-      cub::DeviceRadixSort::SortKeys(sort_tmp, sort_bytes, plan + lo, tmp, hi - lo, 0, end_bit, st);
-      RRHD_CUDA(cudaMemcpyAsync(plan + lo, tmp, sizeof(uint32_t) * (hi - lo), cudaMemcpyDeviceToDevice, st));
-      off.push_back(hi);
-      R.max_level = std::max(R.max_level, hi - lo);
-      k_plan_expand<T><<<grid_for(hi - lo, 256), 256, 0, st>>>(plan + lo, hi - lo, nbd, R.shift, d0,
-                                                                (const T *)R.d_w, (const T *)R.d_rec, R.RW,
-                                                                indeg, plan, d_tail);
-      RRHD_CUDA(cudaGetLastError());
-      lo = hi;
-    }
-    if (lo != N * nbd) {
-      cleanup();
-      return rrhd_fail(RRHD_ERR_STATE, "sweep dependency cycle: %lld of %lld (cell, direction) pairs of batch %d "
-                                       "have an upwind neighbour that depends on them",
-                       (long long)(N * nbd - lo), (long long)(N * nbd), b);
-    }
-    R.levels += (int64_t)off.size() - 1;
-    base += N * nbd;
-  }
-  cleanup();
+  RRHD_CUDA(e);
   return RRHD_OK;
 }
 
-template <class T, class TV, class TI, int GT, bool PRE>
-cudaError_t launch_level(const SweepArgs<T, TV> &a, unsigned nb, cudaStream_t st, bool pdl) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nb);
-  cfg.blockDim = dim3(kSweepThreads);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_sweep_level<T, TV, TI, GT, PRE>, a);
+template <class V, bool IMPORT>
+cudaError_t launch_tile(rrhd_ctx *c, int64_t rows, int d0, int nd, const int32_t *perm, const void *in, void *out) {
+  const dim3 tiles((unsigned)((rows + 31) / 32), (unsigned)((nd + 31) / 32));
+  k_tile<V, IMPORT><<<tiles, 256, 0, c->stream>>>(rows, c->rad.G, c->rad.M, d0, nd, perm, (const V *)in, (V *)out);
+  return cudaGetLastError();
 }
 
-// the geometry stream exists for the float-intensity forms only (its distances are float)
-template <class T, class TV, class TI, int GT>
-cudaError_t launch_level_any(const SweepArgs<T, TV> &a, unsigned nb, cudaStream_t st, bool pdl) {
-  if constexpr (sizeof(TI) == 4) {
-    if (a.geo) return launch_level<T, TV, TI, GT, true>(a, nb, st, pdl);
+struct alignas(8) Bytes8 { uint32_t w[2]; };
+struct alignas(16) Bytes16 { uint32_t w[4]; };
+struct alignas(16) Bytes32 { uint32_t w[8]; };
+
+// S or I between the caller's arrays (rows, or [N][M][G] when cdg) and the sweep's layout
+template <class TI, bool IMPORT>
+cudaError_t move_tiles(rrhd_ctx *c, int d0, int nd, const void *in, void *out, bool cdg) {
+  const RadState &R = c->rad;
+  const int64_t N = c->N;
+  if (!cdg) return launch_tile<TI, IMPORT>(c, N * R.G, d0, nd, c->d_perm, in, out);
+  switch (sizeof(TI) * R.G) {
+    case 4: return launch_tile<float, IMPORT>(c, N, d0, nd, nullptr, in, out);
+    case 8: return launch_tile<Bytes8, IMPORT>(c, N, d0, nd, nullptr, in, out);
+    case 16: return launch_tile<Bytes16, IMPORT>(c, N, d0, nd, nullptr, in, out);
+    case 32: return launch_tile<Bytes32, IMPORT>(c, N, d0, nd, nullptr, in, out);
+    default: return cudaErrorNotSupported;
   }
-  return launch_level<T, TV, TI, GT, false>(a, nb, st, pdl);
 }
 
-template <class T, class TV, class TI>
-rrhd_status capture_sweep(rrhd_ctx *c) {
+// One sweep of every direction: S and I [N][M][G] in context numbering (cdg), or [N*G][M] in
+// caller numbering, through the scratch of R.xdirs directions, swept in place there.
+template <class T, class TI>
+rrhd_status run_sweep_t(rrhd_ctx *c, const void *S, void *I, bool cdg) {
   RadState &R = c->rad;
-  cudaStream_t cs = nullptr;
-  RRHD_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-  cudaGraph_t g = nullptr;
-  cudaError_t launch_err = cudaSuccess;
-  cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-  if (e == cudaSuccess) {
-    SweepArgs<T, TV> a;
-    a.io = R.d_io;
-    a.shift = R.shift;
-    a.DB = R.DB;
-    a.M = R.M;
-    a.G = R.G;
-    a.RW = R.RW;
-    a.w = (const T *)R.d_w;
-    a.rec = (const T *)R.d_rec;
-    a.area = (const T *)R.d_area;
-    a.fv = (TV *)R.d_fv;
-    a.NF = c->F;
-    a.geo = nullptr;
-    a.bc = (TV)R.bc;
-    a.last = R.last_cell;
-    a.GS = R.GS;
-    int64_t base = 0;
-    for (int b = 0; b < R.nbatch; b++) {
-      a.d0 = b * R.DB;
-      const int nbd = std::min(R.DB, R.M - a.d0);
-      a.nbd = nbd;
-      const std::vector<int64_t> &off = R.lvl[b];
-      for (size_t L = 0; L + 1 < off.size(); L++) {
-        a.items = R.d_plan + base + off[L];
-        a.n = off[L + 1] - off[L];
-        const unsigned nb = grid_for(a.n, kSweepThreads);
-        const bool pdl = L > 0;  // the first level of a batch follows a full dependency
-        cudaError_t le;
-        a.geo = R.d_geo ? R.d_geo + base + off[L] : nullptr;
-        switch (R.G) {
-          case 1: le = launch_level_any<T, TV, TI, 1>(a, nb, cs, pdl); break;
-          case 2: le = launch_level_any<T, TV, TI, 2>(a, nb, cs, pdl); break;
-          case 4: le = launch_level_any<T, TV, TI, 4>(a, nb, cs, pdl); break;
-          default: le = launch_level_any<T, TV, TI, 0>(a, nb, cs, pdl); break;
-        }
-        if (le != cudaSuccess && launch_err == cudaSuccess) launch_err = le;
-      }
-      const dim3 nr((unsigned)((c->N + kRcCells - 1) / kRcCells), (unsigned)((nbd + kRcDirs - 1) / kRcDirs));
-      switch (R.G) {
-        case 1: k_recalc<T, TV, TI, 1><<<nr, 256, 0, cs>>>(a, c->N); break;
-        case 2: k_recalc<T, TV, TI, 2><<<nr, 256, 0, cs>>>(a, c->N); break;
-        case 4: k_recalc<T, TV, TI, 4><<<nr, 256, 0, cs>>>(a, c->N); break;
-        default: k_recalc<T, TV, TI, 0><<<nr, 256, 0, cs>>>(a, c->N); break;
-      }
-      base += c->N * nbd;
+  const int64_t rows = c->N * R.G;
+  const size_t cd = sizeof(TI) * R.G;  // bytes of a (cell, direction)
+  if (cdg && !(cd == 4 || cd == 8 || cd == 16 || cd == 32))
+    return launch_sweep<T, TI>(c, 0, R.M, S, I, (int64_t)R.M * R.G, R.G, true);
+  if (!R.d_x) {
+    // as many directions as there are, or as memory allows (at least one)
+    R.xdirs = R.M;
+    while (cudaMalloc(&R.d_x, sizeof(TI) * (size_t)rows * R.xdirs) != cudaSuccess) {
+      cudaGetLastError();
+      R.d_x = nullptr;
+      if (R.xdirs == 1) return rrhd_fail(RRHD_ERR_OOM, "sweep scratch allocation failed");
+      R.xdirs = (R.xdirs + 1) / 2;
     }
-    e = cudaStreamEndCapture(cs, &g);
   }
-  if (e == cudaSuccess) e = launch_err;
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&R.graph, g, 0);
-  if (g) cudaGraphDestroy(g);
-  cudaStreamDestroy(cs);
-  RRHD_CUDA(e);
+  for (int d0 = 0; d0 < R.M; d0 += R.xdirs) {
+    const int nd = std::min(R.xdirs, R.M - d0);
+    RRHD_CUDA((move_tiles<TI, true>(c, d0, nd, S, R.d_x, cdg)));
+    const rrhd_status s = launch_sweep<T, TI>(c, d0, nd, R.d_x, R.d_x, R.G, rows, cdg);
+    if (s) return s;
+    RRHD_CUDA((move_tiles<TI, false>(c, d0, nd, R.d_x, I, cdg)));
+  }
+  return RRHD_OK;
+}
+
+rrhd_status run_sweep(rrhd_ctx *c, const void *S, void *I, bool cdg) {
+  switch (c->rad.prec) {
+    case RRHD_RAD_FP64: return run_sweep_t<double, double>(c, S, I, cdg);
+    case RRHD_RAD_MIXED: return run_sweep_t<double, float>(c, S, I, cdg);
+    default: return run_sweep_t<float, float>(c, S, I, cdg);
+  }
+}
+
+// ---------------------------------------------------------------- plan, host side
+struct Scratch {  // device memory of the plan build, freed on every way out
+  std::vector<void *> p;
+  ~Scratch() {
+    for (void *q : p) cudaFree(q);
+  }
+  void *get(size_t bytes) {
+    void *q = nullptr;
+    if (cudaMalloc(&q, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    p.push_back(q);
+    return q;
+  }
+};
+
+int bits_for(int64_t n) {  // bits that hold 0 .. n - 1
+  int b = 0;
+  while ((int64_t(1) << b) < n) b++;
+  return b;
+}
+
+// The sweep order, items and slots of every direction (R.d_ord, the geometry stream, level offsets).
+template <class T>
+rrhd_status build_plan(rrhd_ctx *c) {
+  RadState &R = c->rad;
+  const int64_t N = c->N, total = N * (int64_t)R.M;
+  cudaStream_t st = c->stream;
+  const rrhd_status oom = RRHD_ERR_OOM;
+  if (cudaMalloc(&R.d_ord, sizeof(uint4) * total) != cudaSuccess) {
+    cudaGetLastError();
+    R.d_ord = nullptr;
+    return rrhd_fail(oom, "sweep plan allocation failed (%lld bytes)", (long long)(sizeof(uint4) * total));
+  }
+  // The geometry stream (5 values an item) spares each item its cell's geometry record.  It
+  // is kept where the memory left holds it beside the intensity and scattering-integral
+  // arrays of a coupled step (or of a caller's sweep with its scratch); else the sweep forms
+  // the same values again from the records.
+  {
+    size_t free_b = 0, all_b = 0;
+    RRHD_CUDA(cudaMemGetInfo(&free_b, &all_b));
+    const size_t one = sizeof(T) * (size_t)total;
+    const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
+    const size_t arrays = 3 * ti * (size_t)total * R.G;
+    if (5 * one + arrays <= free_b &&
+        (cudaMalloc(&R.d_dist, 2 * one) != cudaSuccess || cudaMalloc(&R.d_wgt, 2 * one) != cudaSuccess ||
+         cudaMalloc(&R.d_wgt3, one) != cudaSuccess)) {
+      cudaGetLastError();
+      for (void **p : {&R.d_dist, &R.d_wgt, &R.d_wgt3}) {
+        cudaFree(*p);
+        *p = nullptr;
+      }
+    }
+  }
+  // directions of a build pass: six 32-bit words a pair in at most half of the free memory
+  size_t free_b = 0, all_b = 0;
+  RRHD_CUDA(cudaMemGetInfo(&free_b, &all_b));
+  int B = (int)std::max<int64_t>(1, std::min<int64_t>(R.M, (int64_t)(free_b / 2) / (28 * N)));
+  Scratch mem;
+  uint32_t *buf[6];
+  for (uint32_t *&b : buf)
+    if (!(b = (uint32_t *)mem.get(sizeof(uint32_t) * (size_t)N * B))) return rrhd_fail(oom, "sweep plan scratch");
+  uint32_t *const level = buf[0], *const key = buf[1], *const cell = buf[2], *const key2 = buf[3],
+           *const order = buf[4], *const indeg = buf[5], *const queue = key;
+  int32_t *d_count = (int32_t *)mem.get(sizeof(int32_t) * R.M);
+  unsigned int *d_max = (unsigned int *)mem.get(2 * sizeof(unsigned int));
+  if (!d_count || !d_max || cudaMalloc(&R.d_depth, sizeof(int32_t) * R.M) != cudaSuccess ||
+      cudaMalloc(&R.d_lvl_base, sizeof(int64_t) * R.M) != cudaSuccess)
+    return rrhd_fail(oom, "sweep plan scratch");
+  size_t sort_bytes = 0;
+  RRHD_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, key, key2, cell, order, N * B, 0, 32, st));
+  void *sort_tmp = mem.get(sort_bytes);
+  if (!sort_tmp) return rrhd_fail(oom, "sweep plan scratch");
+  RRHD_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned int), st));
+  R.depth.assign(R.M, 0);
+  R.lvl_base.assign(R.M, 0);
+  std::vector<int32_t> count(R.M);
+  const T *w = (const T *)R.d_w, *rec = (const T *)R.d_rec;
+  // levels of every direction first: their number decides the sort keys and the offsets
+  auto levels_of = [&](int d0, int nd) -> rrhd_status {
+    k_plan_levels<T><<<nd, kPlanThreads, 0, st>>>(N, d0, w, rec, indeg, queue, level, R.d_depth, d_count);
+    RRHD_CUDA(cudaGetLastError());
+    RRHD_CUDA(cudaMemcpyAsync(R.depth.data() + d0, R.d_depth + d0, sizeof(int32_t) * nd, cudaMemcpyDeviceToHost, st));
+    RRHD_CUDA(cudaMemcpyAsync(count.data() + d0, d_count + d0, sizeof(int32_t) * nd, cudaMemcpyDeviceToHost, st));
+    RRHD_CUDA(cudaStreamSynchronize(st));
+    return RRHD_OK;
+  };
+  rrhd_status s;
+  for (int d0 = 0; d0 < R.M; d0 += B)
+    if ((s = levels_of(d0, std::min(B, R.M - d0)))) return s;
+  int64_t entries = 0;
+  for (int d = 0; d < R.M; d++) {
+    if (count[d] != N)
+      return rrhd_fail(RRHD_ERR_STATE, "sweep dependency cycle: %lld of %lld cells have, in direction %d, an upwind "
+                                       "neighbour that depends on them", (long long)(N - count[d]), (long long)N, d);
+    R.lvl_base[d] = entries;
+    entries += R.depth[d] + 1;
+  }
+  if (cudaMalloc(&R.d_lvl, sizeof(int32_t) * entries) != cudaSuccess) {
+    cudaGetLastError();
+    R.d_lvl = nullptr;
+    return rrhd_fail(oom, "sweep plan allocation failed");
+  }
+  RRHD_CUDA(cudaMemcpyAsync(R.d_lvl_base, R.lvl_base.data(), sizeof(int64_t) * R.M, cudaMemcpyHostToDevice, st));
+  for (int d0 = 0; d0 < R.M; d0 += B) {
+    const int nd = std::min(B, R.M - d0);
+    if (B < R.M && (s = levels_of(d0, nd))) return s;  // the scratch held another batch's levels
+    const int lbits = std::max(1, bits_for(*std::max_element(R.depth.begin() + d0, R.depth.begin() + d0 + nd)));
+    // directions per sort: its keys are 32-bit
+    const int ns = (int)std::min<int64_t>(nd, lbits < 31 ? int64_t(1) << (32 - lbits) : 1);
+    for (int x = 0; x < nd; x += ns) {
+      const int n = std::min(ns, nd - x);
+      const int64_t at = N * x, pairs = N * n;
+      k_plan_keys<<<grid_for(pairs, 256), 256, 0, st>>>(N, pairs, lbits, level + at, key + at, cell + at);
+      RRHD_CUDA(cudaGetLastError());
+      RRHD_CUDA(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, key + at, key2 + at, cell + at, order + at,
+                                                pairs, 0, std::min(32, lbits + bits_for(n)), st));
+      k_plan_offsets<<<grid_for(pairs, 256), 256, 0, st>>>(N, pairs, lbits, d0 + x, key2 + at, R.d_lvl_base, R.d_lvl);
+      RRHD_CUDA(cudaGetLastError());
+    }
+    auto items = [&]() -> rrhd_status {
+      k_plan_items<T><<<nd, kPlanThreads, 0, st>>>(N, d0, w, rec, R.d_lvl, R.d_lvl_base, R.d_depth, order, indeg, key,
+                                                   cell, R.d_ord, R.d_ord_hi, (const T *)R.d_wt, (T *)R.d_dist, (T *)R.d_wgt,
+                                                   (T *)R.d_wgt3, slot_cap(R), d_max);
+      RRHD_CUDA(cudaGetLastError());
+      unsigned int m[2] = {0, 0};
+      RRHD_CUDA(cudaMemcpyAsync(m, d_max, sizeof m, cudaMemcpyDeviceToHost, st));
+      RRHD_CUDA(cudaStreamSynchronize(st));
+      R.nlow = m[0];
+      R.nhigh = (int64_t)m[1] - slot_cap(R);
+      return RRHD_OK;
+    };
+    if ((s = items())) return s;
+    if (std::max(R.nlow, slot_cap(R) + R.nhigh) > 65536 && !R.d_ord_hi) {
+      // slots beyond 16 bits: their upper halves in a second array (zero for the batches before)
+      if (cudaMalloc(&R.d_ord_hi, sizeof(uint2) * total) != cudaSuccess) {
+        cudaGetLastError();
+        R.d_ord_hi = nullptr;
+        return rrhd_fail(oom, "sweep plan allocation failed");
+      }
+      RRHD_CUDA(cudaMemsetAsync(R.d_ord_hi, 0, sizeof(uint2) * total, st));
+      if ((s = items())) return s;
+    }
+  }
+  // rrhd_rad_plan_info: levels and the largest level over batches of R.DB directions
+  std::vector<int32_t> off((size_t)entries);
+  RRHD_CUDA(cudaMemcpyAsync(off.data(), R.d_lvl, sizeof(int32_t) * entries, cudaMemcpyDeviceToHost, st));
+  RRHD_CUDA(cudaStreamSynchronize(st));
+  R.levels = R.max_level = 0;
+  for (int d0 = 0; d0 < R.M; d0 += R.DB) {
+    std::vector<int64_t> items;
+    for (int d = d0; d < std::min(R.M, d0 + R.DB); d++) {
+      const int32_t *o = off.data() + R.lvl_base[d];
+      if ((int)items.size() < R.depth[d]) items.resize(R.depth[d], 0);
+      for (int L = 0; L < R.depth[d]; L++) items[L] += o[L + 1] - o[L];
+    }
+    R.levels += (int64_t)items.size();
+    for (int64_t n : items) R.max_level = std::max(R.max_level, n);
+  }
   return RRHD_OK;
 }
 
@@ -964,9 +1108,9 @@ rrhd_status capture_sweep(rrhd_ctx *c) {
 
 void rrhd_rad_release(rrhd_ctx *c) {
   RadState &R = c->rad;
-  if (R.graph) cudaGraphExecDestroy(R.graph);
-  void *ptrs[] = {R.d_w, R.d_rec, R.d_area, R.d_plan, R.d_geo, R.d_io, R.d_fv, R.d_I, R.d_S, R.d_G4, R.d_mE, R.d_mF,
-                  R.d_mT, R.d_mom, R.d_cnt};
+  void *ptrs[] = {R.d_w,     R.d_rec, R.d_src, R.d_ord, R.d_ord_hi, R.d_dist, R.d_wgt, R.d_wgt3, R.d_wt, R.d_lvl, R.d_lvl_base, R.d_depth,
+                  R.d_slots, R.d_x,   R.d_I,   R.d_S,   R.d_G4,     R.d_mE,  R.d_mF,  R.d_mT,       R.d_mom,
+                  R.d_cnt};
   for (void *p : ptrs) cudaFree(p);
   for (cudaEvent_t e : R.ev)
     if (e) cudaEventDestroy(e);
@@ -975,31 +1119,21 @@ void rrhd_rad_release(rrhd_ctx *c) {
   R = RadState();
 }
 
-// T: the records (geometry, opacities and sources) and directions; TV: the face values
-// and the transport arithmetic; TI: the intensity and scattering-integral arrays the
-// sweep reads and writes.
-template <class T, class TV, class TI>
+// T: the records (geometry, opacities and sources), directions, slots and arithmetic.
+template <class T>
 static rrhd_status rad_setup_t(rrhd_ctx *c) {
   RadState &R = c->rad;
   const int64_t N = c->N;
-  const int W = ((Rec<T>::DYN + 2 + R.G + Rec<T>::NBRW + Rec<T>::LINE - 1) / Rec<T>::LINE) * Rec<T>::LINE;
-  R.RW = W;
-  std::vector<T> rec((size_t)W * N, (T)0), area(4 * (size_t)N), w(3 * R.M);
+  constexpr int W = Rec<T>::RW;
+  R.SW = (kSrcQ + R.G + 3) / 4 * 4;
+  std::vector<T> rec((size_t)W * N, (T)0), wt((size_t)4 * N), w(3 * R.M);
   std::vector<int32_t> iperm(N);
   for (int64_t i = 0; i < N; i++) iperm[c->h_perm[i]] = (int32_t)i;
-  // face-value slots numbered in order of first use by context cells, so that the
-  // faces of neighbouring cells sit close together
-  std::vector<int32_t> fslot(c->F, -1);
-  int32_t nslot = 0;
-  for (int64_t cn = 0; cn < N; cn++)
-    for (int j = 0; j < 4; j++) {
-      const int32_t fc = c->h_cell_faces[4 * c->h_perm[cn] + j];
-      if (fslot[fc] < 0) fslot[fc] = nslot++;
-    }
   for (int64_t cn = 0; cn < N; cn++) {
     const int64_t p = c->h_perm[cn];
     T *r = rec.data() + (size_t)W * cn;
-    int32_t ids[8];
+    int32_t nbr[4];
+    double area = 0.0;
     for (int j = 0; j < 4; j++) {
       const int32_t fc = c->h_cell_faces[4 * p + j];
       const bool out = (c->h_cell_sign[p] >> j) & 1;
@@ -1008,51 +1142,49 @@ static rrhd_status rad_setup_t(rrhd_ctx *c) {
         r[3 * j + x] = (T)(out ? v : -v);
       }
       r[12 + j] = (T)(3.0 * c->h_cell_V[p] / c->h_face_area[fc]);
-      area[4 * cn + j] = (T)c->h_face_area[fc];
+      area += c->h_face_area[fc];
       const int32_t l = c->h_face_l[fc], rr = c->h_face_r[fc];
       const int32_t o = (l == p) ? rr : l;
-      ids[j] = o < 0 ? (fslot[fc] | kNoNeighbour) : fslot[fc];
-      ids[4 + j] = o < 0 ? -1 : iperm[o];
+      nbr[j] = o < 0 ? -1 : iperm[o];
     }
-    std::memcpy(r + Rec<T>::IDS, ids, 4 * sizeof(int32_t));
-    std::memcpy(r + W - Rec<T>::NBRW, ids + 4, 4 * sizeof(int32_t));
+    std::memcpy(r + Rec<T>::NBR, nbr, sizeof nbr);
+    // ReCalcIllumOpt (illum_utils.cpp:415-430): the plain mean for the caller's last cell
+    for (int j = 0; j < 4; j++)
+      wt[4 * cn + j] = p == N - 1 ? (T)0.25 : (T)(c->h_face_area[c->h_cell_faces[4 * p + j]] / area);
   }
   for (int q = 0; q < 3 * R.M; q++) w[q] = (T)R.dirs->h_w[q];
-  R.last_cell = iperm[N - 1];
-  R.GS = sizeof(TV) == 8 ? ((R.G + 3) & ~3) : ((R.G + 7) & ~7);
-  auto up = [&](void **dst, const void *src, size_t bytes) -> rrhd_status {
-    if (cudaMalloc(dst, bytes) != cudaSuccess) return rrhd_fail(RRHD_ERR_OOM, "sweep allocation failed");
-    RRHD_CUDA(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
+  auto up = [&](void **dst, const void *from, size_t bytes) -> rrhd_status {
+    if (cudaMalloc(dst, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      *dst = nullptr;
+      return rrhd_fail(RRHD_ERR_OOM, "sweep allocation failed");
+    }
+    RRHD_CUDA(cudaMemcpy(*dst, from, bytes, cudaMemcpyHostToDevice));
     return RRHD_OK;
   };
   rrhd_status s;
   if ((s = up(&R.d_rec, rec.data(), sizeof(T) * rec.size())) || (s = up(&R.d_w, w.data(), sizeof(T) * w.size())) ||
-      (s = up(&R.d_area, area.data(), sizeof(T) * area.size())))
+      (s = up(&R.d_wt, wt.data(), sizeof(T) * wt.size())))
     return s;
-  if (cudaMalloc(&R.d_io, sizeof(SweepIO)) != cudaSuccess ||
-      cudaMalloc(&R.d_fv, sizeof(TV) * (size_t)c->F * R.DB * R.GS) != cudaSuccess)
+  if (cudaMalloc(&R.d_src, sizeof(T) * (size_t)R.SW * N) != cudaSuccess) {
+    cudaGetLastError();
+    R.d_src = nullptr;
     return rrhd_fail(RRHD_ERR_OOM, "sweep allocation failed");
-  if ((s = build_plan<T>(c))) return s;
-  if (R.item_geometry) {
-    const int64_t total = N * (int64_t)R.M;
-    if (cudaMalloc(&R.d_geo, sizeof(uint4) * total) != cudaSuccess) {
-      R.d_geo = nullptr;
-      return rrhd_fail(RRHD_ERR_OOM, "sweep geometry stream allocation failed (%lld bytes)",
-                       (long long)(sizeof(uint4) * total));
-    }
-    int64_t base = 0;
-    for (int b = 0; b < R.nbatch; b++) {
-      const int d0 = b * R.DB;
-      const int64_t n = N * std::min(R.DB, R.M - d0);
-      k_plan_geometry<T><<<grid_for(n, 256), 256, 0, c->stream>>>(R.d_plan + base, n, R.shift, R.DB, d0,
-                                                                  (const T *)R.d_w, (const T *)R.d_rec, R.RW,
-                                                                  R.d_geo + base);
-      RRHD_CUDA(cudaGetLastError());
-      base += n;
-    }
-    RRHD_CUDA(cudaStreamSynchronize(c->stream));
   }
-  return capture_sweep<T, TV, TI>(c);
+  if ((s = build_plan<T>(c))) return s;
+  if (R.d_dist) {  // no item reads the geometry records
+    cudaFree(R.d_rec);
+    R.d_rec = nullptr;
+  }
+  if (R.nhigh) {
+    const size_t bytes = sizeof(T) * (size_t)R.nhigh * R.G * R.M;
+    if (cudaMalloc(&R.d_slots, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      R.d_slots = nullptr;
+      return rrhd_fail(RRHD_ERR_OOM, "sweep slot allocation failed (%lld bytes)", (long long)bytes);
+    }
+  }
+  return RRHD_OK;
 }
 
 extern "C" rrhd_status rrhd_rad_setup(rrhd_ctx *c, const rrhd_dirs *dirs, const rrhd_rad_opts *o) {
@@ -1063,7 +1195,7 @@ extern "C" rrhd_status rrhd_rad_setup(rrhd_ctx *c, const rrhd_dirs *dirs, const 
   RRHD_CHECK_ARG(dirs->device == c->device, "direction set lives on another device");
   RRHD_CHECK_ARG(o->item_geometry == 0 || o->item_geometry == 1, "item_geometry: 0 or 1");
   RRHD_CHECK_ARG(o->item_geometry == 0 || o->precision != RRHD_RAD_FP64,
-                 "item_geometry needs RRHD_RAD_FP32 or RRHD_RAD_MIXED (its distances are float)");
+                 "item_geometry needs RRHD_RAD_FP32 or RRHD_RAD_MIXED");
   int DB = o->dirs_per_batch;
   RRHD_CHECK_ARG(DB == 0 || (DB > 0 && DB <= 256 && (DB & (DB - 1)) == 0), "dirs_per_batch: power of two <= 256");
   RRHD_CUDA(cudaSetDevice(c->device));
@@ -1078,18 +1210,12 @@ extern "C" rrhd_status rrhd_rad_setup(rrhd_ctx *c, const rrhd_dirs *dirs, const 
     while (DB < std::min(R.M, 64)) DB <<= 1;
   }
   R.DB = DB;
-  R.shift = 0;  // item = direction << shift | cell
-  while ((int64_t(1) << R.shift) < c->N) R.shift++;
-  if (R.shift > 31 || ((int64_t)DB << R.shift) > (int64_t)UINT32_MAX + 1)
-    return rrhd_fail(RRHD_ERR_LIMIT, "sweep items are 32-bit: dirs_per_batch x 2^ceil(log2 cells) must stay "
-                                     "within 2^32");
-  R.nbatch = (R.M + DB - 1) / DB;
+  const int shift = bits_for(c->N);
+  if (shift > 31 || ((int64_t)DB << shift) > (int64_t)UINT32_MAX + 1)
+    return rrhd_fail(RRHD_ERR_LIMIT, "dirs_per_batch x 2^ceil(log2 cells) must stay within 2^32");
   R.prec = o->precision;
   R.bc = o->boundary_value;
-  R.item_geometry = o->item_geometry != 0;
-  const rrhd_status s = R.prec == RRHD_RAD_FP64   ? rad_setup_t<double, double, double>(c)
-                        : R.prec == RRHD_RAD_MIXED ? rad_setup_t<double, double, float>(c)
-                                                   : rad_setup_t<float, float, float>(c);
+  const rrhd_status s = R.prec == RRHD_RAD_FP32 ? rad_setup_t<float>(c) : rad_setup_t<double>(c);
   if (s) {
     rrhd_rad_release(c);
     return s;
@@ -1111,38 +1237,17 @@ extern "C" rrhd_status rrhd_rad_plan_levels(const rrhd_ctx *c, int32_t *levels) 
   const RadState &R = c->rad;
   if (!R.ready) return rrhd_fail(RRHD_ERR_STATE, "rrhd_rad_setup has not run");
   RRHD_CUDA(cudaSetDevice(c->device));
-  const int64_t N = c->N, total = N * (int64_t)R.M;
-  std::vector<uint32_t> plan((size_t)total);
+  const int64_t N = c->N;
+  std::vector<uint4> ord((size_t)N);
+  std::vector<int32_t> off;
   RRHD_CUDA(cudaStreamSynchronize(c->stream));
-  RRHD_CUDA(cudaMemcpy(plan.data(), R.d_plan, sizeof(uint32_t) * total, cudaMemcpyDeviceToHost));
-  for (int64_t i = 0; i < total; i++) levels[i] = -1;
-  int64_t base = 0;
-  for (int b = 0; b < R.nbatch; b++) {
-    const int d0 = b * R.DB;
-    const int nbd = std::min(R.DB, R.M - d0);
-    const std::vector<int64_t> &off = R.lvl[b];
-    for (size_t L = 0; L + 1 < off.size(); L++)
-      for (int64_t k = off[L]; k < off[L + 1]; k++) {
-        const uint32_t it = plan[(size_t)(base + k)];
-        const int64_t cc = it & ((1u << R.shift) - 1u);
-        const int d = d0 + (int)(it >> R.shift);
-        levels[(int64_t)d * N + c->h_perm[cc]] = (int32_t)L;
-      }
-    base += N * nbd;
+  for (int d = 0; d < R.M; d++) {
+    off.resize(R.depth[d] + 1);
+    RRHD_CUDA(cudaMemcpy(ord.data(), R.d_ord + (int64_t)d * N, sizeof(uint4) * N, cudaMemcpyDeviceToHost));
+    RRHD_CUDA(cudaMemcpy(off.data(), R.d_lvl + R.lvl_base[d], sizeof(int32_t) * off.size(), cudaMemcpyDeviceToHost));
+    for (int L = 0; L < R.depth[d]; L++)
+      for (int32_t k = off[L]; k < off[L + 1]; k++) levels[(int64_t)d * N + c->h_perm[ord[k].x]] = L;
   }
-  return RRHD_OK;
-}
-
-static rrhd_status launch_sweep(rrhd_ctx *c, const SweepIO &io) {
-  RadState &R = c->rad;
-  // the graph reads its pointers from d_io; upload only when they change
-  if (!R.io_valid || std::memcmp(&io, &R.h_io, sizeof io) != 0) {
-    R.h_io = io;
-    RRHD_CUDA(cudaMemcpyAsync(R.d_io, &R.h_io, sizeof io, cudaMemcpyHostToDevice, c->stream));
-    RRHD_CUDA(cudaStreamSynchronize(c->stream));
-    R.io_valid = true;
-  }
-  RRHD_CUDA(cudaGraphLaunch(R.graph, c->stream));
   return RRHD_OK;
 }
 
@@ -1155,16 +1260,15 @@ extern "C" rrhd_status rrhd_sweep(rrhd_ctx *c, const void *alpha, const void *be
   const int64_t N = c->N;
   if (R.prec == RRHD_RAD_FP64)
     k_dyn_from_arrays<double, double><<<grid_for(N, 256), 256, 0, c->stream>>>(
-        N, R.G, R.RW, c->d_perm, (const double *)alpha, (const double *)betta, (const double *)Q, (double *)R.d_rec);
+        N, R.G, R.SW, c->d_perm, (const double *)alpha, (const double *)betta, (const double *)Q, (double *)R.d_src);
   else if (R.prec == RRHD_RAD_MIXED)  // float arrays, double records
     k_dyn_from_arrays<double, float><<<grid_for(N, 256), 256, 0, c->stream>>>(
-        N, R.G, R.RW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q, (double *)R.d_rec);
+        N, R.G, R.SW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q, (double *)R.d_src);
   else
     k_dyn_from_arrays<float, float><<<grid_for(N, 256), 256, 0, c->stream>>>(
-        N, R.G, R.RW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q, (float *)R.d_rec);
+        N, R.G, R.SW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q, (float *)R.d_src);
   RRHD_CUDA(cudaGetLastError());
-  SweepIO io{S, I, c->d_perm, 0};
-  return launch_sweep(c, io);
+  return run_sweep(c, S, I, false);
 }
 
 // ---------------------------------------------------------------- coupled step
@@ -1281,11 +1385,11 @@ extern "C" rrhd_status rrhd_coupled_step(rrhd_ctx *c, double tau, const rrhd_cou
   const Emission em{o->emission.temp_coef, o->emission.sigma_sb, o->emission.pi, o->emission.rad_unit};
   // 2. opacities and emission from the new primitives
   if (rec64)
-    k_dyn_from_state<double><<<grid_for(N, 256), 256, 0, st>>>(N, R.G, R.RW, state, o->absorption, o->scattering,
-                                                                em, (double *)R.d_rec);
+    k_dyn_from_state<double><<<grid_for(N, 256), 256, 0, st>>>(N, R.G, 4, state, o->absorption, o->scattering,
+                                                                em, (double *)R.d_src);
   else
-    k_dyn_from_state<float><<<grid_for(N, 256), 256, 0, st>>>(N, R.G, R.RW, state, o->absorption, o->scattering, em,
-                                                               (float *)R.d_rec);
+    k_dyn_from_state<float><<<grid_for(N, 256), 256, 0, st>>>(N, R.G, 4, state, o->absorption, o->scattering, em,
+                                                               (float *)R.d_src);
   RRHD_CUDA(cudaGetLastError());
   // 4. 4-force from the previous intensity's moments and the source con2prim, on the side
   // stream beside the sweep: they read the state after the opacities were taken from it and
@@ -1307,8 +1411,7 @@ extern "C" rrhd_status rrhd_coupled_step(rrhd_ctx *c, double tau, const rrhd_cou
   }
   RRHD_CUDA(cudaEventRecord(R.ev[4], ss_st));
   // 3. sweep with the previous scattering integral
-  SweepIO io{R.d_S, R.d_I, nullptr, 1};
-  if ((s = launch_sweep(c, io))) return s;
+  if ((s = run_sweep(c, R.d_S, R.d_I, true))) return s;
   RRHD_CUDA(cudaEventRecord(R.ev[2], st));
   // the scattering below overwrites the moments the source read, and the next step reads
   // the state the source wrote: join the side stream

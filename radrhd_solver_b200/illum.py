@@ -200,10 +200,9 @@ class TransportSweep:
     outputs (sorted_graph, vec_x0), built on the GPU as levels.  precision:
     "fp64" or "fp32" (storage and arithmetic of alpha, betta, Q, S, I), or "mixed"
     (float arrays as "fp32", face values and the transport update in double).
-    item_geometry ("fp32" and "mixed"): precompute every (cell, direction) item's
-    in/out faces, node choices and in-face distances (float) at setup, 16 bytes per
-    item, and stream them in sweep order instead of reading each cell's geometry per
-    item."""
+    dirs_per_batch: directions whose levels plan_info counts together.  item_geometry
+    ("fp32" and "mixed" only): accepted; every sweep keeps its items' geometry in sweep
+    order where device memory holds it."""
 
     def __init__(self, grid, dg: DirectionGrid, groups: int = 1, precision: str = "fp64", dirs_per_batch: int = 0,
                  boundary_value: float = 0.0, item_geometry: bool = False):
