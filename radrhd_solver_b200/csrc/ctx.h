@@ -68,14 +68,16 @@ struct RadState {
   uint2 *d_ord_hi = nullptr;  // [M][N] upper halves of the slots, where 16 bits do not hold them
   // geometry stream, where memory allows: [M][N][2] distances, [M][N][2] and [M][N] in-face weights
   void *d_dist = nullptr, *d_wgt = nullptr, *d_wgt3 = nullptr;
+  uint32_t *d_pos = nullptr;  // [M][N] each cell's position in sweep order, with the stream
   int32_t *d_lvl = nullptr, *d_depth = nullptr;  // level offsets of all directions; levels per direction
   int64_t *d_lvl_base = nullptr;                 // first entry of a direction in d_lvl
   std::vector<int32_t> depth;
   std::vector<int64_t> lvl_base;
   int64_t levels = 0, max_level = 0;
+  bool two = false;             // two CTAs of the sweep share an SM
   int64_t nlow = 0, nhigh = 0;  // most slots a direction has in shared (slot 0: the boundary value) and global memory
   void *d_slots = nullptr;      // [M][nhigh][G]
-  void *d_x = nullptr;          // S and I in the sweep's layout, [xdirs][N][G]
+  void *d_x = nullptr;          // S, then I, in the sweep's layout, [xdirs][N][G]
   int xdirs = 0;
   // phase marks of the last coupled step: 0 start, 1 hydro done, 2 sweep done, 3 source
   // start and 4 source done (side stream), 5 join, 6 scattering done

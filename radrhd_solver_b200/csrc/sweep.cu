@@ -91,6 +91,8 @@ __device__ __forceinline__ void load_nbr(const T *r, int *nbr) {
   nbr[0] = n.x, nbr[1] = n.y, nbr[2] = n.z, nbr[3] = n.w;
 }
 
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double ex(double x) { return exp(x); }
 __device__ __forceinline__ float ex(float x) { return __expf(x); }
 __device__ __forceinline__ double dv(double a, double b) { return a / b; }
@@ -108,7 +110,8 @@ __device__ __forceinline__ void face_cos(const T *g, T wx, T wy, T wz, T *cosf) 
 //                       the face areas sum to zero)
 //   bits 8-11           out-faces (cos > 0)
 //   bit 12              the node at b1's vertex is traced to b2 (else to b1, lam = 2/3)
-constexpr uint32_t kCodeB2 = 1u << 12;
+//   bit 13              some face is neither (parallel to the direction)
+constexpr uint32_t kCodeB2 = 1u << 12, kCodeOdd = 1u << 13;
 
 // Code word and distances of one (cell, direction) from the cell's normals and heights
 // g[16]: tA = r_b1 / 6, tB = r_b2 / 6 (bit 12; else 0).  b1, b2: the smallest by (t, face
@@ -144,6 +147,7 @@ __device__ __forceinline__ uint32_t item_geometry(const T *g, const T *cosf, T &
   tA = tb1;
   tB = (T)0;
   uint32_t code = out << 8 | (uint32_t)n << 6;
+  if (n + __popc(out) != 4) code |= kCodeOdd;
   if (n >= 1) code |= (uint32_t)b1;
   if (n >= 2) {
     code |= (uint32_t)b2 << 2;
@@ -227,29 +231,42 @@ struct SweepArgs {
   T *slots;                 // [directions of the launch][nhigh][G]: slots from `cap` on
   uint32_t cap;             // slots in shared memory
   int64_t nhigh;
-  const TI *S;              // S and I element (cell c, direction d0 + x, group g) at c * sc + x * sd + g
-  TI *I;
+  const TI *S;              // S and I element (cell c, direction d0 + x, group g) at q * sc + x * sd + g,
+  TI *I;                    // q the item's position in sweep order (by_pos) or its cell
   int64_t sc, sd;
+  bool by_pos;
   T bc;
 };
 
-// One CTA per direction.  GT: compile-time group count (1, 2 or 4), 0 for any other.
-// HIGH: slots from a.cap on are in global memory (the others in shared memory).  GEO: distances and weights from the stream, else
-// from the cell's records.  Slot 0 holds the boundary value for the whole sweep; an item
+// Asks L2 for n bytes at p (both multiples of 16 after rounding p down).
+template <class P>
+__device__ __forceinline__ void bulk_prefetch(const P *p, uint32_t n) {
+  const uint64_t b = reinterpret_cast<uint64_t>(p);
+  const uint32_t skip = (uint32_t)(b & 15);
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b - skip), "r"((n + skip) & ~15u) : "memory");
+}
+
+// One CTA per direction.  GT: compile-time group count (1, 2 or 4; S and I in the sweep's own
+// layout), 0 for any other.  HIGH: slots from a.cap on are in global memory (the others in
+// shared memory).  GEO: distances and weights from the stream, else from the cell's records.
+// Slots 0 and 1 hold the boundary value and zero (for in-faces an item does not have); an item
 // whose own slot is 0 has no downwind neighbour and writes none.
 //
-// Each item has three uncoalesced accesses, each one access of up to 32 bytes: its source
-// record, S and I; the slots are in shared memory as far as they fit.  Only the slot values
-// depend on the levels before, so a thread loads the record of its item after the next, and
-// the source and S of its next one, while it works on one item.  Measured (whole sweep with
-// its copies, before: one launch per level of all directions, face values in HBM): 48^3 x 6
-// cells x 256 directions FP64, one group, 28.1 -> 5.2 ms; 12^3 x 6 x 64, 269 -> 87 us; the
-// mixed sweep of 4 groups at 48^3 x 256, 37.0 -> 13 ms.  What bounds it: issue slots and the
-// latency of those accesses at 16 warps an SM (about 400 instructions an item of a warp).
+// Only the slot values depend on the levels before.  A thread loads the record and distances of
+// its item after the next, and the source record of its next one, while it works on one item;
+// one thread asks L2 for the streams' lines four CTA widths ahead.  What an SM can send of
+// uncoalesced accesses (a request every few cycles when each misses L1) decides the rest: per
+// item one 32-byte source record, and by cell also S and I.
+// Measured (whole sweep with its copies; before: one launch per level of all directions, face
+// values in HBM): 48^3 x 6 cells x 256 directions FP64, one group, 28.1 -> 5.5 ms; 12^3 x 6 x
+// 64, 269 -> 80 us; 32^3 x 256 x 4 FP64 12.6 -> 4.0 ms; 48^3 x 256 x 4 mixed 37.0 -> 10.2 ms.
+// With every load from L1 it would take half of that: issue slots and the latency of the FP64
+// chains at 16 warps an SM, and the wait at each level's barrier.
 template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB>
 __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
   extern __shared__ __align__(16) uint8_t sweep_smem[];
   constexpr int GR = GT > 0 ? GT : 1;
+  constexpr int kAhead = 4 * NT;
   const int x = blockIdx.x, d = a.d0 + x;
   const int G = GT > 0 ? GT : a.G;
   T *const low = reinterpret_cast<T *>(sweep_smem);
@@ -265,62 +282,63 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
     return low + q * (uint32_t)G;
   };
   const int64_t at = (int64_t)d * a.N;
-  const uint4 *ord = a.ord + at;
+  const uint4 *const ord = a.ord + at;
+  const T *const dist = a.dist + 2 * at, *const wgt = a.wgt + 2 * at, *const wgt3 = a.wgt3 + at;
   const int32_t *lvl = a.lvl + a.lvl_base[d];
   const int depth = a.depth[d];
-  const TI *S = a.S + x * a.sd;
-  TI *I = a.I + x * a.sd;
+  const TI *const S = a.S + x * a.sd;
+  TI *const I = a.I + x * a.sd;
+  const char *const src = reinterpret_cast<const char *>(a.src);
+  const uint32_t src_bytes = (uint32_t)(a.SW * (int)sizeof(T));
   const int N = (int)a.N;
   T wx = 0, wy = 0, wz = 0;
   if (!GEO) wx = a.w[3 * d], wy = a.w[3 * d + 1], wz = a.w[3 * d + 2];
-  for (int g = threadIdx.x; g < G; g += NT) low[g] = a.bc;
+  for (int g = threadIdx.x; g < 2 * G; g += NT) low[g] = g < G ? a.bc : (T)0;
   __syncthreads();
 
   struct Item {
     uint4 o;
     uint2 hi;
-    T tA, tB, w[3];
-    T k, bk, q[GR];
-    TI s[GR];
+    T tA, tB;
+    T k, bk, q0, q1;  // q1: of the second group where each has its own
   };
   auto load_record = [&](int i, Item &it) {
     it.o = __ldcs(ord + i);
     if constexpr (WIDE) it.hi = __ldcs(a.ord_hi + at + i);
     if constexpr (GEO) {
       if constexpr (sizeof(T) == 8) {
-        const double2 t = __ldcs(reinterpret_cast<const double2 *>(a.dist) + at + i);
-        const double2 u = __ldcs(reinterpret_cast<const double2 *>(a.wgt) + at + i);
-        it.tA = t.x, it.tB = t.y, it.w[0] = u.x, it.w[1] = u.y;
+        const double2 t = __ldcs(reinterpret_cast<const double2 *>(dist) + i);
+        it.tA = t.x, it.tB = t.y;
       } else {
-        const float2 t = __ldcs(reinterpret_cast<const float2 *>(a.dist) + at + i);
-        const float2 u = __ldcs(reinterpret_cast<const float2 *>(a.wgt) + at + i);
-        it.tA = t.x, it.tB = t.y, it.w[0] = u.x, it.w[1] = u.y;
+        const float2 t = __ldcs(reinterpret_cast<const float2 *>(dist) + i);
+        it.tA = t.x, it.tB = t.y;
       }
-      it.w[2] = __ldcs(a.wgt3 + at + i);
     }
   };
   auto load_cell = [&](Item &it) {
-    const int64_t c = it.o.x;
-    const T *sr = a.src + c * a.SW;
-    T q0, q1;
+    const T *sr = reinterpret_cast<const T *>(src + (uint64_t)it.o.x * src_bytes);
     if constexpr (sizeof(T) == 8) {
-      ld_32(sr, it.k, it.bk, q0, q1);
+      ld_32(sr, it.k, it.bk, it.q0, it.q1);
     } else {
       const float4 t = __ldg(reinterpret_cast<const float4 *>(sr));
-      it.k = t.x, it.bk = t.y, q0 = t.z, q1 = t.w;
+      it.k = t.x, it.bk = t.y, it.q0 = t.z, it.q1 = t.w;
     }
-    if constexpr (GT > 0) {
-      ld_groups<true>(S + c * a.sc, it.s);
-#pragma unroll
-      for (int g = 0; g < GT; g++) it.q[g] = q0;
-      if constexpr (GT > 1) {
-        if (a.qs) {
-          it.q[1] = q1;
-#pragma unroll
-          for (int g = 2; g < GT; g++) it.q[g] = __ldg(sr + kSrcQ + g);
-        }
-      }
+  };
+  // one thread asks L2 for the streams' lines some levels ahead
+  int fetched = 0;
+  auto fetch = [&](int to) {
+    to = min(to, N) & ~1;  // whole 16-byte pieces
+    if (to <= fetched) return;
+    const int64_t q = fetched;
+    const uint32_t n = (uint32_t)(to - fetched);
+    bulk_prefetch(ord + q, 16 * n);
+    if (GEO) {
+      bulk_prefetch(dist + 2 * q, 2 * (uint32_t)sizeof(T) * n);
+      bulk_prefetch(wgt + 2 * q, 2 * (uint32_t)sizeof(T) * n);
+      if (sizeof(T) == 8) bulk_prefetch(wgt3 + q, 8 * n);
     }
+    if (a.by_pos && sizeof(TI) * G % 8 == 0) bulk_prefetch(S + (int64_t)fetched * G, (uint32_t)sizeof(TI) * G * n);
+    fetched = to;
   };
 
   // this thread's items in order, two ahead of the one in work: position p in the level that
@@ -346,8 +364,11 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
   }
   int hi = lvl[1], hi2 = lvl[min(2, depth)];
   for (int L = 0; L < depth; L++) {
+    if (threadIdx.x == 0) fetch(hi + kAhead);
     while (i < hi) {
       const Item now = it;
+      const int at_i = i;
+      const uint32_t iq = a.by_pos ? (uint32_t)i : now.o.x;
       i = p;
       it = next;
       if (p < N) {
@@ -356,8 +377,21 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
         settle();
         if (p < N) load_record(p, next);
       }
-      const int64_t c = now.o.x;
+      const uint64_t c = now.o.x;
       const uint32_t code = now.o.y;
+      T w[3];
+      TI sv[GR];
+      if constexpr (GT > 0) ld_groups<true>(S + (uint64_t)iq * (uint32_t)GT, sv);
+      if constexpr (GEO) {
+        if constexpr (sizeof(T) == 8) {
+          const double2 u = __ldcs(reinterpret_cast<const double2 *>(wgt) + at_i);
+          w[0] = u.x, w[1] = u.y;
+        } else {
+          const float2 u = __ldcs(reinterpret_cast<const float2 *>(wgt) + at_i);
+          w[0] = u.x, w[1] = u.y;
+        }
+        w[2] = __ldcs(wgt3 + at_i);
+      }
       uint32_t own = now.o.z & 0xffffu, s0 = now.o.z >> 16, s1 = now.o.w & 0xffffu, s2 = now.o.w >> 16;
       if constexpr (WIDE) {
         own |= now.hi.x << 16;
@@ -365,9 +399,9 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
         s1 |= now.hi.y << 16;
         s2 |= now.hi.y & 0xffff0000u;
       }
-      T tA, tB, w[3];
+      T tA, tB;
       if constexpr (GEO) {
-        tA = now.tA, tB = now.tB, w[0] = now.w[0], w[1] = now.w[1], w[2] = now.w[2];
+        tA = now.tA, tB = now.tB;
       } else {
         T g[16], cosf[4];
         load_vec<T>(a.rec + c * Rec<T>::RW, g, 16);
@@ -376,15 +410,14 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
         in_weights(a.wt + 4 * c, code, w);
       }
       const T k = now.k, bk = now.bk;
-      const int nin = (int)(code >> 6) & 3;
       const bool two = (code & kCodeB2) != 0;
       const T EA = ex(-k * tA);
-      T EB = EA * EA;
-      EB = EB * EB;
-      if (two) EB = ex(-k * tB);
+      const T E2 = EA * EA, EX = ex(-k * tB);  // formed in any case: the two chains overlap
+      const T EB = two ? EX : E2 * E2;
       T wo = ((T)1 - w[0]) - (w[1] + w[2]);  // all out-faces together
       T par = (T)0;                          // a face parallel to the direction holds the boundary value
-      if (nin + __popc((code >> 8) & 15u) != 4) {
+      if (code & kCodeOdd) {
+        const int nin = (int)(code >> 6) & 3;
         uint32_t seen = (code >> 8) & 15u;
         if (nin > 0) seen |= 1u << (code & 3);
         if (nin > 1) seen |= 1u << ((code >> 2) & 3);
@@ -398,41 +431,41 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
         }
       }
       auto value = [&](T v0, T v1, T v2, T rhs, T &cell) {
-        const T A = EA * (v0 - rhs) + rhs;
-        const T B = EB * ((two ? v1 : v0) - rhs) + rhs;
-        const T o = ((A + A) + B) * (T)0.3333333333333333;
-        cell = (v0 * w[0] + v1 * w[1]) + (v2 * w[2] + o * wo) + par;
+        const T A = fma_rn(EA, v0 - rhs, rhs);
+        const T B = fma_rn(EB, (two ? v1 : v0) - rhs, rhs);
+        const T o = fma_rn((T)2, A, B) * (T)0.3333333333333333;
+        cell = fma_rn(v0, w[0], fma_rn(v1, w[1], fma_rn(v2, w[2], fma_rn(o, wo, par))));
         return o;
       };
-      TI *Ic = I + c * a.sc;
       if constexpr (GT > 0) {
         TI iv[GT];
         T v0[GT], v1[GT], v2[GT], o[GT];
         get_slot(s0, v0);
-#pragma unroll
-        for (int g = 0; g < GT; g++) v1[g] = v2[g] = (T)0;
-        if (nin > 1) get_slot(s1, v1);
-        if (nin > 2) get_slot(s2, v2);
+        get_slot(s1, v1);
+        get_slot(s2, v2);
 #pragma unroll
         for (int g = 0; g < GT; g++) {
-          T cell;
-          o[g] = value(v0[g], v1[g], v2[g], now.q[g] + bk * (T)now.s[g], cell);
+          T q = now.q0, cell;
+          if (g > 0 && a.qs)
+            q = g == 1 ? now.q1 : __ldg(reinterpret_cast<const T *>(src + c * src_bytes) + kSrcQ + g);
+          o[g] = value(v0[g], v1[g], v2[g], fma_rn(bk, (T)sv[g], q), cell);
           iv[g] = (TI)cell;
         }
         if (HIGH && own >= a.cap)
           st_groups<true>(high + (int64_t)(own - a.cap) * GR, o);
         else if (own)
           st_groups<false>(low + own * GR, o);
-        st_groups<true>(Ic, iv);
+        st_groups<true>(I + (uint64_t)iq * (uint32_t)GT, iv);
       } else {
         const T *sr = a.src + c * a.SW + kSrcQ;
-        const TI *Sc = S + c * a.sc;
+        const TI *Sc = S + (int64_t)iq * a.sc;
+        TI *Ic = I + (int64_t)iq * a.sc;
         for (int g = 0; g < G; g++) {
           const T v0 = slot(s0)[g];
-          const T v1 = nin > 1 ? slot(s1)[g] : (T)0;
-          const T v2 = nin > 2 ? slot(s2)[g] : (T)0;
+          const T v1 = slot(s1)[g];
+          const T v2 = slot(s2)[g];
           T cell;
-          const T o = value(v0, v1, v2, sr[g * a.qs] + bk * (T)Sc[g], cell);
+          const T o = value(v0, v1, v2, fma_rn(bk, (T)Sc[g], sr[g * a.qs]), cell);
           if (own) slot(own)[g] = o;
           Ic[g] = (TI)cell;
         }
@@ -444,38 +477,94 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
   }
 }
 
-// The sweep's own layout is [direction][cell * G + g] in context numbering (V = TI), so that
-// the cells of a front, close together in Morton order, lie close together in memory.  These
-// tiles of 32 x 32 values of type V bring an array there and back through shared memory,
-// whole lines on both sides, directions d0 .. d0 + nd - 1:
-//   rows [rows][M] in caller numbering (perm; row = cell * G + g, V = TI), or
-//   [cells][M][G] in context numbering (perm null; V = the G values of a cell and direction).
+// The sweep's own layout is [direction][item][G], items in sweep order (pos: the position of
+// each cell [M][N]) or, without pos, cells in context numbering.  These tiles of 32 rows x DX
+// directions of values of type V bring an array there and back through shared memory,
+// directions d0 .. d0 + nd - 1, gw values of V a cell:
+//   rows [rows][M] in caller numbering (perm; row = cell * gw + g, V = TI, gw = G), or
+//   [cells][M][G] in context numbering (perm null; V = the G values of a cell and direction,
+//   gw = 1).
+// The caller's side moves whole lines.  On the other side the cells of a tile, neighbours in
+// Morton order, lie in few runs (a level holds its cells in that order), and the tiles around
+// it fill up the same lines while they are in L2: the scattered accesses are here, where 64
+// warps an SM hide them, and not in the sweep, whose warps could not send them fast enough
+// (a front's S by cell held them up 2 of 5 ms at 32^3 x 256 x 4 FP64).  All indices are loaded
+// before the first value.
+struct alignas(8) Bytes8 { uint32_t w[2]; };
+struct alignas(16) Bytes16 { uint32_t w[4]; };
+struct alignas(32) Bytes32 { double w[4]; };
+
+// one access a value in global memory, 32 bytes included
+template <class V>
+__device__ __forceinline__ V ld_value(const V *p) {
+  if constexpr (sizeof(V) == 32) {
+    V v;
+    ld_32(reinterpret_cast<const double *>(p), v.w[0], v.w[1], v.w[2], v.w[3]);
+    return v;
+  } else {
+    return *p;
+  }
+}
+template <class V>
+__device__ __forceinline__ void st_value(V *p, const V &v) {
+  if constexpr (sizeof(V) == 32)
+    st_32(reinterpret_cast<double *>(p), v.w[0], v.w[1], v.w[2], v.w[3]);
+  else
+    *p = v;
+}
+template <class V>
+constexpr int kTileDirs = sizeof(V) <= 8 ? 64 : 32;
 template <class V, bool IMPORT>
-__global__ void __launch_bounds__(256) k_tile(int64_t rows, int G, int M, int d0, int nd, const int32_t *perm,
-                                              const V *in, V *out) {
-  __shared__ V tile[32][33];
+__global__ void __launch_bounds__(256) k_tile(int64_t N, int gw, int M, int d0, int nd, const int32_t *perm,
+                                              const uint32_t *pos, const V *in, V *out) {
+  constexpr int DX = kTileDirs<V>;
+  __shared__ V tile[DX][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t rows = N * gw;
   const int64_t r0 = (int64_t)blockIdx.x * 32;
-  const int x0 = blockIdx.y * 32;
-  auto row = [&](int64_t r) { return (perm ? (int64_t)perm[r / G] * G + r % G : r) * M + d0 + x0 + tx; };
+  const int x0 = blockIdx.y * DX;
+  int64_t line[4];        // offset of row ty + 8 k on the caller's side
+  int64_t item[DX / 8];   // offset of (row tx, direction ty + 8 k) on the sweep's side
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const int y = ty + 8 * k;
-    if (IMPORT) {
-      if (r0 + y < rows && x0 + tx < nd) tile[y][tx] = in[row(r0 + y)];
-    } else {
-      if (r0 + tx < rows && x0 + y < nd) tile[y][tx] = in[(int64_t)(x0 + y) * rows + r0 + tx];
+    const int64_t r = r0 + ty + 8 * k;
+    line[k] = -1;
+    if (r < rows) {
+      const int64_t c = gw == 1 ? r : r / gw;
+      line[k] = ((perm ? (int64_t)perm[c] : c) * gw + (r - c * gw)) * M + d0 + x0;
     }
   }
-  __syncthreads();
+  {
+    const int64_t r = r0 + tx, c = gw == 1 ? r : r / gw;
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int y = ty + 8 * k;
-    if (IMPORT) {
-      if (r0 + tx < rows && x0 + y < nd) out[(int64_t)(x0 + y) * rows + r0 + tx] = tile[tx][y];
-    } else {
-      if (r0 + y < rows && x0 + tx < nd) out[row(r0 + y)] = tile[tx][y];
+    for (int k = 0; k < DX / 8; k++) {
+      const int x = x0 + ty + 8 * k;
+      item[k] = -1;
+      if (r < rows && x < nd) item[k] = x * rows + (pos ? (int64_t)pos[(d0 + x) * N + c] : c) * gw + (r - c * gw);
     }
+  }
+  if (IMPORT) {
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int h = 0; h < DX; h += 32)
+        if (line[k] >= 0 && x0 + h + tx < nd) tile[h + tx][ty + 8 * k] = ld_value(in + line[k] + h + tx);
+  } else {
+#pragma unroll
+    for (int k = 0; k < DX / 8; k++)
+      if (item[k] >= 0) tile[ty + 8 * k][tx] = ld_value(in + item[k]);
+  }
+  __syncthreads();
+  if (IMPORT) {
+#pragma unroll
+    for (int k = 0; k < DX / 8; k++)
+      if (item[k] >= 0) st_value(out + item[k], tile[ty + 8 * k][tx]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int h = 0; h < DX; h += 32)
+        if (line[k] >= 0 && x0 + h + tx < nd) st_value(out + line[k] + h + tx, tile[h + tx][ty + 8 * k]);
   }
 }
 
@@ -566,15 +655,17 @@ __global__ void k_plan_offsets(int64_t N, int64_t total, int lbits, int d0, cons
 // Items of one direction per CTA in sweep order: face choice, distances and slots.  Within a
 // level the cells' own slots are taken first (from the free list, or a new one), then the
 // slots whose last reader sits in this level go back, so a slot is never written in a level
-// that reads it.  Slots below `cap` (those in shared memory) are preferred: the free list of
-// the low slots grows from the front of `freed`, that of the high ones from its end.  order [nd][N] cells in sweep order; slot_of, readers, freed [nd][N] scratch.
+// that reads it.  Slots below cap2 (the shared memory of one CTA of two per SM) are preferred,
+// then those below cap1 (of a CTA that has the SM alone): the free lists of these two sit at
+// the front of `freed` and from cap2 on, that of the rest at its end (there are never more
+// slots than cells).  need [M]: one more than a direction's largest slot.
 template <class T>
 __global__ void __launch_bounds__(kPlanThreads)
     k_plan_items(int64_t N, int d0, const T *w, const T *rec, const int32_t *lvl_all, const int64_t *lvl_base,
                  const int32_t *depth, const uint32_t *order_all, uint32_t *slot_all, uint32_t *readers_all,
                  uint32_t *freed_all, uint4 *ord_all, uint2 *hi_all, const T *wt, T *dist_all, T *wgt_all, T *wgt3_all,
-                 uint32_t cap, unsigned int *max_slots) {
-  __shared__ int top, next, htop, hnext;
+                 uint32_t *pos_all, int cap2, int cap1, int32_t *need) {
+  __shared__ int top[3], next[3];  // free list and next new slot below cap2, below cap1, beyond
   const int x = blockIdx.x, d = d0 + x;
   const uint32_t *order = order_all + x * N;
   uint32_t *slot_of = slot_all + x * N, *readers = readers_all + x * N, *freed = freed_all + x * N;
@@ -583,7 +674,12 @@ __global__ void __launch_bounds__(kPlanThreads)
   const int64_t at = (int64_t)d * N;
   const int32_t *lvl = lvl_all + lvl_base[d];
   const T wx = w[3 * d], wy = w[3 * d + 1], wz = w[3 * d + 2];
-  if (threadIdx.x == 0) top = htop = 0, next = 1, hnext = (int)cap;  // slot 0 is the boundary value
+  if (threadIdx.x == 0) {
+    top[0] = top[1] = top[2] = 0;
+    next[0] = 2;  // slots 0 and 1 hold the boundary value and zero
+    next[1] = cap2;
+    next[2] = cap1;
+  }
   __syncthreads();
   int lo = 0;
   for (int L = 0; L < depth[d]; L++) {
@@ -601,27 +697,31 @@ __global__ void __launch_bounds__(kPlanThreads)
       for (int j = 0; j < 4; j++) n += (cosf[j] > 0 && nbr[j] >= 0) ? 1u : 0u;
       uint32_t own = 0;
       if (n) {
-        const int q = atomicSub(&top, 1) - 1;
+        int q = atomicSub(&top[0], 1) - 1;
         if (q >= 0) {
           own = freed[q];
+        } else if ((q = atomicAdd(&next[0], 1)) < cap2) {
+          own = (uint32_t)q;
+        } else if ((q = atomicSub(&top[1], 1) - 1) >= 0) {
+          own = freed[cap2 + q];
+        } else if ((q = atomicAdd(&next[1], 1)) < cap1) {
+          own = (uint32_t)q;
         } else {
-          own = (uint32_t)atomicAdd(&next, 1);
-          if (own >= cap) {
-            const int h = atomicSub(&htop, 1) - 1;
-            own = h >= 0 ? freed[N - 1 - h] : (uint32_t)atomicAdd(&hnext, 1);
-          }
+          q = atomicSub(&top[2], 1) - 1;
+          own = q >= 0 ? freed[N - 1 - q] : (uint32_t)atomicAdd(&next[2], 1);
         }
         slot_of[c] = own;
         readers[c] = n;
       }
       const int nin = (int)(code >> 6) & 3;
-      uint32_t s[3] = {0u, 0u, 0u};
+      uint32_t s[3] = {0u, 1u, 1u};  // no such in-face (a cell without any starts from the boundary value)
 #pragma unroll
       for (int q = 0; q < 3; q++) {
         const int f = (int)(code >> (2 * q)) & 3;
         const int b = f == 0 ? nbr[0] : f == 1 ? nbr[1] : f == 2 ? nbr[2] : nbr[3];
-        if (q < nin && b >= 0) s[q] = slot_of[b];
+        if (q < nin) s[q] = b >= 0 ? slot_of[b] : 0u;
       }
+      if (pos_all) pos_all[at + c] = (uint32_t)i;
       ord[i] = make_uint4((uint32_t)c, code, (own & 0xffffu) | s[0] << 16, (s[1] & 0xffffu) | s[2] << 16);
       if (hi16) hi16[i] = make_uint2(own >> 16 | (s[0] & 0xffff0000u), s[1] >> 16 | (s[2] & 0xffff0000u));
       if (dist_all) {
@@ -636,9 +736,9 @@ __global__ void __launch_bounds__(kPlanThreads)
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      top = max(top, 0);
-      htop = max(htop, 0);
-      next = min(next, (int)cap);
+      for (int q = 0; q < 3; q++) top[q] = max(top[q], 0);
+      next[0] = min(next[0], cap2);
+      next[1] = min(next[1], cap1);
     }
     __syncthreads();
     for (int i = lo + (int)threadIdx.x; i < hi; i += kPlanThreads) {
@@ -652,19 +752,18 @@ __global__ void __launch_bounds__(kPlanThreads)
       for (int j = 0; j < 4; j++)
         if (cosf[j] < 0 && nbr[j] >= 0 && atomicSub(readers + nbr[j], 1u) == 1u) {
           const uint32_t q = slot_of[nbr[j]];
-          if (q < cap)
-            freed[atomicAdd(&top, 1)] = q;
+          if (q < (uint32_t)cap2)
+            freed[atomicAdd(&top[0], 1)] = q;
+          else if (q < (uint32_t)cap1)
+            freed[cap2 + atomicAdd(&top[1], 1)] = q;
           else
-            freed[N - 1 - atomicAdd(&htop, 1)] = q;
+            freed[N - 1 - atomicAdd(&top[2], 1)] = q;
         }
     }
     lo = hi;
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    atomicMax(max_slots, (unsigned int)next);
-    atomicMax(max_slots + 1, (unsigned int)hnext);
-  }
+  if (threadIdx.x == 0) need[d] = next[2] > cap1 ? next[2] : next[1] > cap2 ? next[1] : next[0];
 }
 
 // Source record {k = alpha + betta, betta / k, alpha Q_g / k} of each context cell
@@ -803,14 +902,20 @@ Eos eos_of(const rrhd_ctx *c) {
 }
 
 // ---------------------------------------------------------------- launches
-// Shared memory of a sweep's CTA: two CTAs of 256 threads per SM while the slots of every
-// direction fit half an SM (the one works while the other waits at its level's barrier), else
-// one of 512 threads, with the slots beyond its shared memory in global memory.
-constexpr int kSweepSMs = 148, kSmemTwo = 112 * 1024, kSmemOne = 226 * 1024;
+// Shared memory of a sweep's CTA.  With more directions than SMs two CTAs of 256 threads share
+// an SM, so that one works while the other waits at its level's barrier, where their half of
+// it holds all but a few of the slots and S and I are in sweep order; else one of 512 threads
+// has it alone.  The slots beyond are in global memory.  32^3 x 256 directions, four groups
+// FP64 (7 % of the slots beyond half an SM): 4.0 ms with two, 4.5 with one; 48^3, four groups
+// mixed (57 % beyond): 14.4 and 10.2; 48^3, one group FP64 (none beyond, but S by cell: twice
+// the directions at work push each other's lines out of L2): 9.5 and 5.5.  More threads an SM
+// run out of registers (1024: 8.1 ms in the first).
+constexpr int kSweepSMs = 148, kSmemTwo = 113 * 1024, kSmemOne = 226 * 1024;
+constexpr double kTwoBeyond = 0.1;  // slots that may be beyond half an SM
 
-uint32_t slot_cap(const RadState &R) {  // slots a CTA's shared memory can hold
+int slot_cap(const RadState &R, bool two) {  // slots a CTA's shared memory can hold
   const size_t tv = R.prec == RRHD_RAD_FP32 ? sizeof(float) : sizeof(double);
-  return (uint32_t)(kSmemOne / (tv * R.G));
+  return (int)((two ? kSmemTwo : kSmemOne) / (tv * R.G));
 }
 
 template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB>
@@ -831,15 +936,21 @@ cudaError_t launch_sweep_geo(const SweepArgs<T, TI> &a, int nd, size_t smem, cud
 template <class T, class TI, int GT>
 cudaError_t launch_sweep_groups(const SweepArgs<T, TI> &a, int64_t low, bool two, int nd, cudaStream_t st) {
   const size_t smem = sizeof(T) * (size_t)low * a.G;
-  if (two && !a.nhigh && smem <= kSmemTwo) return launch_sweep_geo<T, TI, GT, false, false, 256, 2>(a, nd, smem, st);
+  if (two) {
+    if (a.ord_hi) return launch_sweep_geo<T, TI, GT, true, true, 256, 2>(a, nd, smem, st);
+    if (a.nhigh) return launch_sweep_geo<T, TI, GT, true, false, 256, 2>(a, nd, smem, st);
+    return launch_sweep_geo<T, TI, GT, false, false, 256, 2>(a, nd, smem, st);
+  }
   if (a.ord_hi) return launch_sweep_geo<T, TI, GT, true, true, 512, 1>(a, nd, smem, st);
   if (a.nhigh) return launch_sweep_geo<T, TI, GT, true, false, 512, 1>(a, nd, smem, st);
   return launch_sweep_geo<T, TI, GT, false, false, 512, 1>(a, nd, smem, st);
 }
 
-// directions d0 .. d0 + nd - 1; S and I: element (cell, d0 + x, group) at cell * sc + x * sd + group
+// directions d0 .. d0 + nd - 1; S and I: element (cell, d0 + x, group) at q * sc + x * sd + group,
+// q the cell or its position in the direction's sweep order
 template <class T, class TI>
-rrhd_status launch_sweep(rrhd_ctx *c, int d0, int nd, const void *S, void *I, int64_t sc, int64_t sd, bool one_q) {
+rrhd_status launch_sweep(rrhd_ctx *c, int d0, int nd, const void *S, void *I, int64_t sc, int64_t sd, bool by_pos,
+                         bool one_q) {
   RadState &R = c->rad;
   SweepArgs<T, TI> a;
   a.N = c->N;
@@ -860,46 +971,51 @@ rrhd_status launch_sweep(rrhd_ctx *c, int d0, int nd, const void *S, void *I, in
   a.depth = R.d_depth;
   a.src = (const T *)R.d_src;
   a.slots = (T *)R.d_slots;
-  a.cap = slot_cap(R);
+  a.cap = (uint32_t)slot_cap(R, R.two);
   a.nhigh = R.nhigh;
   a.S = (const TI *)S;
   a.I = (TI *)I;
   a.sc = sc;
   a.sd = sd;
+  a.by_pos = by_pos;
   a.bc = (T)R.bc;
   cudaError_t e;
   switch (R.G) {
-    case 1: e = launch_sweep_groups<T, TI, 1>(a, R.nlow, R.M > kSweepSMs, nd, c->stream); break;
-    case 2: e = launch_sweep_groups<T, TI, 2>(a, R.nlow, R.M > kSweepSMs, nd, c->stream); break;
-    case 4: e = launch_sweep_groups<T, TI, 4>(a, R.nlow, R.M > kSweepSMs, nd, c->stream); break;
-    default: e = launch_sweep_groups<T, TI, 0>(a, R.nlow, R.M > kSweepSMs, nd, c->stream); break;
+    case 1: e = launch_sweep_groups<T, TI, 1>(a, R.nlow, R.two, nd, c->stream); break;
+    case 2: e = launch_sweep_groups<T, TI, 2>(a, R.nlow, R.two, nd, c->stream); break;
+    case 4: e = launch_sweep_groups<T, TI, 4>(a, R.nlow, R.two, nd, c->stream); break;
+    default: e = launch_sweep_groups<T, TI, 0>(a, R.nlow, R.two, nd, c->stream); break;
   }
   RRHD_CUDA(e);
   return RRHD_OK;
 }
 
-template <class V, bool IMPORT>
-cudaError_t launch_tile(rrhd_ctx *c, int64_t rows, int d0, int nd, const int32_t *perm, const void *in, void *out) {
-  const dim3 tiles((unsigned)((rows + 31) / 32), (unsigned)((nd + 31) / 32));
-  k_tile<V, IMPORT><<<tiles, 256, 0, c->stream>>>(rows, c->rad.G, c->rad.M, d0, nd, perm, (const V *)in, (V *)out);
-  return cudaGetLastError();
+// S and I in sweep order when a (cell, direction)'s values fill half a sector or more (32^3 x
+// 256 x 4 FP64, kernel and tiles 4.8 -> 4.0 ms); else by cell: values of 8 bytes of neighbouring
+// cells share sectors, and the coalesced tiles save more (48^3 x 256 x 1 FP64 6.1 -> 5.5 ms)
+template <class TI>
+bool by_position(const RadState &R) {
+  return R.d_pos != nullptr && sizeof(TI) * R.G >= 16;
 }
 
-struct alignas(8) Bytes8 { uint32_t w[2]; };
-struct alignas(16) Bytes16 { uint32_t w[4]; };
-struct alignas(16) Bytes32 { uint32_t w[8]; };
+template <class TI, class V, bool IMPORT>
+cudaError_t launch_tile(rrhd_ctx *c, int gw, int d0, int nd, const int32_t *perm, const void *in, void *out) {
+  const dim3 tiles((unsigned)((c->N * gw + 31) / 32), (unsigned)((nd + kTileDirs<V> - 1) / kTileDirs<V>));
+  k_tile<V, IMPORT><<<tiles, 256, 0, c->stream>>>(c->N, gw, c->rad.M, d0, nd, perm, by_position<TI>(c->rad) ? c->rad.d_pos : nullptr, (const V *)in,
+                                                  (V *)out);
+  return cudaGetLastError();
+}
 
 // S or I between the caller's arrays (rows, or [N][M][G] when cdg) and the sweep's layout
 template <class TI, bool IMPORT>
 cudaError_t move_tiles(rrhd_ctx *c, int d0, int nd, const void *in, void *out, bool cdg) {
   const RadState &R = c->rad;
-  const int64_t N = c->N;
-  if (!cdg) return launch_tile<TI, IMPORT>(c, N * R.G, d0, nd, c->d_perm, in, out);
+  if (!cdg) return launch_tile<TI, TI, IMPORT>(c, R.G, d0, nd, c->d_perm, in, out);
   switch (sizeof(TI) * R.G) {
-    case 4: return launch_tile<float, IMPORT>(c, N, d0, nd, nullptr, in, out);
-    case 8: return launch_tile<Bytes8, IMPORT>(c, N, d0, nd, nullptr, in, out);
-    case 16: return launch_tile<Bytes16, IMPORT>(c, N, d0, nd, nullptr, in, out);
-    case 32: return launch_tile<Bytes32, IMPORT>(c, N, d0, nd, nullptr, in, out);
+    case 4: return launch_tile<TI, float, IMPORT>(c, 1, d0, nd, nullptr, in, out);
+    case 8: return launch_tile<TI, Bytes8, IMPORT>(c, 1, d0, nd, nullptr, in, out);
+    case 16: return launch_tile<TI, Bytes16, IMPORT>(c, 1, d0, nd, nullptr, in, out);
+    case 32: return launch_tile<TI, Bytes32, IMPORT>(c, 1, d0, nd, nullptr, in, out);
     default: return cudaErrorNotSupported;
   }
 }
@@ -912,7 +1028,7 @@ rrhd_status run_sweep_t(rrhd_ctx *c, const void *S, void *I, bool cdg) {
   const int64_t rows = c->N * R.G;
   const size_t cd = sizeof(TI) * R.G;  // bytes of a (cell, direction)
   if (cdg && !(cd == 4 || cd == 8 || cd == 16 || cd == 32))
-    return launch_sweep<T, TI>(c, 0, R.M, S, I, (int64_t)R.M * R.G, R.G, true);
+    return launch_sweep<T, TI>(c, 0, R.M, S, I, (int64_t)R.M * R.G, R.G, false, true);
   if (!R.d_x) {
     // as many directions as there are, or as memory allows (at least one)
     R.xdirs = R.M;
@@ -926,7 +1042,7 @@ rrhd_status run_sweep_t(rrhd_ctx *c, const void *S, void *I, bool cdg) {
   for (int d0 = 0; d0 < R.M; d0 += R.xdirs) {
     const int nd = std::min(R.xdirs, R.M - d0);
     RRHD_CUDA((move_tiles<TI, true>(c, d0, nd, S, R.d_x, cdg)));
-    const rrhd_status s = launch_sweep<T, TI>(c, d0, nd, R.d_x, R.d_x, R.G, rows, cdg);
+    const rrhd_status s = launch_sweep<T, TI>(c, d0, nd, R.d_x, R.d_x, R.G, rows, by_position<TI>(R), cdg);
     if (s) return s;
     RRHD_CUDA((move_tiles<TI, false>(c, d0, nd, R.d_x, I, cdg)));
   }
@@ -976,21 +1092,22 @@ rrhd_status build_plan(rrhd_ctx *c) {
     R.d_ord = nullptr;
     return rrhd_fail(oom, "sweep plan allocation failed (%lld bytes)", (long long)(sizeof(uint4) * total));
   }
-  // The geometry stream (5 values an item) spares each item its cell's geometry record.  It
-  // is kept where the memory left holds it beside the intensity and scattering-integral
-  // arrays of a coupled step (or of a caller's sweep with its scratch); else the sweep forms
-  // the same values again from the records.
+  // The geometry stream (5 values an item) spares each item its cell's geometry record, and
+  // the cells' positions bring S and I into sweep order.  They are kept where the memory left
+  // holds them beside the intensity and scattering-integral arrays of a coupled step (or of a
+  // caller's sweep) and the sweep's scratch; else the sweep forms the same values again from
+  // the records and takes S and I by cell.
   {
     size_t free_b = 0, all_b = 0;
     RRHD_CUDA(cudaMemGetInfo(&free_b, &all_b));
-    const size_t one = sizeof(T) * (size_t)total;
+    const size_t one = sizeof(T) * (size_t)total, pos = sizeof(uint32_t) * (size_t)total;
     const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
     const size_t arrays = 3 * ti * (size_t)total * R.G;
-    if (5 * one + arrays <= free_b &&
+    if (5 * one + pos + arrays <= free_b &&
         (cudaMalloc(&R.d_dist, 2 * one) != cudaSuccess || cudaMalloc(&R.d_wgt, 2 * one) != cudaSuccess ||
-         cudaMalloc(&R.d_wgt3, one) != cudaSuccess)) {
+         cudaMalloc(&R.d_wgt3, one) != cudaSuccess || cudaMalloc(&R.d_pos, pos) != cudaSuccess)) {
       cudaGetLastError();
-      for (void **p : {&R.d_dist, &R.d_wgt, &R.d_wgt3}) {
+      for (void **p : {&R.d_dist, &R.d_wgt, &R.d_wgt3, (void **)&R.d_pos}) {
         cudaFree(*p);
         *p = nullptr;
       }
@@ -1007,18 +1124,17 @@ rrhd_status build_plan(rrhd_ctx *c) {
   uint32_t *const level = buf[0], *const key = buf[1], *const cell = buf[2], *const key2 = buf[3],
            *const order = buf[4], *const indeg = buf[5], *const queue = key;
   int32_t *d_count = (int32_t *)mem.get(sizeof(int32_t) * R.M);
-  unsigned int *d_max = (unsigned int *)mem.get(2 * sizeof(unsigned int));
-  if (!d_count || !d_max || cudaMalloc(&R.d_depth, sizeof(int32_t) * R.M) != cudaSuccess ||
+  int32_t *d_need = (int32_t *)mem.get(sizeof(int32_t) * R.M);
+  if (!d_count || !d_need || cudaMalloc(&R.d_depth, sizeof(int32_t) * R.M) != cudaSuccess ||
       cudaMalloc(&R.d_lvl_base, sizeof(int64_t) * R.M) != cudaSuccess)
     return rrhd_fail(oom, "sweep plan scratch");
   size_t sort_bytes = 0;
   RRHD_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, key, key2, cell, order, N * B, 0, 32, st));
   void *sort_tmp = mem.get(sort_bytes);
   if (!sort_tmp) return rrhd_fail(oom, "sweep plan scratch");
-  RRHD_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned int), st));
   R.depth.assign(R.M, 0);
   R.lvl_base.assign(R.M, 0);
-  std::vector<int32_t> count(R.M);
+  std::vector<int32_t> count(R.M), need(R.M, 0);
   const T *w = (const T *)R.d_w, *rec = (const T *)R.d_rec;
   // levels of every direction first: their number decides the sort keys and the offsets
   auto levels_of = [&](int d0, int nd) -> rrhd_status {
@@ -1065,17 +1181,14 @@ rrhd_status build_plan(rrhd_ctx *c) {
     auto items = [&]() -> rrhd_status {
       k_plan_items<T><<<nd, kPlanThreads, 0, st>>>(N, d0, w, rec, R.d_lvl, R.d_lvl_base, R.d_depth, order, indeg, key,
                                                    cell, R.d_ord, R.d_ord_hi, (const T *)R.d_wt, (T *)R.d_dist, (T *)R.d_wgt,
-                                                   (T *)R.d_wgt3, slot_cap(R), d_max);
+                                                   (T *)R.d_wgt3, R.d_pos, slot_cap(R, true), slot_cap(R, false), d_need);
       RRHD_CUDA(cudaGetLastError());
-      unsigned int m[2] = {0, 0};
-      RRHD_CUDA(cudaMemcpyAsync(m, d_max, sizeof m, cudaMemcpyDeviceToHost, st));
+      RRHD_CUDA(cudaMemcpyAsync(need.data() + d0, d_need + d0, sizeof(int32_t) * nd, cudaMemcpyDeviceToHost, st));
       RRHD_CUDA(cudaStreamSynchronize(st));
-      R.nlow = m[0];
-      R.nhigh = (int64_t)m[1] - slot_cap(R);
       return RRHD_OK;
     };
     if ((s = items())) return s;
-    if (std::max(R.nlow, slot_cap(R) + R.nhigh) > 65536 && !R.d_ord_hi) {
+    if (*std::max_element(need.begin(), need.end()) > 65536 && !R.d_ord_hi) {
       // slots beyond 16 bits: their upper halves in a second array (zero for the batches before)
       if (cudaMalloc(&R.d_ord_hi, sizeof(uint2) * total) != cudaSuccess) {
         cudaGetLastError();
@@ -1086,6 +1199,18 @@ rrhd_status build_plan(rrhd_ctx *c) {
       if ((s = items())) return s;
     }
   }
+  const int cap2 = slot_cap(R, true);
+  int64_t all = 0, beyond = 0, most = 0;
+  for (int32_t n : need) {
+    all += n;
+    beyond += std::max(0, n - cap2);
+    most = std::max<int64_t>(most, n);
+  }
+  const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
+  R.two = R.M > kSweepSMs && R.d_pos && ti * R.G >= 16 && (double)beyond <= kTwoBeyond * (double)all;
+  const int cap = slot_cap(R, R.two);
+  R.nlow = std::min<int64_t>(most, cap);
+  R.nhigh = std::max<int64_t>(0, most - cap);
   // rrhd_rad_plan_info: levels and the largest level over batches of R.DB directions
   std::vector<int32_t> off((size_t)entries);
   RRHD_CUDA(cudaMemcpyAsync(off.data(), R.d_lvl, sizeof(int32_t) * entries, cudaMemcpyDeviceToHost, st));
@@ -1108,7 +1233,7 @@ rrhd_status build_plan(rrhd_ctx *c) {
 
 void rrhd_rad_release(rrhd_ctx *c) {
   RadState &R = c->rad;
-  void *ptrs[] = {R.d_w,     R.d_rec, R.d_src, R.d_ord, R.d_ord_hi, R.d_dist, R.d_wgt, R.d_wgt3, R.d_wt, R.d_lvl, R.d_lvl_base, R.d_depth,
+  void *ptrs[] = {R.d_w,     R.d_rec, R.d_src, R.d_ord, R.d_ord_hi, R.d_dist, R.d_wgt, R.d_wgt3, R.d_wt, R.d_pos, R.d_lvl, R.d_lvl_base, R.d_depth,
                   R.d_slots, R.d_x,   R.d_I,   R.d_S,   R.d_G4,     R.d_mE,  R.d_mF,  R.d_mT,       R.d_mom,
                   R.d_cnt};
   for (void *p : ptrs) cudaFree(p);
