@@ -124,6 +124,23 @@ __device__ __forceinline__ void split4(const float (&x)[4], uint2 &hi, uint2 &lo
   }
 }
 
+// v + iso, iso = hi + lo (a double split in two floats), rounded to float once but for terms of
+// 2^-48: conversions to double and back run at a fraction of the FP32 rate and were a third of
+// the drain's store phase.  |v| <= hi (the kernel's anisotropic part is at most the isotropic
+// one); where their sum is not finite it is the result.
+__device__ __forceinline__ float add_iso(float v, float hi, float lo) {
+  const float s = __fadd_rn(hi, v);
+  const float r = __fadd_rn(__fsub_rn(v, __fsub_rn(s, hi)), lo);
+  return fabsf(s) < INFINITY ? __fadd_rn(s, r) : s;
+}
+
+// eight floats of one row, a whole 32-byte sector in one access (32-byte aligned)
+__device__ __forceinline__ void st_sector(float *p, const float4 &a, const float4 &b) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+               "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+
 struct TcParams {
   const float *I;
   float *S;
@@ -145,130 +162,171 @@ struct TcParams {
 //   mom    (MOM) the ten moments in FP64, stored as FP32 [rows][16] (columns 10-15 zero):
 //          the scaled forms take them from here, not from the tensor cores.
 // mw [10][M] holds (a_d / A) {1, wx, wy, wz, wx^2, wx wy, wx wz, wy^2, wy wz, wz^2}
-// (cuda_illum_sep_param.cu:9-69).  A warp takes four cells, eight lanes per cell: a cell's
-// values are NV = M NG / 4 float4 vectors (P = 4 / NG directions of NG groups each), lane q
-// takes vectors q, q + 8, q + 16, ..., so each load instruction reads a whole 128-byte line
-// of each of the four cells.  Each term is one fused multiply-add in FP64; the eight lanes'
-// partial sums are combined by a fixed butterfly (reduce-scatter over lane bits 4, 2, 1), the
-// same order for every cell.  The weight table sits in shared memory by (sub-direction,
-// vector), so the eight lanes of a cell read eight consecutive records (no bank conflicts).
+// (cuda_illum_sep_param.cu:9-69).  A contraction [rows x M] x [M x 10] on the FP64 matrix
+// instruction (mma.sync m8n8k4; the fifth-generation tensor cores take no FP64): a warp takes
+// 32 rows as four tiles of eight, two tiles of moments (8 + 2).  A lane's float4 loads hold
+// each value where its fragment wants it, with no exchange between lanes, because the order of
+// the directions in a k step and of the rows in a tile is free:
+//   NG = 1: rows g + 8 r (g = lane / 4), float4 f of row tile f: directions 4 t + s (t = lane % 4)
+//   NG = 2: cells g and g + 8, float4 f: cell set f / 2, directions 8 (f % 2) + 2 t + (0, 1);
+//           row tile 2 (f / 2) + group
+//   NG = 4: cell g, float4 f: direction 4 f + t, its component the group = row tile
+// for k steps s = 0 .. 3 of every 16 directions, and the table in shared memory follows that
+// order, 12 doubles a direction (no bank conflicts).  One table load serves 4 x 256
+// multiply-adds; one thread's plain FMAs loaded ten doubles for four rows and were bound by
+// that: 663,552 rows x 256 directions 0.35 -> 0.17 ms.
 constexpr int kPrepassThreads = 256;
-template <int NG, bool MOM>
-__global__ void __launch_bounds__(kPrepassThreads, 2) k_row_prepass(const float *__restrict__ I, int64_t rows, int M,
+constexpr int kPrepassPitch = 12;
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+// SPLIT: the four warps of a CTA share a task, a quarter of the directions each (small calls)
+template <int NG, bool MOM, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 128 : kPrepassThreads, 2) k_row_prepass(const float *__restrict__ I, int64_t rows, int M,
                                                                  const double *__restrict__ mw,
                                                                  float *__restrict__ scale, double *__restrict__ erow,
                                                                  float *__restrict__ mom) {
   constexpr int NM = MOM ? 10 : 1;
-  constexpr int P = 4 / NG;                 // directions per float4
-  constexpr int V = NG * NM;                // sums per cell
-  constexpr int VP = (V + 7) / 8 * 8;       // padded to the reduce-scatter's eight lanes
-  extern __shared__ double2 smw2[];         // [P][M / P][NM]
+  extern __shared__ double2 smw2[];  // [M / 16][k step][t][kPrepassPitch], then the same order without moments
   double *smw = reinterpret_cast<double *>(smw2);
-  const int MP = M / P;
-  for (int x = threadIdx.x; x < NM * M; x += blockDim.x) {
-    const int k = x / M, d = x - k * M;
-    smw[((d % P) * MP + d / P) * NM + k] = __ldg(mw + x);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, q = lane & 7;
-  const int NV = M * NG / 4;  // float4 per cell, a multiple of 8
-  const int64_t cells = rows / NG;
-  const int64_t quads = (cells + 3) / 4;
-  const int64_t wid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const float4 *I4 = reinterpret_cast<const float4 *>(I);
-  // the four cells of a group are contiguous (16 NV bytes each): one lane asks L2 for the
-  // warp's next group while the warp works on this one, so that the lanes' loads find it there
-  auto prefetch = [&](int64_t g4) {
-    if (lane == 0 && g4 < quads) {
-      const int64_t n = min((int64_t)4, cells - 4 * g4) * NV * 16;  // bytes, a multiple of 16
-      const float4 *src = I4 + 4 * g4 * NV;
+  constexpr int PITCH = MOM ? kPrepassPitch : 1;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int64_t tasks = (rows + 31) / 32;
+  const int warp = threadIdx.x >> 5;
+  const int64_t wid = SPLIT ? blockIdx.x : (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = SPLIT ? gridDim.x : ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int nj = M / 16;  // a multiple of 4
+  // the 32 rows of a task are contiguous: one lane asks L2 for the warp's next ones
+  auto prefetch = [&](int64_t task) {
+    if (lane == 0 && task < tasks) {
+      const int64_t n = min((int64_t)32, rows - 32 * task) * M * 4;  // bytes, a multiple of 16
+      const char *src = reinterpret_cast<const char *>(I + 32 * task * M);
       for (int64_t o = 0; o < n; o += 65536)
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(reinterpret_cast<const char *>(src) + o),
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src + o),
                      "r"((uint32_t)min((int64_t)65536, n - o))
                      : "memory");
     }
   };
-  prefetch(wid);
-  for (int64_t c4 = wid; c4 < quads; c4 += nw) {  // warp-uniform
-    prefetch(c4 + nw);
-    const int64_t c = c4 * 4 + (lane >> 3);
-    const bool valid = c < cells;
-    double acc[VP];
+  if (!SPLIT || warp == 0) prefetch(wid);
+  for (int d = threadIdx.x; d < M; d += blockDim.x) {
+    const int q = d & 15;
+    const int ks = NG == 1 ? q & 3 : NG == 2 ? 2 * (q >> 3) + (q & 1) : q >> 2;
+    const int kt = NG == 1 ? q >> 2 : NG == 2 ? (q & 7) >> 1 : q & 3;
+    double w[NM];
 #pragma unroll
-    for (int k = 0; k < VP; k++) acc[k] = 0.0;
-    float mx[NG];
+    for (int k = 0; k < NM; k++) w[k] = __ldg(mw + (int64_t)k * M + d);
 #pragma unroll
-    for (int g = 0; g < NG; g++) mx[g] = 0.f;
-    if (valid) {
-      const float4 *row = I4 + c * NV;
-#pragma unroll 2
-      for (int v = q; v < NV; v += 8) {
-        const float4 x = __ldcs(row + v);
-        const float e[4] = {x.x, x.y, x.z, x.w};
+    for (int k = 0; k < NM; k++) smw[((d >> 4) * 16 + 4 * ks + kt) * PITCH + k] = w[k];
+  }
+  __syncthreads();
+  for (int64_t task = wid; task < tasks; task += nw) {  // warp-uniform
+    if (!SPLIT) prefetch(task + nw);
+    const int64_t row0 = 32 * task;
+    // row of this lane in row tile r
+    auto row_of = [&](int r) {
+      return NG == 1 ? row0 + g + 8 * r : NG == 2 ? row0 + 2 * (g + 8 * (r >> 1)) + (r & 1) : row0 + 4 * g + r;
+    };
+    // this lane's float4 f of the 16 directions j (its rows are valid or not together)
+    const float4 *src[4];
+    bool ok[4];
 #pragma unroll
-        for (int s = 0; s < P; s++) {
-          double w[NM];
-          const double2 *wr = smw2 + ((s * MP + v) * NM) / 2;
-          if constexpr (MOM) {
-#pragma unroll
-            for (int j = 0; j < NM / 2; j++) {
-              const double2 t = wr[j];
-              w[2 * j] = t.x;
-              w[2 * j + 1] = t.y;
-            }
-          } else {
-            w[0] = smw[s * MP + v];
-          }
-#pragma unroll
-          for (int g = 0; g < NG; g++) {
-            const float val = e[s * NG + g];
-            mx[g] = fmaxf(mx[g], fabsf(val));
-#pragma unroll
-            for (int k = 0; k < NM; k++) acc[g * NM + k] = __fma_rn((double)val, w[k], acc[g * NM + k]);
-          }
-        }
-      }
+    for (int f = 0; f < 4; f++) {
+      const int64_t r = row_of(NG == 1 ? f : NG == 2 ? (f & 2) : 0);
+      ok[f] = r < rows;
+      const int64_t first = NG == 1 ? r * M + 4 * t : NG == 2 ? r * M + (8 * (f & 1) + 2 * t) * 2 : r * M + (4 * f + t) * 4;
+      src[f] = reinterpret_cast<const float4 *>(I + (ok[f] ? first : 0));
     }
-    // the group maxima to every lane of the cell; the sums reduce-scattered
+    constexpr int STEP = 4 * NG;  // float4s from one j to the next
+    double acc[4][2][2];
+    float mx[4];
 #pragma unroll
-    for (int o = 4; o >= 1; o >>= 1)
-#pragma unroll
-      for (int g = 0; g < NG; g++) mx[g] = fmaxf(mx[g], __shfl_xor_sync(0xffffffffu, mx[g], o));
-#pragma unroll
-    for (int o = 4, h = VP / 2; o >= 1; o >>= 1, h >>= 1) {
-      const bool up = lane & o;
-#pragma unroll
-      for (int k = 0; k < VP / 2; k++) {
-        if (k < h) {
-          const double send = up ? acc[k] : acc[h + k];
-          const double keep = up ? acc[h + k] : acc[k];
-          acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-      }
+    for (int r = 0; r < 4; r++) {
+      acc[r][0][0] = acc[r][0][1] = acc[r][1][0] = acc[r][1][1] = 0.0;
+      mx[r] = 0.f;
     }
-    // this lane now holds sums base .. base + VP/8 - 1 of its cell
-    const int base = ((lane >> 2) & 1) * (VP / 2) + ((lane >> 1) & 1) * (VP / 4) + (lane & 1) * (VP / 8);
+    auto load = [&](int j, float4 (&x)[4]) {
 #pragma unroll
-    for (int k = 0; k < VP / 8; k++) {
-      const int f = base + k;
-      if (valid && f < V) {
-        const int g = f / NM, kk = f - g * NM;
-        const int64_t r = c * NG + g;
-        if (kk == 0) {
-          float m = mx[0];
+      for (int f = 0; f < 4; f++) x[f] = ok[f] ? __ldcs(src[f] + j * STEP) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto work = [&](int j, const float4 (&x)[4]) {
+      const double *b = smw + (j * 16 + t) * PITCH;
 #pragma unroll
-          for (int gg = 1; gg < NG; gg++)
-            if (g == gg) m = mx[gg];
-          scale[r] = (m > 0.f && isfinite(m)) ? ldexpf(1.f, 14 - ilogbf(m)) : 1.f;
-          erow[r] = acc[k];
-        }
+      for (int s = 0; s < 4; s++) {
+        const double *bs = b + 4 * s * PITCH;
+        double b0, b1 = 0.0;
         if (MOM) {
-          mom[16 * r + kk] = (float)acc[k];
-          if (kk == NM - 1)
-#pragma unroll
-            for (int z = NM; z < 16; z++) mom[16 * r + z] = 0.f;
+          b0 = bs[g];
+          if (g < 2) b1 = bs[8 + g];
+        } else {
+          b0 = g == 0 ? bs[0] : 0.0;
         }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const float4 v = NG == 1 ? x[r] : NG == 2 ? x[2 * (r >> 1) + (s >> 1)] : x[s];
+          const int comp = NG == 1 ? s : NG == 2 ? 2 * (s & 1) + (r & 1) : r;
+          const float a = comp == 0 ? v.x : comp == 1 ? v.y : comp == 2 ? v.z : v.w;
+          mx[r] = fmaxf(mx[r], fabsf(a));
+          dmma(acc[r][0], (double)a, b0);
+          if (MOM) dmma(acc[r][1], (double)a, b1);
+        }
+      }
+    };
+    constexpr int D = 2;               // sets of 16 directions in flight
+    constexpr int JS = SPLIT ? 4 : 1;  // a warp's sets are j0, j0 + JS, ...
+    const int j0 = SPLIT ? warp : 0;
+    float4 x[D][4];
+#pragma unroll
+    for (int i = 0; i < D; i++)
+      if (!SPLIT || j0 + JS * i < nj) load(j0 + JS * i, x[i]);
+    for (int j = j0; j < nj; j += JS * D) {
+#pragma unroll
+      for (int i = 0; i < D; i++) {
+        if (!SPLIT || j + JS * i < nj) work(j + JS * i, x[i]);
+        if (j + JS * (i + D) < nj) load(j + JS * (i + D), x[i]);
+      }
+    }
+    if constexpr (SPLIT) {  // the warps' sums in order, and the largest of their maxima
+      __shared__ double part[3][18][32];
+      __syncthreads();
+      if (warp > 0) {
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+#pragma unroll
+          for (int q = 0; q < 4; q++) part[warp - 1][4 * r + q][lane] = acc[r][q >> 1][q & 1];
+        }
+        float2 *m = reinterpret_cast<float2 *>(&part[warp - 1][16][lane]);
+        m[0] = make_float2(mx[0], mx[1]);
+        m[32] = make_float2(mx[2], mx[3]);
+      }
+      __syncthreads();
+      if (warp > 0) continue;
+#pragma unroll
+      for (int w = 0; w < 3; w++) {
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) acc[r][q >> 1][q & 1] += part[w][4 * r + q][lane];
+        const float2 *m = reinterpret_cast<const float2 *>(&part[w][16][lane]);
+        mx[0] = fmaxf(mx[0], m[0].x), mx[1] = fmaxf(mx[1], m[0].y);
+        mx[2] = fmaxf(mx[2], m[32].x), mx[3] = fmaxf(mx[3], m[32].y);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+#pragma unroll
+      for (int o = 1; o <= 2; o <<= 1) mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], o));
+      const int64_t row = row_of(r);
+      if (row >= rows) continue;
+      if (t == 0) {
+        scale[row] = (mx[r] > 0.f && isfinite(mx[r])) ? ldexpf(1.f, 14 - ilogbf(mx[r])) : 1.f;
+        erow[row] = acc[r][0][0];
+      }
+      if (MOM) {
+        float2 *o = reinterpret_cast<float2 *>(mom + 16 * row);
+        o[t] = make_float2((float)acc[r][0][0], (float)acc[r][0][1]);
+        o[4 + t] = t == 0 ? make_float2((float)acc[r][1][0], (float)acc[r][1][1]) : make_float2(0.f, 0.f);
       }
     }
   }
@@ -560,7 +618,10 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       if (ok && gr < P.rows) {
         const float inv = (SCALED ? 1.f / __ldg(P.scale + gr) : 1.f) * P.b_unscale;
-        const double eiso = SCALED ? __ldg(P.erow + gr) : 0.0;  // the isotropic part, added in FP64
+        const double eiso = SCALED ? kIsoWeight * __ldg(P.erow + gr) : 0.0;  // the isotropic part
+        const float iso_hi = (float)eiso, iso_lo = fabsf(iso_hi) < INFINITY ? (float)(eiso - (double)iso_hi) : 0.f;
+        const bool sector = (reinterpret_cast<uintptr_t>(P.S) & 31) == 0;
+        float4 held = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < MAX_HALF / 4; j++) {
           const int col = c0 + 4 * j;
@@ -568,10 +629,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             float4 v = make_float4(run[4 * j] * inv, run[4 * j + 1] * inv, run[4 * j + 2] * inv,
                                    run[4 * j + 3] * inv);
             if (SCALED && col < nS) {
-              v.x = (float)((double)v.x + kIsoWeight * eiso);
-              v.y = (float)((double)v.y + kIsoWeight * eiso);
-              v.z = (float)((double)v.z + kIsoWeight * eiso);
-              v.w = (float)((double)v.w + kIsoWeight * eiso);
+              v.x = add_iso(v.x, iso_hi, iso_lo);
+              v.y = add_iso(v.y, iso_hi, iso_lo);
+              v.z = add_iso(v.z, iso_hi, iso_lo);
+              v.w = add_iso(v.w, iso_hi, iso_lo);
             }
             if (col < nS) {
               if constexpr (NG > 1) {
@@ -581,7 +642,13 @@ __global__ void __launch_bounds__(THREADS, 1)
                 o[2 * NG] = v.z;
                 o[3 * NG] = v.w;
               } else {
-                *reinterpret_cast<float4 *>(P.S + gr * P.M + nt * NT + col) = v;
+                // columns come in eights (c0 is a multiple of 8): a sector per access
+                float *o = P.S + gr * P.M + nt * NT + col;
+                if (!sector)
+                  *reinterpret_cast<float4 *>(o) = v;
+                else if (j % 2 == 1)
+                  st_sector(o - 4, held, v);
+                held = v;
               }
             } else
               *reinterpret_cast<float4 *>(P.mom + gr * NMOM + (col - nS)) = v;
@@ -982,6 +1049,7 @@ __global__ void __launch_bounds__(R_THREADS, 1)
     const int q = warp & 3, hf = (warp - R_DRAIN0) >> 2;
     const int row = q * 32 + lane;
     const int64_t ncell = P.rows / NG;
+    const bool sector = (reinterpret_cast<uintptr_t>(P.S) & 31) == 0;
     int64_t g = 0;
     bool ok = true;
     for (int64_t rt = blockIdx.x; rt < n_rt && ok && !*abort_flag; rt += gridDim.x) {
@@ -989,7 +1057,8 @@ __global__ void __launch_bounds__(R_THREADS, 1)
       const int64_t cell = gr / NG;  // the quad (pair) of lanes holding one cell's groups
       // the row's unscale factor, loaded before the sums arrive
       const float inv = (SCALED ? 1.f / (gr < P.rows ? __ldg(P.scale + gr) : 1.f) : 1.f) * P.b_unscale;
-      const double eiso = (SCALED && gr < P.rows) ? __ldg(P.erow + gr) : 0.0;  // the isotropic part, in FP64
+      const double eiso = (SCALED && gr < P.rows) ? kIsoWeight * __ldg(P.erow + gr) : 0.0;  // the isotropic part
+      const float iso_hi = (float)eiso, iso_lo = fabsf(iso_hi) < INFINITY ? (float)(eiso - (double)iso_hi) : 0.f;
       for (int h = 0; h < n_h && ok; h++) {
         const bool with_mom = (h == 0) && mom;
         const int half = (nS + (with_mom ? NMOM : 0)) >> 1;  // multiple of 8
@@ -1040,6 +1109,7 @@ __global__ void __launch_bounds__(R_THREADS, 1)
                                    : NG == 2 ? (cell * P.M + h * nS + c0 + 2 * (lane & 1)) * 2
                                              : gr * P.M + h * nS + c0);
         const bool row_ok = NG > 1 ? cell < ncell : gr < P.rows;
+        float4 held = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < MAX_HALF / 4; j++) {
           const int col = c0 + 4 * j;
@@ -1047,7 +1117,7 @@ __global__ void __launch_bounds__(R_THREADS, 1)
             float v[4] = {run[4 * j] * inv, run[4 * j + 1] * inv, run[4 * j + 2] * inv, run[4 * j + 3] * inv};
             if (SCALED && col < nS) {
 #pragma unroll
-              for (int i = 0; i < 4; i++) v[i] = (float)((double)v[i] + kIsoWeight * eiso);
+              for (int i = 0; i < 4; i++) v[i] = add_iso(v[i], iso_hi, iso_lo);
             }
             if (col < nS) {
               if constexpr (NG == 4) {
@@ -1060,7 +1130,14 @@ __global__ void __launch_bounds__(R_THREADS, 1)
                 ungroup2(v, lane, x);
                 if (row_ok) __stcs(reinterpret_cast<float4 *>(so + 8 * j), make_float4(x[0], x[1], x[2], x[3]));
               } else {
-                if (row_ok) __stcs(reinterpret_cast<float4 *>(so + 4 * j), make_float4(v[0], v[1], v[2], v[3]));
+                // columns come in eights (c0 is a multiple of 8): a sector per access
+                const float4 x = make_float4(v[0], v[1], v[2], v[3]);
+                if (!sector) {
+                  if (row_ok) __stcs(reinterpret_cast<float4 *>(so + 4 * j), x);
+                } else if (j % 2 == 1 && row_ok) {
+                  st_sector(so + 4 * j - 4, held, x);
+                }
+                held = x;
               }
             } else if (gr < P.rows) {
               *reinterpret_cast<float4 *>(P.mom + gr * NMOM + (col - nS)) = make_float4(v[0], v[1], v[2], v[3]);
@@ -1230,6 +1307,23 @@ extern "C" rrhd_status rrhd_scatter_tc_destroy(rrhd_scatter_tc *t) {
   return RRHD_OK;
 }
 
+// A warp per 32 rows, two resident CTAs of eight warps an SM, where the rows fill half of them;
+// else four warps per 32 rows (one warp's chain of 128 dependent matrix instructions at M = 512
+// is most of a small call: 2,000 rows, both kernels, 43 -> 33 us).
+template <int NG, bool MOM>
+static cudaError_t launch_prepass(const rrhd_scatter_tc *t, const float *I, int64_t rows, float *mom, cudaStream_t st) {
+  const int64_t tasks = (rows + 31) / 32;
+  const bool small = tasks < 8 * t->num_sms;
+  const int nt = small ? 128 : kPrepassThreads;
+  const unsigned nb = (unsigned)(small ? tasks : std::min<int64_t>((tasks + 7) / 8, 2 * t->num_sms));
+  const size_t smem = sizeof(double) * (MOM ? kPrepassPitch : 1) * t->M;  // <= 96 KiB (M <= 1024)
+  auto *k = small ? k_row_prepass<NG, MOM, true> : k_row_prepass<NG, MOM, false>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k<<<nb, nt, smem, st>>>(I, rows, t->M, t->d_mw, t->d_scale, t->d_erow, mom);
+  return cudaGetLastError();
+}
+
 // NG = 1: I, S are [rows][M]; NG = 2, 4: [rows / NG][M][NG] (row = cell * NG + group)
 template <int FORM, int NG>
 static rrhd_status launch_tc(const rrhd_scatter_tc *t, const float *I, float *S, float *mom, int64_t rows,
@@ -1242,22 +1336,8 @@ static rrhd_status launch_tc(const rrhd_scatter_tc *t, const float *I, float *S,
   }
   constexpr bool SCALED = (FORM == FORM_F16X3 || FORM == FORM_F16);
   if (SCALED) {
-    // a warp per four cells
-    const unsigned nb = (unsigned)std::min<int64_t>((rows / ng + 4 * (kPrepassThreads / 32) - 1) /
-                                                        (4 * (kPrepassThreads / 32)), 8 * t->num_sms);
-    const size_t wbytes = sizeof(double) * (mom ? 10 : 1) * t->M;  // <= 80 KiB (M <= 1024)
-    if (mom) {
-      static bool attr = false;
-      if (!attr) {
-        RRHD_CUDA(cudaFuncSetAttribute(k_row_prepass<NG, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(sizeof(double) * 10 * 1024)));
-        attr = true;
-      }
-      k_row_prepass<NG, true><<<nb, kPrepassThreads, wbytes, st>>>(I, rows, t->M, t->d_mw, t->d_scale, t->d_erow, mom);
-    } else {
-      k_row_prepass<NG, false><<<nb, kPrepassThreads, wbytes, st>>>(I, rows, t->M, t->d_mw, t->d_scale, t->d_erow, nullptr);
-    }
-    RRHD_CUDA(cudaGetLastError());
+    const cudaError_t e = mom ? launch_prepass<NG, true>(t, I, rows, mom, st) : launch_prepass<NG, false>(t, I, rows, mom, st);
+    RRHD_CUDA(e);
   }
   // the scaled forms' moments come from the pre-pass, in FP64
   TcParams P{I, S, SCALED ? nullptr : mom, t->d_scale, t->d_erow, rows, t->M, t->b_unscale, t->d_err, t->copies};
