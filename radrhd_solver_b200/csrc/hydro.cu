@@ -318,6 +318,42 @@ __global__ void k_get_state(int64_t N, double *W, int64_t sw, double *U, int64_t
     for (int k = 0; k < 5; k++) W[i * sw + k] = src[5 + k];
 }
 
+// Both arrays packed ([N][5]): a CTA moves 128 cells through shared memory, so that the caller's
+// side moves whole lines and a cell's 80 bytes are five 16-byte accesses of neighbouring threads
+// (one thread a cell strode 40 and 80 bytes): 1,572,864 cells, set 152 -> 60 us, get 88 -> 60 us.
+// Bound: HBM (320 B a cell).
+constexpr int kStateCells = 128;
+template <bool SET>
+__global__ void __launch_bounds__(256) k_move_state(int64_t N, double *W, double *U, const int32_t *iperm,
+                                                    double *state) {
+  __shared__ __align__(16) double rec[kStateCells][10];
+  __shared__ int32_t at[kStateCells];
+  const int64_t c0 = (int64_t)blockIdx.x * kStateCells;
+  const int n = (int)min((int64_t)kStateCells, N - c0);
+  for (int q = threadIdx.x; q < n; q += 256) at[q] = iperm[c0 + q];
+  if (SET)
+    for (int q = threadIdx.x; q < 5 * n; q += 256) {
+      rec[q / 5][q % 5] = __ldcs(U + 5 * c0 + q);
+      rec[q / 5][5 + q % 5] = __ldcs(W + 5 * c0 + q);
+    }
+  __syncthreads();
+  for (int q = threadIdx.x; q < 5 * n; q += 256) {
+    const int c = q / 5, k = q % 5;
+    double2 *g = reinterpret_cast<double2 *>(state + 10 * (size_t)at[c]) + k;
+    double2 *s = reinterpret_cast<double2 *>(&rec[c][2 * k]);
+    if (SET)
+      *g = *s;
+    else
+      *s = *g;
+  }
+  if (SET) return;
+  __syncthreads();
+  for (int q = threadIdx.x; q < 5 * n; q += 256) {
+    __stcs(U + 5 * c0 + q, rec[q / 5][q % 5]);
+    __stcs(W + 5 * c0 + q, rec[q / 5][5 + q % 5]);
+  }
+}
+
 __global__ void k_prim2con_state(int64_t N, Eos eos, double *state) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= N) return;
@@ -492,6 +528,20 @@ __global__ void k_p2c_batch(Eos eos, double *W, double *U, int64_t n) {
 }
 
 inline unsigned grid1d(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
+
+void move_state(rrhd_ctx *c, double *W, double *U, int64_t stride, double *state, bool set) {
+  const int64_t N = c->N;
+  if (W && U && stride == 5) {
+    if (set)
+      k_move_state<true><<<grid1d(N, kStateCells), 256, 0, c->stream>>>(N, W, U, c->d_iperm, state);
+    else
+      k_move_state<false><<<grid1d(N, kStateCells), 256, 0, c->stream>>>(N, W, U, c->d_iperm, state);
+  } else if (set) {
+    k_set_state<<<grid1d(N, 256), 256, 0, c->stream>>>(N, W, stride, U, stride, c->d_iperm, state);
+  } else {
+    k_get_state<<<grid1d(N, 256), 256, 0, c->stream>>>(N, W, stride, U, stride, c->d_iperm, state);
+  }
+}
 
 Eos make_eos(int eos, double gamma) {
   Eos e;
@@ -710,10 +760,7 @@ static rrhd_status state_transfer(rrhd_ctx *c, double *W, double *U, int64_t str
   const int64_t N = c->N;
   double *state = c->d_state[c->cur];
   if (where == RRHD_DEVICE) {
-    if (set)
-      k_set_state<<<grid1d(N, 256), 256, 0, c->stream>>>(N, W, stride, U, stride, c->d_iperm, state);
-    else
-      k_get_state<<<grid1d(N, 256), 256, 0, c->stream>>>(N, W, stride, U, stride, c->d_iperm, state);
+    move_state(c, W, U, stride, state, set);
     RRHD_CUDA(cudaGetLastError());
     return RRHD_OK;
   }
@@ -733,13 +780,11 @@ static rrhd_status state_transfer(rrhd_ctx *c, double *W, double *U, int64_t str
     }
     if (W) RRHD_CUDA(cudaMemcpyAsync(dW, stride == 5 ? W : hW, bytes, cudaMemcpyHostToDevice, c->stream));
     if (U) RRHD_CUDA(cudaMemcpyAsync(dU, stride == 5 ? U : hU, bytes, cudaMemcpyHostToDevice, c->stream));
-    k_set_state<<<grid1d(N, 256), 256, 0, c->stream>>>(N, W ? dW : nullptr, 5, U ? dU : nullptr, 5,
-                                                        c->d_iperm, state);
+    move_state(c, W ? dW : nullptr, U ? dU : nullptr, 5, state, true);
     RRHD_CUDA(cudaGetLastError());
     if (stride != 5) RRHD_CUDA(cudaStreamSynchronize(c->stream));
   } else {
-    k_get_state<<<grid1d(N, 256), 256, 0, c->stream>>>(N, W ? dW : nullptr, 5, U ? dU : nullptr, 5,
-                                                        c->d_iperm, state);
+    move_state(c, W ? dW : nullptr, U ? dU : nullptr, 5, state, false);
     RRHD_CUDA(cudaGetLastError());
     if (W) RRHD_CUDA(cudaMemcpyAsync(stride == 5 ? W : hW, dW, bytes, cudaMemcpyDeviceToHost, c->stream));
     if (U) RRHD_CUDA(cudaMemcpyAsync(stride == 5 ? U : hU, dU, bytes, cudaMemcpyDeviceToHost, c->stream));
