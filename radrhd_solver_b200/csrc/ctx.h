@@ -127,6 +127,8 @@ struct rrhd_ctx {
   uint8_t *d_status = nullptr;  // [N] status of the last step (new numbering)
 
   rrhd::StepScalars *d_scal = nullptr;  // [2]
+  rrhd::StepScalars *h_scal = nullptr;  // mapped host copy for steps that report
+  unsigned int *d_ticket = nullptr;     // CTAs of such a step that have added their share
   int scal_cur = 0;
 
   // split of the hydro step over ranks (rrhd_hydro_set_part): this context updates the

@@ -61,6 +61,8 @@ struct StepParams {
   double *__restrict__ face_flux;
   const StepScalars *prev;
   StepScalars *out;
+  StepScalars *host;        // mapped host copy of `out` (kReport)
+  unsigned int *ticket;     // CTAs that have added their share (0 between steps)
   double tau;
   int device_tau;
   double cfl_hmin;
@@ -140,8 +142,10 @@ __device__ __forceinline__ void load_state_smem(const double *s, int slot, doubl
 #define RRHD_STEP_MIN_BLOCKS 3  // CTAs per SM the register budget is sized for
 #endif
 // kFaceFlux: also write every face's flux to P.face_flux (caller numbering), for
-// rrhd_keep_face_flux; a separate instantiation keeps the common one lean.
-template <bool kFaceFlux>
+// rrhd_keep_face_flux; kReport: the last CTA also writes the step's scalars to mapped host
+// memory (a copy after the kernel and its wait cost a step of 120,000 cells 5 of 57 us).
+// Separate instantiations keep the common one lean.
+template <bool kFaceFlux, bool kReport>
 __global__ void __launch_bounds__(kStepThreads, RRHD_STEP_MIN_BLOCKS) k_hydro_step(const StepParams P) {
   extern __shared__ double2 smem_raw[];
   double *sstate = reinterpret_cast<double *>(smem_raw);      // [cpb + max_halo][10]
@@ -292,6 +296,20 @@ __global__ void __launch_bounds__(kStepThreads, RRHD_STEP_MIN_BLOCKS) k_hydro_st
     if (s_cnt[0]) atomicAdd(&P.out->n_fallback, s_cnt[0]);
     if (s_cnt[1]) atomicAdd(&P.out->n_failed, s_cnt[1]);
     if (blockIdx.x == 0) P.out->tau = tau;
+    if (kReport) {
+      __threadfence();
+      if (atomicAdd(P.ticket, 1u) == gridDim.x - 1) {
+        __threadfence();
+        const volatile StepScalars *o = P.out;
+        volatile StepScalars *h = P.host;
+        h->max_speed = o->max_speed;
+        h->tau = o->tau;
+        h->n_fallback = o->n_fallback;
+        h->n_failed = o->n_failed;
+        *P.ticket = 0u;
+        __threadfence_system();
+      }
+    }
   }
 }
 
@@ -564,11 +582,12 @@ void free_ctx(rrhd_ctx *c) {
   rrhd_rad_release(c);
   void *ptrs[] = {c->d_perm, c->d_iperm, c->d_bface_off, c->d_bface_rec, c->d_halo_off, c->d_halo_ids,
                   c->d_bface_gid, c->d_cell_rec, c->d_state[0],
-                  c->d_state[1], c->d_status, c->d_scal, c->d_face_flux, c->d_scratch_io,
+                  c->d_state[1], c->d_status, c->d_scal, c->d_ticket, c->d_face_flux, c->d_scratch_io,
                   c->d_send_ids, c->d_recv_ids};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (c->h_pinned) cudaFreeHost(c->h_pinned);
+  if (c->h_scal) cudaFreeHost(c->h_scal);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -698,11 +717,14 @@ extern "C" rrhd_status rrhd_create(const rrhd_mesh_desc *m, const rrhd_opts *opt
   const size_t ssz = sizeof(double) * 10 * N;
   if (cudaMalloc(&c->d_state[0], ssz) != cudaSuccess || cudaMalloc(&c->d_state[1], ssz) != cudaSuccess ||
       cudaMalloc(&c->d_status, N) != cudaSuccess || cudaMalloc(&c->d_scal, 2 * sizeof(StepScalars)) != cudaSuccess ||
+      cudaMalloc(&c->d_ticket, sizeof(unsigned int)) != cudaSuccess ||
+      cudaHostAlloc(&c->h_scal, sizeof(StepScalars), cudaHostAllocMapped) != cudaSuccess ||
       cudaMalloc(&c->d_scratch_io, ssz) != cudaSuccess)
     return fail(rrhd_fail(RRHD_ERR_OOM, "device allocation of the state failed"));
   cudaMemset(c->d_state[0], 0, ssz);
   cudaMemset(c->d_state[1], 0, ssz);
   cudaMemset(c->d_status, 0, N);
+  cudaMemset(c->d_ticket, 0, sizeof(unsigned int));
   StepScalars init[2] = {{0, 0, 0, 0}, {1.0, 0, 0, 0}};  // rhllc::max_signal_speed = 1 initially
   cudaMemcpy(c->d_scal, init, sizeof init, cudaMemcpyHostToDevice);
   c->scal_cur = 0;
@@ -713,9 +735,9 @@ extern "C" rrhd_status rrhd_create(const rrhd_mesh_desc *m, const rrhd_opts *opt
   c->step_smem = smem;
   if (smem > 227 * 1024)
     return fail(rrhd_fail(RRHD_ERR_LIMIT, "step needs %zu B of shared memory per CTA; lower cells_per_block", smem));
-  if (cudaFuncSetAttribute(k_hydro_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_hydro_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return fail(rrhd_fail(RRHD_ERR_LIMIT, "cannot reserve %zu B of shared memory", smem));
+  for (auto *k : {k_hydro_step<false, false>, k_hydro_step<false, true>, k_hydro_step<true, false>, k_hydro_step<true, true>})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return fail(rrhd_fail(RRHD_ERR_LIMIT, "cannot reserve %zu B of shared memory", smem));
   if (cudaDeviceSynchronize() != cudaSuccess) return fail(rrhd_fail(RRHD_ERR_CUDA, "%s", cudaGetErrorString(cudaGetLastError())));
   *out = c;
   return RRHD_OK;
@@ -862,22 +884,22 @@ extern "C" rrhd_status rrhd_hydro_step(rrhd_ctx *c, double tau, rrhd_step_stats 
   P.face_flux = c->keep_face_flux ? c->d_face_flux : nullptr;
   P.prev = c->d_scal + (c->scal_cur ^ 1);
   P.out = c->d_scal + c->scal_cur;
+  P.host = c->h_scal;
+  P.ticket = c->d_ticket;
   P.tau = tau;
   P.device_tau = tau <= 0 ? 1 : 0;
   P.cfl_hmin = c->cfl * c->h_min;
   P.bc = c->bc;
   RRHD_CUDA(cudaMemsetAsync(P.out, 0, sizeof(StepScalars), c->stream));
-  if (P.face_flux)
-    k_hydro_step<true><<<c->part_b1 - c->part_b0, kStepThreads, c->step_smem, c->stream>>>(P);
-  else
-    k_hydro_step<false><<<c->part_b1 - c->part_b0, kStepThreads, c->step_smem, c->stream>>>(P);
+  auto *k = P.face_flux ? (stats ? k_hydro_step<true, true> : k_hydro_step<true, false>)
+                        : (stats ? k_hydro_step<false, true> : k_hydro_step<false, false>);
+  k<<<c->part_b1 - c->part_b0, kStepThreads, c->step_smem, c->stream>>>(P);
   RRHD_CUDA(cudaGetLastError());
   c->cur ^= 1;
   c->scal_cur ^= 1;
   if (stats) {
-    StepScalars s;
-    RRHD_CUDA(cudaMemcpyAsync(&s, P.out, sizeof s, cudaMemcpyDeviceToHost, c->stream));
     RRHD_CUDA(cudaStreamSynchronize(c->stream));
+    const volatile StepScalars &s = *c->h_scal;  // written by the step's last CTA
     stats->max_speed = s.max_speed;
     stats->n_fallback = (int64_t)s.n_fallback;
     stats->n_failed = (int64_t)s.n_failed;
