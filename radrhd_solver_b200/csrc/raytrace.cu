@@ -36,7 +36,7 @@ struct rrhd_ray_surface {
   int64_t n = 0;
   double *tri = nullptr;  // [n][9] {A, E1 = B - A, E2 = C - A}
   int32_t *ids = nullptr;
-  // image-plane bins (one trace call at a time per surface)
+  // image-plane bins (one trace call at a time per surface), one allocation that begins at bins
   int32_t *bins = nullptr;    // [NB + 1] counts, then offsets
   int32_t *cursor = nullptr;  // [NB]
   int32_t *entries = nullptr; // [max_bins(n) * n] triangle indices by bin
@@ -821,11 +821,6 @@ extern "C" rrhd_status rrhd_ray_surface_destroy(rrhd_ray_surface *s) {
   cudaFree(s->tri);
   cudaFree(s->ids);
   cudaFree(s->bins);
-  cudaFree(s->cursor);
-  cudaFree(s->entries);
-  cudaFree(s->glist);
-  cudaFree(s->pack);
-  cudaFree(s->ctrl);
   cudaFree(s->ray2d);
   delete s;
   return RRHD_OK;
@@ -847,16 +842,25 @@ extern "C" rrhd_status rrhd_ray_trace(const rrhd_ray_surface *s, const double *r
     return RRHD_OK;
   }
   rrhd_ray_surface *sm = const_cast<rrhd_ray_surface *>(s);
-  if (!sm->bins) {  // allocated last: a call that ran out of memory is taken up by the next one
-    const auto need = [](auto *&p, size_t count) {
-      return p || count == 0 ? cudaSuccess : cudaMalloc(&p, sizeof(*p) * count);
+  if (!sm->bins) {  // one allocation: the first call of a surface pays for it
+    size_t at = 0;
+    const auto place = [&at](size_t bytes) {
+      const size_t here = at;
+      at += (bytes + 255) & ~(size_t)255;
+      return here;
     };
-    RRHD_CUDA(need(sm->cursor, kNB));
-    RRHD_CUDA(need(sm->ctrl, 8));
-    RRHD_CUDA(need(sm->entries, (size_t)max_bins(s->n) * (size_t)s->n));
-    RRHD_CUDA(need(sm->glist, (size_t)s->n));
-    RRHD_CUDA(need(sm->pack, kPack * (size_t)s->n));
-    RRHD_CUDA(need(sm->bins, kNB + 1));
+    const size_t n = (size_t)s->n;
+    const size_t bins = place(sizeof(int32_t) * (kNB + 1)), cursor = place(sizeof(int32_t) * kNB),
+                 ctrl = place(sizeof(long long) * 8), entries = place(sizeof(int32_t) * max_bins(s->n) * n),
+                 glist = place(sizeof(int32_t) * n), pack = place(sizeof(double) * kPack * n);
+    char *base = nullptr;
+    RRHD_CUDA(cudaMalloc(&base, at));
+    sm->bins = reinterpret_cast<int32_t *>(base + bins);
+    sm->cursor = reinterpret_cast<int32_t *>(base + cursor);
+    sm->ctrl = reinterpret_cast<long long *>(base + ctrl);
+    sm->entries = reinterpret_cast<int32_t *>(base + entries);
+    sm->glist = reinterpret_cast<int32_t *>(base + glist);
+    sm->pack = reinterpret_cast<double *>(base + pack);
   }
   if (sm->ray_cap < M) {
     RRHD_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
