@@ -506,7 +506,7 @@ typedef struct {
                              (cell, direction) item, which faces are in- and out-faces, the traced
                              distances and the face weights (16 bytes and five values of the
                              arithmetic's precision) whatever this says, where device memory holds
-                             them beside three arrays of the intensity's size; else it forms the
+                             them beside a coupled step's arrays; else it forms the             
                              distances and weights again from the cells' records               */
 } rrhd_rad_opts;
 /* Builds the sweep geometry and plan for ctx's mesh and the direction set (which

@@ -60,7 +60,7 @@ struct RadState {
   int SW = 0;    // stride (values) of the per-cell source record
   double bc = 0.0;
   void *d_w = nullptr;    // [M][3] directions in the sweep precision
-  void *d_rec = nullptr;  // [N] geometry records (normals, heights, neighbours); freed once d_dist stands
+  void *d_rec = nullptr;  // [N] geometry records (normals, heights, neighbours); read by a sweep without d_dist
   void *d_wt = nullptr;   // [N][4] face weights of the cell value
   void *d_src = nullptr;  // [N][SW] source records {k, betta/k, alpha Q_g/k}
   // the plan: per direction its N items in level order and the level offsets
