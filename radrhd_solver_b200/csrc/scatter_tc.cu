@@ -198,7 +198,11 @@ __global__ void __launch_bounds__(SPLIT ? 128 : kPrepassThreads, 2) k_row_prepas
   const int64_t wid = SPLIT ? blockIdx.x : (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = SPLIT ? gridDim.x : ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int nj = M / 16;  // a multiple of 4
-  // the 32 rows of a task are contiguous: one lane asks L2 for the warp's next ones
+  // The 32 rows of a task are contiguous: one lane asks L2 for the warp's first ones while the
+  // table is staged.  The later tasks' rows come with the loads alone, two sets of 16 directions
+  // (64 KB an SM) in flight: asked for a task ahead, all warps' rows (78 MB at 256 directions, 155
+  // at 512) pushed one another out of L2 and were read 1.4 times (663,552 cells x 4 groups x 256:
+  // scattering 2.74 -> 2.71 ms; 1,048,576 rows x 512: 3.69 -> 3.55).
   auto prefetch = [&](int64_t task) {
     if (lane == 0 && task < tasks) {
       const int64_t n = min((int64_t)32, rows - 32 * task) * M * 4;  // bytes, a multiple of 16
@@ -222,7 +226,6 @@ __global__ void __launch_bounds__(SPLIT ? 128 : kPrepassThreads, 2) k_row_prepas
   }
   __syncthreads();
   for (int64_t task = wid; task < tasks; task += nw) {  // warp-uniform
-    if (!SPLIT) prefetch(task + nw);
     const int64_t row0 = 32 * task;
     // row of this lane in row tile r
     auto row_of = [&](int r) {
