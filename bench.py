@@ -458,9 +458,8 @@ def coupled_component(dev, m, W, steps=100, warm=1, M=256, G=4, train_epochs=2, 
     Q = a_R T^4 / pi / G per grey group, sweep of M directions x G groups,
     4-force + source con2prim, scattering integral + moments.  Plain form: FP64
     sweep, FP64 scattering (one FMA per term), reference con2prim guess.  Chosen
-    form: mixed-precision sweep (FP64 arithmetic and face values, FP32 intensity
-    and scattering integral; with item_geometry, each (cell, direction) item's
-    geometry precomputed at setup and streamed), tensor-core F16X3 scattering,
+    form: mixed-precision sweep (FP64 arithmetic and outgoing values, FP32 intensity
+    and scattering integral), tensor-core F16X3 scattering,
     learned con2prim guess trained on the plain run's own states.  "plain_lowrank" / "chosen_lowrank": the
     same with the scattering through the rank-7 Thomson identity (FP64 arithmetic).
     All forms start from the same state; the intensity arrays (N*G*M = 5.4e9
@@ -523,10 +522,9 @@ def coupled_component(dev, m, W, steps=100, warm=1, M=256, G=4, train_epochs=2, 
         states[form] = Ug
         if form == "plain":
             states["plain_dump"] = (Wg, Ug)
-        bio = 8 if fp64 else 4  # bytes per intensity / scattering value; face values are double
-        sweep_alg = (2.0 * m.n_cells * bio + 2.0 * m.n_faces * 8) * M * G + m.n_cells * (20 * 8 + 32.0)
-        if geo:
-            sweep_alg += 16.0 * m.n_cells * M  # the item-geometry stream
+        bio = 8 if fp64 else 4  # bytes per intensity / scattering value
+        # S in, I out, an item's 16-byte record; the outgoing values stay on chip
+        sweep_alg = (2.0 * bio * G + 16.0) * m.n_cells * M + m.n_cells * 32.0
         out[form] = {"dirs_per_batch": batch[0] if fp64 else batch[1], "item_geometry": geo, "ms_per_step": ms, "steps_per_s": 1e3 / ms, "cell_updates_per_s": m.n_cells / (ms / 1e3),
                      "cell_dir_group_per_s": m.n_cells * M * G / (ms / 1e3), "phase_ms_last_step": ph,
                      "sweep_levels": levels, "largest_level": biggest, "plan_build_s": t_plan,
@@ -583,7 +581,7 @@ def sweep_component(dev, nhex=32, M=256, G=4, reps=3, precisions=("fp64", "fp32"
         ms = _time(lambda: illum.CalculateIllum(sw, alpha, betta, Q, S, I), reps, stream, warm=1)
         levels, biggest = sw.plan_info()
         bpv = 8 if prec == "fp64" else 4
-        alg = (2.0 * m.n_cells + 2.0 * m.n_faces) * M * G * bpv + m.n_cells * (20 * bpv + 32.0)
+        alg = (2.0 * G * bpv + 16.0) * m.n_cells * M + m.n_cells * 32.0
         out[prec] = {"ms": ms, "cell_dir_per_s": m.n_cells * M / (ms / 1e3), "levels": levels,
                      "largest_level": biggest, "plan_build_s": t_plan, "alg_gbs": alg / (ms / 1e3) / 1e9}
         del alpha, betta, Q, S, I
@@ -856,7 +854,7 @@ def main():
     ap.add_argument("--coupled-forms", default="plain,chosen", help="forms of --coupled-only")
     ap.add_argument("--coupled-batch", default="128,256", help="directions per sweep batch (plain,chosen)")
     ap.add_argument("--coupled-item-geometry", type=int, default=1,
-                    help="chosen forms: stream the precomputed per-item sweep geometry (1) or not (0)")
+                    help="chosen forms: the sweep's item_geometry option (no effect on the sweep)")
     ap.add_argument("--c2p-only", type=int, default=0, metavar="STATES",
                     help="only time the con2prim component on STATES states (profiling runs)")
     ap.add_argument("--no-compton", action="store_true", help="skip the full-spectrum Compton component")
