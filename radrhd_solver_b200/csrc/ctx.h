@@ -75,6 +75,7 @@ struct RadState {
   std::vector<int64_t> lvl_base;
   int64_t levels = 0, max_level = 0;
   bool two = false;             // two CTAs of the sweep share an SM
+  int cl = 1;  // CTAs that share a direction of the sweep
   int64_t nlow = 0, nhigh = 0;  // most slots a direction has in shared (slot 0: the boundary value) and global memory
   void *d_slots = nullptr;      // [M][nhigh][G]
   void *d_x = nullptr;          // S, then I, in the sweep's layout, [xdirs][N][G]

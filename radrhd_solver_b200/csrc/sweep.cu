@@ -230,6 +230,7 @@ struct SweepArgs {
   const T *src;             // [N][SW]
   T *slots;                 // [directions of the launch][nhigh][G]: slots from `cap` on
   uint32_t cap;             // slots in shared memory
+  int cl;                   // CTAs a direction
   int64_t nhigh;
   const TI *S;              // S and I element (cell c, direction d0 + x, group g) at q * sc + x * sd + g,
   TI *I;                    // q the item's position in sweep order (by_pos) or its cell
@@ -262,12 +263,17 @@ __device__ __forceinline__ void bulk_prefetch(const P *p, uint32_t n) {
 // 64, 269 -> 80 us; 32^3 x 256 x 4 FP64 12.6 -> 4.0 ms; 48^3 x 256 x 4 mixed 37.0 -> 10.2 ms.
 // With every load from L1 it would take half of that: issue slots and the latency of the FP64
 // chains at 16 warps an SM, and the wait at each level's barrier.
-template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB>
+//
+// CLUSTER: a.cl CTAs of a cluster share a direction's levels (few directions with long fronts);
+// slots 2 and up are in global memory, where a level's values pass from CTA to CTA over the
+// cluster barrier.
+template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB, bool CLUSTER>
 __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
   extern __shared__ __align__(16) uint8_t sweep_smem[];
   constexpr int GR = GT > 0 ? GT : 1;
-  constexpr int kAhead = 4 * NT;
-  const int x = blockIdx.x, d = a.d0 + x;
+  const int cl = CLUSTER ? a.cl : 1, x = (int)blockIdx.x / cl, d = a.d0 + x;
+  const int first = CLUSTER ? ((int)blockIdx.x - x * cl) * NT + (int)threadIdx.x : (int)threadIdx.x;  // in a level
+  const int step = cl * NT, kAhead = 4 * step;
   const int G = GT > 0 ? GT : a.G;
   T *const low = reinterpret_cast<T *>(sweep_smem);
   T *const high = HIGH ? a.slots + (int64_t)x * a.nhigh * G : nullptr;
@@ -343,10 +349,10 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
 
   // this thread's items in order, two ahead of the one in work: position p in the level that
   // ends at p_hi (the next one at p_hi2); N when there are none left
-  int p = (int)threadIdx.x, p_lvl = 0, p_hi = lvl[1], p_hi2 = lvl[min(2, depth)];
+  int p = first, p_lvl = 0, p_hi = lvl[1], p_hi2 = lvl[min(2, depth)];
   auto settle = [&]() {
     while (p >= p_hi && p_hi < N) {
-      p = p_hi + (int)threadIdx.x;
+      p = p_hi + first;
       p_lvl++;
       p_hi = p_hi2;
       p_hi2 = lvl[min(p_lvl + 2, depth)];
@@ -358,13 +364,13 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
   if (p < N) {
     load_record(p, it);
     load_cell(it);
-    p += NT;
+    p += step;
     settle();
     if (p < N) load_record(p, next);
   }
   int hi = lvl[1], hi2 = lvl[min(2, depth)];
   for (int L = 0; L < depth; L++) {
-    if (threadIdx.x == 0) fetch(hi + kAhead);
+    if (first == 0) fetch(hi + kAhead);
     while (i < hi) {
       const Item now = it;
       const int at_i = i;
@@ -373,7 +379,7 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
       it = next;
       if (p < N) {
         load_cell(it);
-        p += NT;
+        p += step;
         settle();
         if (p < N) load_record(p, next);
       }
@@ -473,7 +479,10 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
     }
     hi = hi2;
     hi2 = lvl[min(L + 3, depth)];
-    __syncthreads();
+    if constexpr (CLUSTER)
+      asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else
+      __syncthreads();
   }
 }
 
@@ -918,9 +927,38 @@ int slot_cap(const RadState &R, bool two) {  // slots a CTA's shared memory can 
   return (int)((two ? kSmemTwo : kSmemOne) / (tv * R.G));
 }
 
+// CTAs that share a direction.  Where a direction's slots fit one CTA's shared memory, one: the
+// values stay there (48^3 x 6 cells x 8, 32 and 74 directions, one group FP64: 2.1, 2.4 and 2.9
+// ms; 3.1, 3.7 and 4.6 with 8, 4 and 2 CTAs).  Where they do not, they are all in global memory
+// and few directions take as many CTAs as there are SMs for, at most the portable eight: four
+// groups 3.9, 4.8 and 6.7 ms, 5.9, 6.5 and 8.6 with one; 96^3 x 8 and 32 directions x 4 groups 13.5
+// and 23 ms, 67 and 82 with one.
+int cluster_size(const RadState &R, int64_t slots) {
+  int cl = 1;
+  if (slots > slot_cap(R, false))
+    while (cl < 8 && 2 * cl * R.M <= kSweepSMs) cl *= 2;
+  return cl;
+}
+
 template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB>
 cudaError_t launch_sweep_kernel(const SweepArgs<T, TI> &a, int nd, size_t smem, cudaStream_t st) {
-  auto *k = k_sweep<T, TI, GT, HIGH, WIDE, GEO, NT, NB>;
+  if constexpr (HIGH && NT == 512) {
+    if (a.cl > 1) {
+      cudaLaunchAttribute cluster;
+      cluster.id = cudaLaunchAttributeClusterDimension;
+      cluster.val.clusterDim.x = (unsigned)a.cl;
+      cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(nd * a.cl));
+      cfg.blockDim = dim3(NT);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st;
+      cfg.attrs = &cluster;
+      cfg.numAttrs = 1;
+      return cudaLaunchKernelEx(&cfg, k_sweep<T, TI, GT, HIGH, WIDE, GEO, NT, NB, true>, a);
+    }
+  }
+  auto *k = k_sweep<T, TI, GT, HIGH, WIDE, GEO, NT, NB, false>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k<<<nd, NT, smem, st>>>(a);
@@ -971,7 +1009,8 @@ rrhd_status launch_sweep(rrhd_ctx *c, int d0, int nd, const void *S, void *I, in
   a.depth = R.d_depth;
   a.src = (const T *)R.d_src;
   a.slots = (T *)R.d_slots;
-  a.cap = (uint32_t)slot_cap(R, R.two);
+  a.cap = R.cl > 1 ? 2u : (uint32_t)slot_cap(R, R.two);
+  a.cl = R.cl;
   a.nhigh = R.nhigh;
   a.S = (const TI *)S;
   a.I = (TI *)I;
@@ -1231,7 +1270,9 @@ rrhd_status build_plan(rrhd_ctx *c) {
   }
   const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
   R.two = R.M > kSweepSMs && R.d_pos && ti * R.G >= 16 && (double)beyond <= kTwoBeyond * (double)all;
-  const int cap = slot_cap(R, R.two);
+  R.cl = cluster_size(R, most);
+  if (R.cl > 1) R.two = false;
+  const int cap = R.cl > 1 ? 2 : slot_cap(R, R.two);
   R.nlow = std::min<int64_t>(most, cap);
   R.nhigh = std::max<int64_t>(0, most - cap);
   // rrhd_rad_plan_info: levels and the largest level over batches of R.DB directions
