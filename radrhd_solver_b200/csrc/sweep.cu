@@ -1498,36 +1498,79 @@ __global__ void k_rows_to_cdg(int64_t N, int M, int G, const int32_t *perm, cons
 }
 }  // namespace
 
-// T: the element type of the intensity and scattering-integral arrays.
-template <class T>
-static rrhd_status alloc_coupled(rrhd_ctx *c) {
+namespace {
+// Frees what a sweep can do without: its scratch (a later sweep makes another), then the geometry
+// stream.  False: nothing left.
+rrhd_status give_back(rrhd_ctx *c, bool &freed) {
   RadState &R = c->rad;
-  const int64_t N = c->N, rows = N * R.G;
-  const size_t big = sizeof(T) * (size_t)rows * R.M;
-  if (cudaMalloc(&R.d_I, big) != cudaSuccess || cudaMalloc(&R.d_S, big) != cudaSuccess ||
-      cudaMalloc(&R.d_G4, sizeof(double) * 4 * N) != cudaSuccess ||
-      cudaMalloc(&R.d_cnt, sizeof(unsigned long long) * 8) != cudaSuccess)
-    return rrhd_fail(RRHD_ERR_OOM, "coupled-step allocation failed");
-  for (cudaEvent_t &e : R.ev) RRHD_CUDA(cudaEventCreate(&e));
-  RRHD_CUDA(cudaStreamCreateWithFlags(&R.side, cudaStreamNonBlocking));
-  RRHD_CUDA(cudaMemsetAsync(R.d_I, 0, big, c->stream));
-  RRHD_CUDA(cudaMemsetAsync(R.d_S, 0, big, c->stream));
-  RRHD_CUDA(cudaMemsetAsync(R.d_G4, 0, sizeof(double) * 4 * N, c->stream));
-  if (R.prec == RRHD_RAD_FP64) {
-    if (cudaMalloc(&R.d_mE, sizeof(double) * rows) != cudaSuccess ||
-        cudaMalloc(&R.d_mF, sizeof(double) * 3 * rows) != cudaSuccess ||
-        cudaMalloc(&R.d_mT, sizeof(double) * 9 * rows) != cudaSuccess)
-      return rrhd_fail(RRHD_ERR_OOM, "coupled-step allocation failed");
-    RRHD_CUDA(cudaMemsetAsync(R.d_mE, 0, sizeof(double) * rows, c->stream));
-    RRHD_CUDA(cudaMemsetAsync(R.d_mF, 0, sizeof(double) * 3 * rows, c->stream));
-    RRHD_CUDA(cudaMemsetAsync(R.d_mT, 0, sizeof(double) * 9 * rows, c->stream));
+  freed = R.d_x || R.d_dist;
+  if (!freed) return RRHD_OK;
+  RRHD_CUDA(cudaStreamSynchronize(c->stream));
+  if (R.d_x) {
+    cudaFree(R.d_x);
+    R.d_x = nullptr;
   } else {
-    if (cudaMalloc(&R.d_mom, sizeof(float) * 16 * rows) != cudaSuccess)
-      return rrhd_fail(RRHD_ERR_OOM, "coupled-step allocation failed");
-    RRHD_CUDA(cudaMemsetAsync(R.d_mom, 0, sizeof(float) * 16 * rows, c->stream));
+    drop_stream(R);
   }
   return RRHD_OK;
 }
+
+void drop_coupled(RadState &R) {
+  for (void **p : {&R.d_I, &R.d_S, (void **)&R.d_G4, (void **)&R.d_mE, (void **)&R.d_mF, (void **)&R.d_mT,
+                   (void **)&R.d_mom, (void **)&R.d_cnt}) {
+    cudaFree(*p);
+    *p = nullptr;
+  }
+  for (cudaEvent_t &e : R.ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
+  if (R.side) cudaStreamDestroy(R.side);
+  R.side = nullptr;
+}
+
+// The arrays, events and side stream of the coupled step, zeroed: all of them, or (R.d_I is null) none.
+rrhd_status make_coupled(rrhd_ctx *c) {
+  RadState &R = c->rad;
+  const size_t N = (size_t)c->N, rows = N * R.G;
+  const bool fp64 = R.prec == RRHD_RAD_FP64;
+  const size_t big = (fp64 ? sizeof(double) : sizeof(float)) * rows * R.M;
+  const struct {
+    void **p;
+    size_t bytes;
+  } parts[] = {{&R.d_I, big},
+               {&R.d_S, big},
+               {(void **)&R.d_G4, sizeof(double) * 4 * N},
+               {(void **)&R.d_cnt, sizeof(unsigned long long) * 8},
+               {(void **)&R.d_mE, fp64 ? sizeof(double) * rows : 0},
+               {(void **)&R.d_mF, fp64 ? sizeof(double) * 3 * rows : 0},
+               {(void **)&R.d_mT, fp64 ? sizeof(double) * 9 * rows : 0},
+               {(void **)&R.d_mom, fp64 ? 0 : sizeof(float) * 16 * rows}};
+  for (const auto &q : parts) {
+    if (!q.bytes) continue;
+    while (cudaMalloc(q.p, q.bytes) != cudaSuccess) {
+      cudaGetLastError();
+      *q.p = nullptr;
+      bool freed = false;
+      const rrhd_status s = give_back(c, freed);
+      if (s) return s;
+      if (!freed) return rrhd_fail(RRHD_ERR_OOM, "coupled-step allocation failed (%lld bytes)", (long long)q.bytes);
+    }
+    RRHD_CUDA(cudaMemsetAsync(*q.p, 0, q.bytes, c->stream));
+  }
+  for (cudaEvent_t &e : R.ev) RRHD_CUDA(cudaEventCreate(&e));
+  RRHD_CUDA(cudaStreamCreateWithFlags(&R.side, cudaStreamNonBlocking));
+  return RRHD_OK;
+}
+rrhd_status alloc_coupled(rrhd_ctx *c) {
+  const rrhd_status s = make_coupled(c);
+  if (s) {
+    cudaStreamSynchronize(c->stream);  // the zeroing of what is freed
+    drop_coupled(c->rad);
+  }
+  return s;
+}
+}  // namespace
 
 extern "C" rrhd_status rrhd_coupled_step(rrhd_ctx *c, double tau, const rrhd_coupled_opts *o, rrhd_step_stats *hs,
                                          rrhd_c2p_stats *ss) {
@@ -1548,7 +1591,7 @@ extern "C" rrhd_status rrhd_coupled_step(rrhd_ctx *c, double tau, const rrhd_cou
   RRHD_CHECK_ARG(k_stall > 0 && k_stall <= 40, "k_stall must be in [1, 40]");
   RRHD_CUDA(cudaSetDevice(c->device));
   rrhd_status s;
-  if (!R.d_I && (s = fp64 ? alloc_coupled<double>(c) : alloc_coupled<float>(c))) return s;
+  if (!R.d_I && (s = alloc_coupled(c))) return s;
   if (!fp64 && !lowrank && (!R.tc || R.tc_form != o->scatter)) {
     if (R.tc) rrhd_scatter_tc_destroy(R.tc);
     R.tc = nullptr;
@@ -1905,7 +1948,7 @@ extern "C" rrhd_status rrhd_rad_set(rrhd_ctx *c, int32_t what, const double *in)
   if (!R.ready) return rrhd_fail(RRHD_ERR_STATE, "rrhd_rad_setup has not run");
   RRHD_CUDA(cudaSetDevice(c->device));
   rrhd_status s;
-  if (!R.d_I && (s = R.prec == RRHD_RAD_FP64 ? alloc_coupled<double>(c) : alloc_coupled<float>(c))) return s;
+  if (!R.d_I && (s = alloc_coupled(c))) return s;
   const int64_t N = c->N, width = (int64_t)R.G * R.M;
   double *tmp = nullptr;
   RRHD_CUDA(cudaMalloc(&tmp, sizeof(double) * N * width));
