@@ -1458,14 +1458,15 @@ extern "C" rrhd_status rrhd_sweep(rrhd_ctx *c, const void *alpha, const void *be
 
 // ---------------------------------------------------------------- coupled step
 namespace {
+// I or S of the caller's cells p0 .. p0 + n - 1 as rows [n * G][M]
 template <class T>
-__global__ void k_cdg_to_rows(int64_t N, int M, int G, const int32_t *perm, const T *src, double *dst) {
+__global__ void k_cdg_to_rows(int64_t p0, int64_t n, int M, int G, const int32_t *iperm, const T *src, double *dst) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t per = (int64_t)M * G;
-  if (i >= N * per) return;
-  const int64_t c = i / per, rem = i - c * per;
-  const int d = (int)(rem / G), g = (int)(rem - (int64_t)d * G);
-  dst[((int64_t)perm[c] * G + g) * M + d] = (double)src[i];
+  if (i >= n * per) return;
+  const int64_t p = i / per, rem = i - p * per;
+  const int g = (int)(rem / M), d = (int)(rem - (int64_t)g * M);
+  dst[i] = (double)src[((int64_t)iperm[p0 + p] * M + d) * G + g];
 }
 
 // Moments of the last scattering per row (cell * G + g), caller order, as
@@ -1488,13 +1489,57 @@ __global__ void k_mom_to_rows(int64_t N, int G, const int32_t *perm, const doubl
 }
 
 template <class T>
-__global__ void k_rows_to_cdg(int64_t N, int M, int G, const int32_t *perm, const double *src, T *dst) {
+__global__ void k_rows_to_cdg(int64_t p0, int64_t n, int M, int G, const int32_t *iperm, const double *src, T *dst) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t per = (int64_t)M * G;
-  if (i >= N * per) return;
-  const int64_t c = i / per, rem = i - c * per;
-  const int d = (int)(rem / G), g = (int)(rem - (int64_t)d * G);
-  dst[i] = (T)src[((int64_t)perm[c] * G + g) * M + d];
+  if (i >= n * per) return;
+  const int64_t p = i / per, rem = i - p * per;
+  const int g = (int)(rem / M), d = (int)(rem - (int64_t)g * M);
+  dst[((int64_t)iperm[p0 + p] * M + d) * G + g] = (T)src[i];
+}
+
+// I or S between the context and the caller's host rows [N * G][M], a piece of the caller's
+// cells at a time through a buffer of at most kPieceBytes (one cell at least): at 96^3 x 6
+// cells, 256 directions and 4 groups a whole array is 43.5 GB, more than a coupled step leaves.
+// What bounds it is the copy to or from the host; a piece's kernel moves its bytes once on the device.
+constexpr size_t kPieceBytes = (size_t)256 << 20;
+rrhd_status move_rows(rrhd_ctx *c, void *array, double *to, const double *from) {
+  const RadState &R = c->rad;
+  const int64_t N = c->N, per = (int64_t)R.M * R.G;
+  int64_t cells = std::min<int64_t>(N, std::max<int64_t>(1, (int64_t)(kPieceBytes / (sizeof(double) * per))));
+  double *tmp = nullptr;
+  while (cudaMalloc(&tmp, sizeof(double) * cells * per) != cudaSuccess) {
+    cudaGetLastError();
+    if (cells == 1) return rrhd_fail(RRHD_ERR_OOM, "transfer buffer allocation failed");
+    cells = (cells + 1) / 2;
+  }
+  cudaError_t e = cudaSuccess;
+  for (int64_t p = 0; p < N && e == cudaSuccess; p += cells) {
+    const int64_t n = std::min(cells, N - p);
+    const unsigned nb = grid_for(n * per, 256);
+    const size_t bytes = sizeof(double) * n * per;
+    if (to) {
+      if (R.prec == RRHD_RAD_FP64)
+        k_cdg_to_rows<double><<<nb, 256, 0, c->stream>>>(p, n, R.M, R.G, c->d_iperm, (const double *)array, tmp);
+      else
+        k_cdg_to_rows<float><<<nb, 256, 0, c->stream>>>(p, n, R.M, R.G, c->d_iperm, (const float *)array, tmp);
+      e = cudaGetLastError();
+      if (e == cudaSuccess) e = cudaMemcpyAsync(to + p * per, tmp, bytes, cudaMemcpyDeviceToHost, c->stream);
+    } else {
+      e = cudaMemcpyAsync(tmp, from + p * per, bytes, cudaMemcpyHostToDevice, c->stream);
+      if (e != cudaSuccess) break;
+      if (R.prec == RRHD_RAD_FP64)
+        k_rows_to_cdg<double><<<nb, 256, 0, c->stream>>>(p, n, R.M, R.G, c->d_iperm, tmp, (double *)array);
+      else
+        k_rows_to_cdg<float><<<nb, 256, 0, c->stream>>>(p, n, R.M, R.G, c->d_iperm, tmp, (float *)array);
+      e = cudaGetLastError();
+    }
+  }
+  const cudaError_t e2 = cudaStreamSynchronize(c->stream);
+  cudaFree(tmp);
+  RRHD_CUDA(e);
+  RRHD_CUDA(e2);
+  return RRHD_OK;
 }
 }  // namespace
 
@@ -1918,21 +1963,16 @@ extern "C" rrhd_status rrhd_rad_get(rrhd_ctx *c, int32_t what, double *out) {
                  "bad array id");
   if (!R.ready || !R.d_I) return rrhd_fail(RRHD_ERR_STATE, "no coupled step has run");
   RRHD_CUDA(cudaSetDevice(c->device));
+  if (what == RRHD_RAD_I || what == RRHD_RAD_S) return move_rows(c, what == RRHD_RAD_I ? R.d_I : R.d_S, out, nullptr);
   const int64_t N = c->N;
-  const int64_t width = what == RRHD_RAD_G4 ? 4 : what == RRHD_RAD_MOM ? 10 * (int64_t)R.G : (int64_t)R.G * R.M;
+  const int64_t width = what == RRHD_RAD_G4 ? 4 : 10 * (int64_t)R.G;
   double *tmp = nullptr;
   RRHD_CUDA(cudaMalloc(&tmp, sizeof(double) * N * width));
   if (what == RRHD_RAD_MOM)
     k_mom_to_rows<<<grid_for(N * R.G, 256), 256, 0, c->stream>>>(N, R.G, c->d_perm, R.d_mom ? nullptr : R.d_mE,
                                                                   R.d_mF, R.d_mT, R.d_mom, tmp);
-  else if (what == RRHD_RAD_G4)
-    k_rows_to_host_order<double><<<grid_for(N * width, 256), 256, 0, c->stream>>>(N, width, c->d_perm, R.d_G4, tmp);
-  else if (R.prec == RRHD_RAD_FP64)
-    k_cdg_to_rows<double><<<grid_for(N * width, 256), 256, 0, c->stream>>>(
-        N, R.M, R.G, c->d_perm, (const double *)(what == RRHD_RAD_I ? R.d_I : R.d_S), tmp);
   else
-    k_cdg_to_rows<float><<<grid_for(N * width, 256), 256, 0, c->stream>>>(
-        N, R.M, R.G, c->d_perm, (const float *)(what == RRHD_RAD_I ? R.d_I : R.d_S), tmp);
+    k_rows_to_host_order<double><<<grid_for(N * width, 256), 256, 0, c->stream>>>(N, width, c->d_perm, R.d_G4, tmp);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, sizeof(double) * N * width, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1949,22 +1989,5 @@ extern "C" rrhd_status rrhd_rad_set(rrhd_ctx *c, int32_t what, const double *in)
   RRHD_CUDA(cudaSetDevice(c->device));
   rrhd_status s;
   if (!R.d_I && (s = alloc_coupled(c))) return s;
-  const int64_t N = c->N, width = (int64_t)R.G * R.M;
-  double *tmp = nullptr;
-  RRHD_CUDA(cudaMalloc(&tmp, sizeof(double) * N * width));
-  void *dst = what == RRHD_RAD_I ? R.d_I : R.d_S;
-  cudaError_t e = cudaMemcpyAsync(tmp, in, sizeof(double) * N * width, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) {
-    if (R.prec == RRHD_RAD_FP64)
-      k_rows_to_cdg<double><<<grid_for(N * width, 256), 256, 0, c->stream>>>(N, R.M, R.G, c->d_perm, tmp,
-                                                                             (double *)dst);
-    else
-      k_rows_to_cdg<float><<<grid_for(N * width, 256), 256, 0, c->stream>>>(N, R.M, R.G, c->d_perm, tmp,
-                                                                            (float *)dst);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  cudaFree(tmp);
-  RRHD_CUDA(e);
-  return RRHD_OK;
+  return move_rows(c, what == RRHD_RAD_I ? R.d_I : R.d_S, nullptr, in);
 }

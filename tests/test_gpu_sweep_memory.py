@@ -32,7 +32,7 @@ def mesh():
 
 
 class Context:
-    def __init__(self, m, G):
+    def __init__(self, m, G, precision="fp64"):
         W = np.zeros((m.n_cells, 5))
         W[:, 0] = 10 ** np.random.default_rng(52).uniform(-1, 1, m.n_cells)
         W[:, 4] = 0.1
@@ -40,8 +40,9 @@ class Context:
         self.grid = rhllc.Grid(m, gamma=GAMMA_43)
         self.grid.set_state_prim(W)
         self.dg = illum.DirectionGrid(fibonacci_directions(M))
-        self.sw = illum.TransportSweep(self.grid, self.dg, groups=G, precision="fp64")
-        self.step = rad_rhd.RadRHDStep(self.sw, em=rad_rhd.emission(1.0, 10.0))
+        self.sw = illum.TransportSweep(self.grid, self.dg, groups=G, precision=precision)
+        self.step = rad_rhd.RadRHDStep(self.sw, em=rad_rhd.emission(1.0, 10.0),
+                                       scatter="fp64" if precision == "fp64" else "f16x3")
 
     def steps(self):
         for _ in range(2):
@@ -94,3 +95,21 @@ def test_coupled_step_takes_the_sweeps_memory(mesh, megabytes):
         assert np.array_equal(a, b)
     c.close()
     want.close()
+
+
+@pytest.mark.parametrize("precision,G", [("fp64", 4), ("mixed", 3)])
+def test_transfers_in_pieces(mesh, precision, G):
+    """I and S to and from the host with less free than one of them takes (201 and 151 MB of doubles)."""
+    c = Context(mesh, G, precision)
+    rng = np.random.default_rng(54)
+    values = [rng.uniform(0, 1, (mesh.n_cells * G, M)).astype(np.float32).astype(np.float64) for _ in range(2)]
+    c.step.set("I", values[0])
+    held = leave(20)
+    assert np.array_equal(c.step.get("I"), values[0])
+    c.step.set("S", values[1])
+    assert np.array_equal(c.step.get("S"), values[1])
+    assert np.array_equal(c.step.get("I"), values[0])
+    del held
+    torch.cuda.empty_cache()
+    assert np.array_equal(c.step.get("S"), values[1])
+    c.close()
