@@ -111,6 +111,7 @@ __device__ __forceinline__ void face_cos(const T *g, T wx, T wy, T wz, T *cosf) 
 //   bits 8-11           out-faces (cos > 0)
 //   bit 12              the node at b1's vertex is traced to b2 (else to b1, lam = 2/3)
 //   bit 13              some face is neither (parallel to the direction)
+//   bits 14-15          how the stream holds the weights (item_weights)
 constexpr uint32_t kCodeB2 = 1u << 12, kCodeOdd = 1u << 13;
 
 // Code word and distances of one (cell, direction) from the cell's normals and heights
@@ -161,12 +162,52 @@ __device__ __forceinline__ uint32_t item_geometry(const T *g, const T *cosf, T &
   return code;
 }
 
-// weights (area_j / sum of the areas) of the in-faces b1, b2 and the third, 0 where there is none
+// Weights of an item: w of the in-faces b1, b2 and the third (0 where there is none), wo of all
+// out-faces together, from the cell's four (area_j / sum of the areas).  wo is the sum of the
+// out-faces' weights: as one minus the others it would lose the digits of a small out-face, and
+// with them the value of a cell that takes nothing from its in-faces.
 template <class T>
-__device__ __forceinline__ void in_weights(const T *wt, uint32_t code, T (&w)[3]) {
+__device__ __forceinline__ void item_weights(const T (&f)[4], uint32_t code, T (&w)[3], T &wo) {
   const int nin = (int)(code >> 6) & 3;
+  const auto pick = [&](uint32_t j) { return j & 2 ? (j & 1 ? f[3] : f[2]) : (j & 1 ? f[1] : f[0]); };
+  w[0] = nin > 0 ? pick(code & 3) : (T)0;
+  w[1] = nin > 1 ? pick((code >> 2) & 3) : (T)0;
+  w[2] = nin > 2 ? pick((code >> 4) & 3) : (T)0;
+  wo = (T)0;
 #pragma unroll
-  for (int q = 0; q < 3; q++) w[q] = q < nin ? wt[(code >> (2 * q)) & 3] : (T)0;
+  for (int j = 0; j < 4; j++) wo += (code >> (8 + j)) & 1u ? f[j] : (T)0;
+}
+
+// The stream keeps three of the four (in double; a sweep in float takes them from the cell's
+// sector).  They sum to one, so the largest, at least a quarter, is found again to a few roundings:
+// bits 14-15 of the code word say whose place (b1, b2, third) holds wo, 3 that wo is left out.
+// With one or two in-faces it is the third's, whose weight nothing is multiplied by.
+constexpr int kLeftBit = 14;
+template <class T>
+__device__ __forceinline__ uint32_t left_out(uint32_t code, const T (&w)[3], T wo) {
+  if (((code >> 6) & 3u) < 3u) return 2u;
+  uint32_t left = 3;
+  T most = wo;
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    if (w[q] > most) left = (uint32_t)q, most = w[q];
+  return left;
+}
+// the three of the stream ...
+template <class T>
+__device__ __forceinline__ void pack_weights(uint32_t left, T (&w)[3], T wo) {
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    if (left == (uint32_t)q) w[q] = wo;
+}
+// ... and all four again
+template <class T>
+__device__ __forceinline__ void unpack_weights(uint32_t left, T (&w)[3], T &wo) {
+  const T rest = ((T)1 - w[0]) - (w[1] + w[2]);
+  wo = rest;
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    if (left == (uint32_t)q) wo = w[q], w[q] = rest;
 }
 
 // 32 bytes of global memory in one access (32-byte aligned)
@@ -175,6 +216,12 @@ __device__ __forceinline__ void ld_32(const double *p, double &a, double &b, dou
 }
 __device__ __forceinline__ void st_32(double *p, double a, double b, double c, double d) {
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+__device__ __forceinline__ void ld_cell_weights(const double *p, double (&f)[4]) { ld_32(p, f[0], f[1], f[2], f[3]); }
+__device__ __forceinline__ void ld_cell_weights(const float *p, float (&f)[4]) {
+  const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
+  f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
 }
 
 // G values at p (contiguous), vectorised for 2 and 4 groups; GMEM: p is in global memory,
@@ -222,7 +269,7 @@ struct SweepArgs {
   const uint4 *ord;         // [M][N] items in sweep order {cell, code, own | in0 << 16, in1 | in2 << 16}
   const uint2 *ord_hi;      // [M][N] upper halves of the slots (WIDE)
   const T *dist;            // [M][N][2] {tA, tB} (GEO)
-  const T *wgt, *wgt3;      // [M][N][2], [M][N] weights of the in-faces (GEO)
+  const T *wgt, *wgt3;      // [M][N][2], [M][N] weights (GEO, double)
   const T *rec, *w, *wt;    // geometry records and directions (not GEO), face weights [N][4]
   const int32_t *lvl;       // level offsets of every direction
   const int64_t *lvl_base;  // [M] first entry in lvl
@@ -249,7 +296,7 @@ __device__ __forceinline__ void bulk_prefetch(const P *p, uint32_t n) {
 
 // One CTA per direction.  GT: compile-time group count (1, 2 or 4; S and I in the sweep's own
 // layout), 0 for any other.  HIGH: slots from a.cap on are in global memory (the others in
-// shared memory).  GEO: distances and weights from the stream, else from the cell's records.
+// shared memory).  GEO: distances, and in double the weights, from the stream, else from the cell's records.
 // Slots 0 and 1 hold the boundary value and zero (for in-faces an item does not have); an item
 // whose own slot is 0 has no downwind neighbour and writes none.
 //
@@ -271,6 +318,7 @@ template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int
 __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
   extern __shared__ __align__(16) uint8_t sweep_smem[];
   constexpr int GR = GT > 0 ? GT : 1;
+  constexpr bool WGT = GEO && sizeof(T) == 8;  // weights from the stream
   const int cl = CLUSTER ? a.cl : 1, x = (int)blockIdx.x / cl, d = a.d0 + x;
   const int first = CLUSTER ? ((int)blockIdx.x - x * cl) * NT + (int)threadIdx.x : (int)threadIdx.x;  // in a level
   const int step = cl * NT, kAhead = 4 * step;
@@ -340,8 +388,10 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
     bulk_prefetch(ord + q, 16 * n);
     if (GEO) {
       bulk_prefetch(dist + 2 * q, 2 * (uint32_t)sizeof(T) * n);
+    }
+    if (WGT) {
       bulk_prefetch(wgt + 2 * q, 2 * (uint32_t)sizeof(T) * n);
-      if (sizeof(T) == 8) bulk_prefetch(wgt3 + q, 8 * n);
+      bulk_prefetch(wgt3 + q, (uint32_t)sizeof(T) * n);
     }
     if (a.by_pos && sizeof(TI) * G % 8 == 0) bulk_prefetch(S + (int64_t)fetched * G, (uint32_t)sizeof(TI) * G * n);
     fetched = to;
@@ -385,18 +435,15 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
       }
       const uint64_t c = now.o.x;
       const uint32_t code = now.o.y;
-      T w[3];
+      T w[3], cw[4];  // cw: the cell's weights, where there is no stream of them
       TI sv[GR];
       if constexpr (GT > 0) ld_groups<true>(S + (uint64_t)iq * (uint32_t)GT, sv);
-      if constexpr (GEO) {
-        if constexpr (sizeof(T) == 8) {
-          const double2 u = __ldcs(reinterpret_cast<const double2 *>(wgt) + at_i);
-          w[0] = u.x, w[1] = u.y;
-        } else {
-          const float2 u = __ldcs(reinterpret_cast<const float2 *>(wgt) + at_i);
-          w[0] = u.x, w[1] = u.y;
-        }
+      if constexpr (WGT) {
+        const double2 u = __ldcs(reinterpret_cast<const double2 *>(wgt) + at_i);
+        w[0] = u.x, w[1] = u.y;
         w[2] = __ldcs(wgt3 + at_i);
+      } else {
+        ld_cell_weights(a.wt + 4 * c, cw);
       }
       uint32_t own = now.o.z & 0xffffu, s0 = now.o.z >> 16, s1 = now.o.w & 0xffffu, s2 = now.o.w >> 16;
       if constexpr (WIDE) {
@@ -413,28 +460,32 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
         load_vec<T>(a.rec + c * Rec<T>::RW, g, 16);
         face_cos(g, wx, wy, wz, cosf);
         (void)item_geometry<T>(g, cosf, tA, tB);  // the code word is the plan's
-        in_weights(a.wt + 4 * c, code, w);
       }
       const T k = now.k, bk = now.bk;
       const bool two = (code & kCodeB2) != 0;
       const T EA = ex(-k * tA);
       const T E2 = EA * EA, EX = ex(-k * tB);  // formed in any case: the two chains overlap
       const T EB = two ? EX : E2 * E2;
-      T wo = ((T)1 - w[0]) - (w[1] + w[2]);  // all out-faces together
-      T par = (T)0;                          // a face parallel to the direction holds the boundary value
+      T wo;
+      if constexpr (!WGT) item_weights(cw, code, w, wo);
+      if constexpr (sizeof(T) == 8) {  // the same bits with and without the stream
+        const uint32_t left = (code >> kLeftBit) & 3u;
+        if constexpr (!WGT) pack_weights(left, w, wo);
+        unpack_weights(left, w, wo);
+      }
+      T par = (T)0;  // a face parallel to the direction holds the boundary value
       if (code & kCodeOdd) {
         const int nin = (int)(code >> 6) & 3;
         uint32_t seen = (code >> 8) & 15u;
         if (nin > 0) seen |= 1u << (code & 3);
         if (nin > 1) seen |= 1u << ((code >> 2) & 3);
         if (nin > 2) seen |= 1u << ((code >> 4) & 3);
-        wo = (T)0;
+        T all[4];
+        ld_cell_weights(a.wt + 4 * c, all);
+        item_weights(all, code, w, wo);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const T wj = a.wt[4 * c + j];
-          if ((code >> (8 + j)) & 1u) wo += wj;
-          if (!((seen >> j) & 1u)) par += wj * a.bc;
-        }
+        for (int j = 0; j < 4; j++)
+          if (!((seen >> j) & 1u)) par += all[j] * a.bc;
       }
       auto value = [&](T v0, T v1, T v2, T rhs, T &cell) {
         const T A = fma_rn(EA, v0 - rhs, rhs);
@@ -700,7 +751,7 @@ __global__ void __launch_bounds__(kPlanThreads)
       load_vec<T>(rec + c * Rec<T>::RW, g, 16);
       load_nbr<T>(rec + c * Rec<T>::RW, nbr);
       face_cos(g, wx, wy, wz, cosf);
-      const uint32_t code = item_geometry<T>(g, cosf, tA, tB);
+      uint32_t code = item_geometry<T>(g, cosf, tA, tB);
       uint32_t n = 0;
 #pragma unroll
       for (int j = 0; j < 4; j++) n += (cosf[j] > 0 && nbr[j] >= 0) ? 1u : 0u;
@@ -731,13 +782,21 @@ __global__ void __launch_bounds__(kPlanThreads)
         if (q < nin) s[q] = b >= 0 ? slot_of[b] : 0u;
       }
       if (pos_all) pos_all[at + c] = (uint32_t)i;
+      T f[4], wq[3], wo;
+      if constexpr (sizeof(T) == 8) {
+        ld_cell_weights(wt + 4 * c, f);
+        item_weights(f, code, wq, wo);
+        const uint32_t left = left_out(code, wq, wo);
+        pack_weights(left, wq, wo);
+        code |= left << kLeftBit;
+      }
       ord[i] = make_uint4((uint32_t)c, code, (own & 0xffffu) | s[0] << 16, (s[1] & 0xffffu) | s[2] << 16);
       if (hi16) hi16[i] = make_uint2(own >> 16 | (s[0] & 0xffff0000u), s[1] >> 16 | (s[2] & 0xffff0000u));
       if (dist_all) {
-        T wq[3];
-        in_weights(wt + 4 * c, code, wq);
         dist_all[2 * (at + i)] = tA;
         dist_all[2 * (at + i) + 1] = tB;
+      }
+      if (wgt_all) {
         wgt_all[2 * (at + i)] = wq[0];
         wgt_all[2 * (at + i) + 1] = wq[1];
         wgt3_all[at + i] = wq[2];
@@ -1157,7 +1216,7 @@ rrhd_status build_plan(rrhd_ctx *c) {
     R.d_ord = nullptr;
     return rrhd_fail(oom, "sweep plan allocation failed (%lld bytes)", (long long)(sizeof(uint4) * total));
   }
-  // The geometry stream (5 values an item) spares each item its cell's geometry record, and
+  // The geometry stream (5 values an item, 2 in float) spares each item its cell's geometry record, and
   // the cells' positions bring S and I into sweep order.  They are kept where the memory left
   // holds them beside what a coupled step allocates (intensity, scattering integral, moments,
   // 4-force); else the sweep forms the same values again from the records and takes S and I by
@@ -1168,9 +1227,11 @@ rrhd_status build_plan(rrhd_ctx *c) {
     const size_t one = sizeof(T) * (size_t)total, pos = sizeof(uint32_t) * (size_t)total;
     const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
     const size_t arrays = 2 * ti * (size_t)total * R.G + 128 * (size_t)N * (R.G + 1) + ((size_t)1 << 30);
-    if (5 * one + pos + arrays <= free_b &&
-        (cudaMalloc(&R.d_dist, 2 * one) != cudaSuccess || cudaMalloc(&R.d_wgt, 2 * one) != cudaSuccess ||
-         cudaMalloc(&R.d_wgt3, one) != cudaSuccess || cudaMalloc(&R.d_pos, pos) != cudaSuccess)) {
+    const bool weights = sizeof(T) == 8;
+    if ((weights ? 5 : 2) * one + pos + arrays <= free_b &&
+        (cudaMalloc(&R.d_dist, 2 * one) != cudaSuccess ||
+         (weights && (cudaMalloc(&R.d_wgt, 2 * one) != cudaSuccess || cudaMalloc(&R.d_wgt3, one) != cudaSuccess)) ||
+         cudaMalloc(&R.d_pos, pos) != cudaSuccess)) {
       cudaGetLastError();
       drop_stream(R);
     }
