@@ -1,0 +1,21 @@
+// The isotropic part of a scattering row added to a float: compiled for the device, and by the tests for the host.
+#pragma once
+#include <cmath>
+
+#ifdef __CUDACC__
+#define RRHD_BOTH __host__ __device__ __forceinline__
+#else
+#define RRHD_BOTH inline
+#endif
+
+// v + iso, iso = hi + lo (a double split in two floats), rounded to float once but for terms of
+// 2^-48 iso: conversions to double and back run at a fraction of the FP32 rate and were a third of
+// the scattering drain's store phase.  The sum of v and hi is taken apart in the form that needs
+// neither to be the larger (signed intensities leave an anisotropic part above the isotropic one);
+// where it is not finite it is the result.  Additions only: there is nothing to contract.
+RRHD_BOTH float add_iso(float v, float hi, float lo) {
+  const float s = hi + v;
+  const float b = s - hi;
+  const float e = (hi - (s - b)) + (v - b);
+  return fabsf(s) < INFINITY ? s + (e + lo) : s;
+}

@@ -50,6 +50,7 @@
 #include "coupled.h"
 #include "rrhd_internal.h"
 
+#include "add_iso.h"
 #include "dirs.h"
 #include "umma.cuh"
 
@@ -122,16 +123,6 @@ __device__ __forceinline__ void split4(const float (&x)[4], uint2 &hi, uint2 &lo
       lo = make_uint2(0u, 0u);
     }
   }
-}
-
-// v + iso, iso = hi + lo (a double split in two floats), rounded to float once but for terms of
-// 2^-48: conversions to double and back run at a fraction of the FP32 rate and were a third of
-// the drain's store phase.  |v| <= hi (the kernel's anisotropic part is at most the isotropic
-// one); where their sum is not finite it is the result.
-__device__ __forceinline__ float add_iso(float v, float hi, float lo) {
-  const float s = __fadd_rn(hi, v);
-  const float r = __fadd_rn(__fsub_rn(v, __fsub_rn(s, hi)), lo);
-  return fabsf(s) < INFINITY ? __fadd_rn(s, r) : s;
 }
 
 // eight floats of one row, a whole 32-byte sector in one access (32-byte aligned)
