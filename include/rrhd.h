@@ -502,12 +502,10 @@ typedef struct {
                              0 = min(64, M).  All directions are swept in one launch        */
   double boundary_value;  /* intensity entering through boundary faces (illum::BoundaryConditions
                              returns 0 for free, lock and outer boundaries, illum_utils.cpp:52-65) */
-  int32_t item_geometry;  /* 0 or 1 (1: RRHD_RAD_FP32 and RRHD_RAD_MIXED only).  The sweep order keeps, per
-                             (cell, direction) item, which faces are in- and out-faces, the traced
-                             distances and the face weights (16 bytes and five values of the
-                             arithmetic's precision) whatever this says, where device memory holds
-                             them beside a coupled step's arrays; else it forms the             
-                             distances and weights again from the cells' records               */
+  int32_t item_geometry;  /* 0 or 1 (1: RRHD_RAD_FP32 and RRHD_RAD_MIXED only); changes nothing.  The plan
+                             keeps 16 bytes per (cell, direction) item, and beside them, as far as
+                             rrhd_rad_memory and the device allow, its traced distances, position
+                             and face weights; else they are formed again from the cells' records */
 } rrhd_rad_opts;
 /* Builds the sweep geometry and plan for ctx's mesh and the direction set (which
  * must outlive the context's radiation use).  RRHD_ERR_STATE if the mesh has a
@@ -515,6 +513,25 @@ typedef struct {
 rrhd_status rrhd_rad_setup(rrhd_ctx *ctx, const rrhd_dirs *dirs, const rrhd_rad_opts *opts);
 /* Levels summed over direction batches and the largest level (items). */
 rrhd_status rrhd_rad_plan_info(const rrhd_ctx *ctx, int64_t *levels, int64_t *max_level_items);
+/* Most device memory, in bytes, that ctx's sweeps keep beyond the plan: the scratch of a caller's
+ * sweep (one direction is always kept, cells x groups values) and the geometry stream (20 bytes an
+ * item for distances and positions and 24 for weights in double arithmetic, 12 in float).  Also bounds the scratch
+ * of the plan's build.  bytes < 0 (the default): no bound, but rrhd_rad_setup leaves room for two
+ * arrays of the intensity's size and a sixteenth of the device's memory, a first sweep or coupled step,
+ * which may add what did not fit at setup, a sixteenth.  Frees what is kept above the bound; stays for later
+ * setups.  Results do not depend on it. */
+rrhd_status rrhd_rad_memory(rrhd_ctx *ctx, int64_t bytes);
+/* The form a sweep of ctx takes now. */
+typedef struct {
+  int32_t cluster;      /* CTAs that share a direction                                                */
+  int32_t ctas_per_sm;  /* 1 or 2                                                                     */
+  int32_t wide_slots;   /* 1: slot numbers beyond 16 bits                                             */
+  int32_t stream;       /* geometry kept: 0 none, 1 distances and positions, 2 all                    */
+  int32_t scratch_dirs; /* directions the scratch of a caller's sweep holds, 0 before it is made      */
+  int32_t build_dirs;   /* directions of one pass of the plan's build                                 */
+  int64_t slots_shared, slots_global; /* outgoing values a direction keeps at most, in shared and in global memory */
+} rrhd_rad_form;
+rrhd_status rrhd_rad_plan_form(const rrhd_ctx *ctx, rrhd_rad_form *form);
 /* The plan as the reference's sweep order would number it: levels [M][N] (caller cell
  * numbering) the level of direction d's batch in which cell c is swept for d -- the
  * depth of c in the upwind graph of d, which is the index of the front graph::

@@ -88,6 +88,11 @@ class RadOpts(C.Structure):
                 ("item_geometry", I32)]
 
 
+class RadForm(C.Structure):
+    _fields_ = [("cluster", I32), ("ctas_per_sm", I32), ("wide_slots", I32), ("stream", I32), ("scratch_dirs", I32),
+                ("build_dirs", I32), ("slots_shared", C.c_int64), ("slots_global", C.c_int64)]
+
+
 class CoupledOpts(C.Structure):
     _fields_ = [("scatter", I32), ("guess", P), ("k_stall", I32), ("absorption", D), ("scattering", D),
                 ("emission", Emission)]
@@ -152,6 +157,8 @@ _SIGS = {
     "rrhd_con2prim_batch_mlp": (I32, [P, I32, D, P, P, P, I64, I32, I32, P, P, P, P]),
     "rrhd_rad_setup": (I32, [P, P, P]),
     "rrhd_rad_plan_info": (I32, [P, P, P]),
+    "rrhd_rad_plan_form": (I32, [P, P]),
+    "rrhd_rad_memory": (I32, [P, I64]),
     "rrhd_rad_plan_levels": (I32, [P, P]),
     "rrhd_sweep": (I32, [P, P, P, P, P, P]),
     "rrhd_coupled_step": (I32, [P, D, P, P, P]),

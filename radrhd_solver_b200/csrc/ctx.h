@@ -66,20 +66,22 @@ struct RadState {
   // the plan: per direction its N items in level order and the level offsets
   uint4 *d_ord = nullptr;     // [M][N] {cell, code word, own and upwind slots (16 bits each)}
   uint2 *d_ord_hi = nullptr;  // [M][N] upper halves of the slots, where 16 bits do not hold them
-  // geometry stream, where memory allows: [M][N][2] distances, [M][N][2] and [M][N] in-face weights
+  // geometry stream, where memory allows: [M][N][2] distances, [M][N][2] and [M][N] weights (double)
   void *d_dist = nullptr, *d_wgt = nullptr, *d_wgt3 = nullptr;
-  uint32_t *d_pos = nullptr;  // [M][N] each cell's position in sweep order, with the stream
+  uint32_t *d_pos = nullptr;  // [M][N] each cell's position in sweep order, with the distances
   int32_t *d_lvl = nullptr, *d_depth = nullptr;  // level offsets of all directions; levels per direction
   int64_t *d_lvl_base = nullptr;                 // first entry of a direction in d_lvl
   std::vector<int32_t> depth;
   std::vector<int64_t> lvl_base;
   int64_t levels = 0, max_level = 0;
-  bool two = false;             // two CTAs of the sweep share an SM
-  int cl = 1;  // CTAs that share a direction of the sweep
-  int64_t nlow = 0, nhigh = 0;  // most slots a direction has in shared (slot 0: the boundary value) and global memory
-  void *d_slots = nullptr;      // [M][nhigh][G]
-  void *d_x = nullptr;          // S, then I, in the sweep's layout, [xdirs][N][G]
+  bool two = false;         // two CTAs of the sweep may share an SM (with S and I in sweep order)
+  int cl = 1;               // CTAs that share a direction of the sweep
+  int build_dirs = 0;       // directions of a pass of the plan's build
+  int64_t slots = 0;        // most slots a direction has (slot 0: the boundary value)
+  void *d_slots = nullptr;  // [M][slots beyond shared memory][G]
+  void *d_x = nullptr;      // S, then I, in the sweep's layout, [xdirs][N][G]
   int xdirs = 0;
+  bool settled = false;  // memory for the stream and the scratch has been looked for with the caller's arrays made
   // phase marks of the last coupled step: 0 start, 1 hydro done, 2 sweep done, 3 source
   // start and 4 source done (side stream), 5 join, 6 scattering done
   cudaEvent_t ev[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -155,6 +157,7 @@ struct rrhd_ctx {
   std::vector<uint8_t> h_cell_sign;
   std::vector<double> h_face_n, h_face_area, h_cell_V;
 
+  int64_t rad_keep = -1;  // most the sweep keeps beyond its plan, in bytes; negative: no bound
   rrhd::RadState rad;
 };
 

@@ -268,9 +268,9 @@ struct SweepArgs {
   int qs;                   // 1: Q per group, 0: one for all
   const uint4 *ord;         // [M][N] items in sweep order {cell, code, own | in0 << 16, in1 | in2 << 16}
   const uint2 *ord_hi;      // [M][N] upper halves of the slots (WIDE)
-  const T *dist;            // [M][N][2] {tA, tB} (GEO)
-  const T *wgt, *wgt3;      // [M][N][2], [M][N] weights (GEO, double)
-  const T *rec, *w, *wt;    // geometry records and directions (not GEO), face weights [N][4]
+  const T *dist;            // [M][N][2] {tA, tB} (GEO >= 1)
+  const T *wgt, *wgt3;      // [M][N][2], [M][N] weights (GEO 2)
+  const T *rec, *w, *wt;    // geometry records and directions (GEO 0), face weights [N][4]
   const int32_t *lvl;       // level offsets of every direction
   const int64_t *lvl_base;  // [M] first entry in lvl
   const int32_t *depth;     // [M] levels
@@ -296,7 +296,8 @@ __device__ __forceinline__ void bulk_prefetch(const P *p, uint32_t n) {
 
 // One CTA per direction.  GT: compile-time group count (1, 2 or 4; S and I in the sweep's own
 // layout), 0 for any other.  HIGH: slots from a.cap on are in global memory (the others in
-// shared memory).  GEO: distances, and in double the weights, from the stream, else from the cell's records.
+// shared memory).  GEO: from the stream come 0 nothing (distances and weights from the cell's
+// records), 1 the distances (weights from the cell's sector), 2 the weights as well (double).
 // Slots 0 and 1 hold the boundary value and zero (for in-faces an item does not have); an item
 // whose own slot is 0 has no downwind neighbour and writes none.
 //
@@ -314,11 +315,11 @@ __device__ __forceinline__ void bulk_prefetch(const P *p, uint32_t n) {
 // CLUSTER: a.cl CTAs of a cluster share a direction's levels (few directions with long fronts);
 // slots 2 and up are in global memory, where a level's values pass from CTA to CTA over the
 // cluster barrier.
-template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB, bool CLUSTER>
+template <class T, class TI, int GT, bool HIGH, bool WIDE, int GEO, int NT, int NB, bool CLUSTER>
 __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
   extern __shared__ __align__(16) uint8_t sweep_smem[];
   constexpr int GR = GT > 0 ? GT : 1;
-  constexpr bool WGT = GEO && sizeof(T) == 8;  // weights from the stream
+  constexpr bool WGT = GEO == 2;
   const int cl = CLUSTER ? a.cl : 1, x = (int)blockIdx.x / cl, d = a.d0 + x;
   const int first = CLUSTER ? ((int)blockIdx.x - x * cl) * NT + (int)threadIdx.x : (int)threadIdx.x;  // in a level
   const int step = cl * NT, kAhead = 4 * step;
@@ -712,7 +713,7 @@ __global__ void k_plan_offsets(int64_t N, int64_t total, int lbits, int d0, cons
   if (k == N - 1) o[L + 1] = (int32_t)N;
 }
 
-// Items of one direction per CTA in sweep order: face choice, distances and slots.  Within a
+// Items of one direction per CTA in sweep order: face choice and slots.  Within a
 // level the cells' own slots are taken first (from the free list, or a new one), then the
 // slots whose last reader sits in this level go back, so a slot is never written in a level
 // that reads it.  Slots below cap2 (the shared memory of one CTA of two per SM) are preferred,
@@ -723,15 +724,13 @@ template <class T>
 __global__ void __launch_bounds__(kPlanThreads)
     k_plan_items(int64_t N, int d0, const T *w, const T *rec, const int32_t *lvl_all, const int64_t *lvl_base,
                  const int32_t *depth, const uint32_t *order_all, uint32_t *slot_all, uint32_t *readers_all,
-                 uint32_t *freed_all, uint4 *ord_all, uint2 *hi_all, const T *wt, T *dist_all, T *wgt_all, T *wgt3_all,
-                 uint32_t *pos_all, int cap2, int cap1, int32_t *need) {
+                 uint32_t *freed_all, uint4 *ord_all, uint2 *hi_all, const T *wt, int cap2, int cap1, int32_t *need) {
   __shared__ int top[3], next[3];  // free list and next new slot below cap2, below cap1, beyond
   const int x = blockIdx.x, d = d0 + x;
   const uint32_t *order = order_all + x * N;
   uint32_t *slot_of = slot_all + x * N, *readers = readers_all + x * N, *freed = freed_all + x * N;
   uint4 *ord = ord_all + (int64_t)d * N;
   uint2 *hi16 = hi_all ? hi_all + (int64_t)d * N : nullptr;
-  const int64_t at = (int64_t)d * N;
   const int32_t *lvl = lvl_all + lvl_base[d];
   const T wx = w[3 * d], wy = w[3 * d + 1], wz = w[3 * d + 2];
   if (threadIdx.x == 0) {
@@ -781,26 +780,14 @@ __global__ void __launch_bounds__(kPlanThreads)
         const int b = f == 0 ? nbr[0] : f == 1 ? nbr[1] : f == 2 ? nbr[2] : nbr[3];
         if (q < nin) s[q] = b >= 0 ? slot_of[b] : 0u;
       }
-      if (pos_all) pos_all[at + c] = (uint32_t)i;
-      T f[4], wq[3], wo;
       if constexpr (sizeof(T) == 8) {
+        T f[4], wq[3], wo;
         ld_cell_weights(wt + 4 * c, f);
         item_weights(f, code, wq, wo);
-        const uint32_t left = left_out(code, wq, wo);
-        pack_weights(left, wq, wo);
-        code |= left << kLeftBit;
+        code |= left_out(code, wq, wo) << kLeftBit;
       }
       ord[i] = make_uint4((uint32_t)c, code, (own & 0xffffu) | s[0] << 16, (s[1] & 0xffffu) | s[2] << 16);
       if (hi16) hi16[i] = make_uint2(own >> 16 | (s[0] & 0xffff0000u), s[1] >> 16 | (s[2] & 0xffff0000u));
-      if (dist_all) {
-        dist_all[2 * (at + i)] = tA;
-        dist_all[2 * (at + i) + 1] = tB;
-      }
-      if (wgt_all) {
-        wgt_all[2 * (at + i)] = wq[0];
-        wgt_all[2 * (at + i) + 1] = wq[1];
-        wgt3_all[at + i] = wq[2];
-      }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -832,6 +819,36 @@ __global__ void __launch_bounds__(kPlanThreads)
     __syncthreads();
   }
   if (threadIdx.x == 0) need[d] = next[2] > cap1 ? next[2] : next[1] > cap2 ? next[1] : next[0];
+}
+
+// The geometry stream of all items from their order: distances and positions (dist), weights
+// (wgt; double), each where it is not null.
+template <class T>
+__global__ void k_fill_stream(int64_t N, int64_t total, const uint4 *ord, const T *w, const T *rec, const T *wt,
+                              T *dist, uint32_t *pos, T *wgt, T *wgt3) {
+  const int64_t at = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (at >= total) return;
+  const int64_t d = at / N;
+  const uint4 o = __ldcs(ord + at);
+  const int64_t c = o.x;
+  if (dist) {
+    T g[16], cosf[4], tA, tB;
+    load_vec<T>(rec + c * Rec<T>::RW, g, 16);
+    face_cos(g, w[3 * d], w[3 * d + 1], w[3 * d + 2], cosf);
+    (void)item_geometry<T>(g, cosf, tA, tB);
+    dist[2 * at] = tA;
+    dist[2 * at + 1] = tB;
+    pos[d * N + c] = (uint32_t)(at - d * N);
+  }
+  if (wgt) {
+    T f[4], wq[3], wo;
+    ld_cell_weights(wt + 4 * c, f);
+    item_weights(f, o.y, wq, wo);
+    pack_weights((o.y >> kLeftBit) & 3u, wq, wo);
+    wgt[2 * at] = wq[0];
+    wgt[2 * at + 1] = wq[1];
+    wgt3[at] = wq[2];
+  }
 }
 
 // Source record {k = alpha + betta, betta / k, alpha Q_g / k} of each context cell
@@ -999,7 +1016,7 @@ int cluster_size(const RadState &R, int64_t slots) {
   return cl;
 }
 
-template <class T, class TI, int GT, bool HIGH, bool WIDE, bool GEO, int NT, int NB>
+template <class T, class TI, int GT, bool HIGH, bool WIDE, int GEO, int NT, int NB>
 cudaError_t launch_sweep_kernel(const SweepArgs<T, TI> &a, int nd, size_t smem, cudaStream_t st) {
   if constexpr (HIGH && NT == 512) {
     if (a.cl > 1) {
@@ -1026,8 +1043,25 @@ cudaError_t launch_sweep_kernel(const SweepArgs<T, TI> &a, int nd, size_t smem, 
 
 template <class T, class TI, int GT, bool HIGH, bool WIDE, int NT, int NB>
 cudaError_t launch_sweep_geo(const SweepArgs<T, TI> &a, int nd, size_t smem, cudaStream_t st) {
-  return a.dist ? launch_sweep_kernel<T, TI, GT, HIGH, WIDE, true, NT, NB>(a, nd, smem, st)
-                : launch_sweep_kernel<T, TI, GT, HIGH, WIDE, false, NT, NB>(a, nd, smem, st);
+  if constexpr (sizeof(T) == 8)
+    if (a.wgt) return launch_sweep_kernel<T, TI, GT, HIGH, WIDE, 2, NT, NB>(a, nd, smem, st);
+  return a.dist ? launch_sweep_kernel<T, TI, GT, HIGH, WIDE, 1, NT, NB>(a, nd, smem, st)
+                : launch_sweep_kernel<T, TI, GT, HIGH, WIDE, 0, NT, NB>(a, nd, smem, st);
+}
+
+// How the slots lie at a launch: two CTAs an SM only with S and I in sweep order.
+struct Shape {
+  bool two;
+  int cap;
+  int64_t low, high;
+};
+Shape shape_of(const RadState &R) {
+  Shape q;
+  q.two = R.two && R.d_pos;
+  q.cap = R.cl > 1 ? 2 : slot_cap(R, q.two);
+  q.low = std::min<int64_t>(R.slots, q.cap);
+  q.high = std::max<int64_t>(0, R.slots - q.cap);
+  return q;
 }
 
 template <class T, class TI, int GT>
@@ -1068,9 +1102,10 @@ rrhd_status launch_sweep(rrhd_ctx *c, int d0, int nd, const void *S, void *I, in
   a.depth = R.d_depth;
   a.src = (const T *)R.d_src;
   a.slots = (T *)R.d_slots;
-  a.cap = R.cl > 1 ? 2u : (uint32_t)slot_cap(R, R.two);
+  const Shape q = shape_of(R);
+  a.cap = (uint32_t)q.cap;
   a.cl = R.cl;
-  a.nhigh = R.nhigh;
+  a.nhigh = q.high;
   a.S = (const TI *)S;
   a.I = (TI *)I;
   a.sc = sc;
@@ -1079,10 +1114,10 @@ rrhd_status launch_sweep(rrhd_ctx *c, int d0, int nd, const void *S, void *I, in
   a.bc = (T)R.bc;
   cudaError_t e;
   switch (R.G) {
-    case 1: e = launch_sweep_groups<T, TI, 1>(a, R.nlow, R.two, nd, c->stream); break;
-    case 2: e = launch_sweep_groups<T, TI, 2>(a, R.nlow, R.two, nd, c->stream); break;
-    case 4: e = launch_sweep_groups<T, TI, 4>(a, R.nlow, R.two, nd, c->stream); break;
-    default: e = launch_sweep_groups<T, TI, 0>(a, R.nlow, R.two, nd, c->stream); break;
+    case 1: e = launch_sweep_groups<T, TI, 1>(a, q.low, q.two, nd, c->stream); break;
+    case 2: e = launch_sweep_groups<T, TI, 2>(a, q.low, q.two, nd, c->stream); break;
+    case 4: e = launch_sweep_groups<T, TI, 4>(a, q.low, q.two, nd, c->stream); break;
+    default: e = launch_sweep_groups<T, TI, 0>(a, q.low, q.two, nd, c->stream); break;
   }
   RRHD_CUDA(e);
   return RRHD_OK;
@@ -1118,66 +1153,209 @@ cudaError_t move_tiles(rrhd_ctx *c, int d0, int nd, const void *in, void *out, b
   }
 }
 
-void drop_stream(RadState &R) {
-  for (void **p : {&R.d_dist, &R.d_wgt, &R.d_wgt3, (void **)&R.d_pos}) {
+// ---------------------------------------------------------------- memory
+// Beyond its plan a sweep keeps, where memory allows, in the order they are taken:
+//   the scratch in the sweep's layout, of all directions or of as many as run at once (one at
+//     least: without it a caller's sweep cannot run);
+//   the first part of the geometry stream, distances (2 values an item) and positions (4 bytes),
+//     which spares an item its cell's 144-byte record and brings S and I into sweep order;
+//   the second part, weights (3 values an item, in double; a sweep in float takes the cell's).
+// 96^3 x 6 cells x 256 directions x 4 groups in double, 21.7 GB of plan and 43.5 GB an array:
+// with both parts (27.2 and 32.6 GB) a coupled step's sweep takes 204 ms, 234 with the first alone,
+// 389 with none; a caller's sweep 294 with the first and 446 with none.  All results are the same bits.
+// At setup they are kept beside the two arrays of the intensity's size that a coupled step or a
+// caller will make; once those exist (first sweep, coupled step), beside a sixteenth of the device's
+// memory, which is the caller's.  c->rad_keep bounds their sum where the caller has set it.
+void drop_weights(RadState &R) {
+  for (void **p : {&R.d_wgt, &R.d_wgt3}) {
     cudaFree(*p);
     *p = nullptr;
   }
 }
+void drop_stream(RadState &R) {
+  drop_weights(R);
+  for (void **p : {&R.d_dist, (void **)&R.d_pos}) {
+    cudaFree(*p);
+    *p = nullptr;
+  }
+}
+void drop_scratch(RadState &R) {
+  cudaFree(R.d_x);
+  R.d_x = nullptr;
+  R.xdirs = 0;
+}
 
-// One sweep of every direction: S and I [N][M][G] in context numbering (cdg), or [N*G][M] in
-// caller numbering, swept in place in a scratch in the sweep's layout.  The caller's arrays go
-// through R.d_x, as many directions at a time as memory allows.  With swapped, S and I are the
-// coupled step's own and neither is needed again as it is: I is the scratch, the result takes
-// S's place, and *swapped says so; at 96^3 x 6 cells, 256 directions and 4 groups in double the
-// 43.5 GB saved are what the geometry stream needs (sweep 204 ms; 389 without the stream).
-template <class T, class TI>
-rrhd_status run_sweep_t(rrhd_ctx *c, const void *S, void *I, bool cdg, bool *swapped) {
-  RadState &R = c->rad;
-  const int64_t rows = c->N * R.G;
-  const size_t cd = sizeof(TI) * R.G;  // bytes of a (cell, direction)
-  if (cdg && !(cd == 4 || cd == 8 || cd == 16 || cd == 32))
-    return launch_sweep<T, TI>(c, 0, R.M, S, I, (int64_t)R.M * R.G, R.G, false, true);
-  if (swapped) {
-    RRHD_CUDA((move_tiles<TI, true>(c, 0, R.M, S, I, cdg)));
-    const rrhd_status s = launch_sweep<T, TI>(c, 0, R.M, I, I, R.G, rows, by_position<TI>(R), cdg);
-    if (s) return s;
-    RRHD_CUDA((move_tiles<TI, false>(c, 0, R.M, I, const_cast<void *>(S), cdg)));
-    *swapped = true;
-    return RRHD_OK;
-  }
-  if (!R.d_x) {
-    // as many directions as there are, or as memory allows (at least one); the geometry stream
-    // makes room if there would be fewer CTAs than SMs
-    R.xdirs = R.M;
-    while (cudaMalloc(&R.d_x, sizeof(TI) * (size_t)rows * R.xdirs) != cudaSuccess) {
-      cudaGetLastError();
-      R.d_x = nullptr;
-      if (R.d_dist && (R.xdirs + 1) / 2 < std::min(R.M, kSweepSMs)) {
-        RRHD_CUDA(cudaStreamSynchronize(c->stream));
-        drop_stream(R);
-        R.xdirs = R.M;
-        continue;
-      }
-      if (R.xdirs == 1) return rrhd_fail(RRHD_ERR_OOM, "sweep scratch allocation failed");
-      R.xdirs = (R.xdirs + 1) / 2;
-    }
-  }
-  for (int d0 = 0; d0 < R.M; d0 += R.xdirs) {
-    const int nd = std::min(R.xdirs, R.M - d0);
-    RRHD_CUDA((move_tiles<TI, true>(c, d0, nd, S, R.d_x, cdg)));
-    const rrhd_status s = launch_sweep<T, TI>(c, d0, nd, R.d_x, R.d_x, R.G, rows, by_position<TI>(R), cdg);
-    if (s) return s;
-    RRHD_CUDA((move_tiles<TI, false>(c, d0, nd, R.d_x, I, cdg)));
+struct Sizes {
+  size_t x;            // scratch of one direction
+  size_t geo, wgt;     // the stream's parts
+  size_t kept;         // what is kept now
+};
+Sizes sizes_of(const rrhd_ctx *c) {
+  const RadState &R = c->rad;
+  const size_t tv = R.prec == RRHD_RAD_FP32 ? sizeof(float) : sizeof(double), total = (size_t)c->N * R.M;
+  Sizes z;
+  z.x = (R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float)) * (size_t)c->N * R.G;
+  z.geo = (2 * tv + sizeof(uint32_t)) * total;
+  z.wgt = R.prec == RRHD_RAD_FP32 ? 0 : 3 * tv * total;
+  z.kept = (R.d_x ? z.x * R.xdirs : 0) + (R.d_dist ? z.geo : 0) + (R.d_wgt ? z.wgt : 0);
+  return z;
+}
+
+// Bytes that may be taken: what is free beside `reserve` (negative: a sixteenth of the device's
+// memory), within the caller's bound.
+rrhd_status room_of(const rrhd_ctx *c, int64_t reserve, size_t &room) {
+  size_t free_b = 0, all_b = 0;
+  RRHD_CUDA(cudaMemGetInfo(&free_b, &all_b));
+  const size_t hold = all_b / 16 + (reserve < 0 ? 0 : (size_t)reserve);
+  room = free_b > hold ? free_b - hold : 0;
+  if (c->rad_keep >= 0) {
+    const size_t kept = sizes_of(c).kept, keep = (size_t)c->rad_keep;
+    room = std::min(room, keep > kept ? keep - kept : (size_t)0);
   }
   return RRHD_OK;
 }
 
-rrhd_status run_sweep(rrhd_ctx *c, const void *S, void *I, bool cdg, bool *swapped = nullptr) {
+bool take(void **p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
+// directions of a sweep that run at once
+int at_once(const RadState &R) { return std::min(R.M, R.two ? 2 * kSweepSMs : kSweepSMs); }
+
+template <class T>
+rrhd_status fill_t(rrhd_ctx *c, int64_t reserve, bool scratch) {
+  RadState &R = c->rad;
+  const Sizes z = sizes_of(c);
+  size_t room = 0;
+  rrhd_status s = room_of(c, reserve, room);
+  if (s) return s;
+  const auto held = [&](bool got, size_t bytes) {
+    if (got) room -= bytes;
+    return got;
+  };
+  if (scratch && !R.d_x) {
+    const size_t geo = R.d_dist ? 0 : z.geo;
+    const int dirs = z.x * R.M + geo <= room ? R.M : z.x * at_once(R) <= room ? at_once(R) : 0;
+    if (dirs && held(take(&R.d_x, z.x * dirs), z.x * dirs)) R.xdirs = dirs;
+  }
+  const size_t tv = sizeof(T), total = (size_t)c->N * R.M;
+  bool geo = false, wgt = false;
+  if (!R.d_dist && z.geo <= room) {
+    geo = take(&R.d_dist, 2 * tv * total) && take((void **)&R.d_pos, sizeof(uint32_t) * total);
+    if (!held(geo, z.geo)) drop_stream(R);
+  }
+  if (z.wgt && R.d_dist && !R.d_wgt && z.wgt <= room) {
+    wgt = take(&R.d_wgt, 2 * tv * total) && take(&R.d_wgt3, tv * total);
+    if (!held(wgt, z.wgt)) drop_weights(R);
+  }
+  if (geo || wgt) {
+    k_fill_stream<T><<<grid_for((int64_t)total, 256), 256, 0, c->stream>>>(
+        c->N, (int64_t)total, R.d_ord, (const T *)R.d_w, (const T *)R.d_rec, (const T *)R.d_wt,
+        geo ? (T *)R.d_dist : nullptr, R.d_pos, wgt ? (T *)R.d_wgt : nullptr, (T *)R.d_wgt3);
+    RRHD_CUDA(cudaGetLastError());
+  }
+  return RRHD_OK;
+}
+rrhd_status fill(rrhd_ctx *c, int64_t reserve, bool scratch) {
+  return c->rad.prec == RRHD_RAD_FP32 ? fill_t<float>(c, reserve, scratch) : fill_t<double>(c, reserve, scratch);
+}
+
+// Frees, in steps, what a sweep can do without: the scratch (a later sweep makes another), the
+// weights, the rest of the stream.
+rrhd_status give_back(rrhd_ctx *c, bool &freed) {
+  RadState &R = c->rad;
+  freed = R.d_x || R.d_dist;
+  if (!freed) return RRHD_OK;
+  RRHD_CUDA(cudaStreamSynchronize(c->stream));
+  if (R.d_x)
+    drop_scratch(R);
+  else if (R.d_wgt)
+    drop_weights(R);
+  else
+    drop_stream(R);
+  return RRHD_OK;
+}
+
+// The scratch of a caller's sweep: of all directions, or of whole runs of as many as run at once;
+// the stream makes room for one such run, and if it is still too much the number is halved down to one.
+rrhd_status make_scratch(rrhd_ctx *c) {
+  RadState &R = c->rad;
+  const Sizes z = sizes_of(c);
+  const int run = at_once(R);
+  size_t room = 0;
+  rrhd_status s = room_of(c, -1, room);
+  if (s) return s;
+  int dirs = (int)std::min<size_t>(R.M, room / z.x);
+  if (dirs < R.M) dirs = std::max(run, dirs - dirs % run);
+  if (c->rad_keep >= 0)
+    dirs = (int)std::min<size_t>(dirs, std::max<size_t>(1, ((size_t)c->rad_keep - std::min((size_t)c->rad_keep, z.kept)) / z.x));
+  while (!take(&R.d_x, z.x * dirs)) {
+    if (dirs <= run && R.d_dist) {
+      bool freed = false;
+      if ((s = give_back(c, freed))) return s;
+      continue;
+    }
+    if (dirs == 1) return rrhd_fail(RRHD_ERR_OOM, "sweep scratch allocation failed");
+    dirs = dirs > run ? (dirs - 1) / run * run : (dirs + 1) / 2;
+  }
+  R.xdirs = dirs;
+  return RRHD_OK;
+}
+
+// One sweep of every direction on the caller's rows [N*G][M], swept in place in the scratch, as
+// many directions at a time as it holds.
+template <class T, class TI>
+rrhd_status run_sweep_rows(rrhd_ctx *c, const void *S, void *I) {
+  RadState &R = c->rad;
+  rrhd_status s;
+  if (!R.settled) {  // the caller's arrays exist by now
+    const bool short_of = !R.d_x || !R.d_dist || (sizeof(T) == 8 && !R.d_wgt);
+    if (short_of && (s = fill(c, -1, true))) return s;
+    R.settled = true;
+  }
+  if (!R.d_x && (s = make_scratch(c))) return s;
+  for (int d0 = 0; d0 < R.M; d0 += R.xdirs) {
+    const int nd = std::min(R.xdirs, R.M - d0);
+    RRHD_CUDA((move_tiles<TI, true>(c, d0, nd, S, R.d_x, false)));
+    if ((s = launch_sweep<T, TI>(c, d0, nd, R.d_x, R.d_x, R.G, c->N * R.G, by_position<TI>(R), false))) return s;
+    RRHD_CUDA((move_tiles<TI, false>(c, d0, nd, R.d_x, I, false)));
+  }
+  return RRHD_OK;
+}
+rrhd_status run_sweep_rows(rrhd_ctx *c, const void *S, void *I) {
   switch (c->rad.prec) {
-    case RRHD_RAD_FP64: return run_sweep_t<double, double>(c, S, I, cdg, swapped);
-    case RRHD_RAD_MIXED: return run_sweep_t<double, float>(c, S, I, cdg, swapped);
-    default: return run_sweep_t<float, float>(c, S, I, cdg, swapped);
+    case RRHD_RAD_FP64: return run_sweep_rows<double, double>(c, S, I);
+    case RRHD_RAD_MIXED: return run_sweep_rows<double, float>(c, S, I);
+    default: return run_sweep_rows<float, float>(c, S, I);
+  }
+}
+
+// ... and on the coupled step's arrays [N][M][G] in context numbering.  Neither is needed again as
+// it is, so the old intensity is the scratch, the result takes the place of the old scattering
+// integral, and the two change places.  Where a (cell, direction) is not a whole access (8 groups
+// and more) S is read and I written as they lie.
+template <class T, class TI>
+rrhd_status run_sweep_coupled(rrhd_ctx *c) {
+  RadState &R = c->rad;
+  const size_t cd = sizeof(TI) * R.G;
+  if (!(cd == 4 || cd == 8 || cd == 16 || cd == 32))
+    return launch_sweep<T, TI>(c, 0, R.M, R.d_S, R.d_I, (int64_t)R.M * R.G, R.G, false, true);
+  RRHD_CUDA((move_tiles<TI, true>(c, 0, R.M, R.d_S, R.d_I, true)));
+  const rrhd_status s =
+      launch_sweep<T, TI>(c, 0, R.M, R.d_I, R.d_I, R.G, c->N * R.G, by_position<TI>(R), true);
+  if (s) return s;
+  RRHD_CUDA((move_tiles<TI, false>(c, 0, R.M, R.d_I, R.d_S, true)));
+  std::swap(R.d_I, R.d_S);
+  return RRHD_OK;
+}
+rrhd_status run_sweep_coupled(rrhd_ctx *c) {
+  switch (c->rad.prec) {
+    case RRHD_RAD_FP64: return run_sweep_coupled<double, double>(c);
+    case RRHD_RAD_MIXED: return run_sweep_coupled<double, float>(c);
+    default: return run_sweep_coupled<float, float>(c);
   }
 }
 
@@ -1204,7 +1382,7 @@ int bits_for(int64_t n) {  // bits that hold 0 .. n - 1
   return b;
 }
 
-// The sweep order, items and slots of every direction (R.d_ord, the geometry stream, level offsets).
+// The sweep order, items and slots of every direction (R.d_ord, level offsets).
 template <class T>
 rrhd_status build_plan(rrhd_ctx *c) {
   RadState &R = c->rad;
@@ -1216,30 +1394,14 @@ rrhd_status build_plan(rrhd_ctx *c) {
     R.d_ord = nullptr;
     return rrhd_fail(oom, "sweep plan allocation failed (%lld bytes)", (long long)(sizeof(uint4) * total));
   }
-  // The geometry stream (5 values an item, 2 in float) spares each item its cell's geometry record, and
-  // the cells' positions bring S and I into sweep order.  They are kept where the memory left
-  // holds them beside what a coupled step allocates (intensity, scattering integral, moments,
-  // 4-force); else the sweep forms the same values again from the records and takes S and I by
-  // cell.
-  {
-    size_t free_b = 0, all_b = 0;
-    RRHD_CUDA(cudaMemGetInfo(&free_b, &all_b));
-    const size_t one = sizeof(T) * (size_t)total, pos = sizeof(uint32_t) * (size_t)total;
-    const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
-    const size_t arrays = 2 * ti * (size_t)total * R.G + 128 * (size_t)N * (R.G + 1) + ((size_t)1 << 30);
-    const bool weights = sizeof(T) == 8;
-    if ((weights ? 5 : 2) * one + pos + arrays <= free_b &&
-        (cudaMalloc(&R.d_dist, 2 * one) != cudaSuccess ||
-         (weights && (cudaMalloc(&R.d_wgt, 2 * one) != cudaSuccess || cudaMalloc(&R.d_wgt3, one) != cudaSuccess)) ||
-         cudaMalloc(&R.d_pos, pos) != cudaSuccess)) {
-      cudaGetLastError();
-      drop_stream(R);
-    }
-  }
-  // directions of a build pass: six 32-bit words a pair in at most half of the free memory
+  // directions of a build pass: six 32-bit words a pair (and a sort's) in at most half of the free
+  // memory, within the caller's bound
   size_t free_b = 0, all_b = 0;
   RRHD_CUDA(cudaMemGetInfo(&free_b, &all_b));
-  int B = (int)std::max<int64_t>(1, std::min<int64_t>(R.M, (int64_t)(free_b / 2) / (28 * N)));
+  int64_t build = (int64_t)(free_b / 2);
+  if (c->rad_keep >= 0) build = std::min(build, c->rad_keep);
+  const int B = (int)std::max<int64_t>(1, std::min<int64_t>(R.M, build / (28 * N)));
+  R.build_dirs = B;
   Scratch mem;
   uint32_t *buf[6];
   for (uint32_t *&b : buf)
@@ -1303,8 +1465,8 @@ rrhd_status build_plan(rrhd_ctx *c) {
     }
     auto items = [&]() -> rrhd_status {
       k_plan_items<T><<<nd, kPlanThreads, 0, st>>>(N, d0, w, rec, R.d_lvl, R.d_lvl_base, R.d_depth, order, indeg, key,
-                                                   cell, R.d_ord, R.d_ord_hi, (const T *)R.d_wt, (T *)R.d_dist, (T *)R.d_wgt,
-                                                   (T *)R.d_wgt3, R.d_pos, slot_cap(R, true), slot_cap(R, false), d_need);
+                                                   cell, R.d_ord, R.d_ord_hi, (const T *)R.d_wt, slot_cap(R, true),
+                                                   slot_cap(R, false), d_need);
       RRHD_CUDA(cudaGetLastError());
       RRHD_CUDA(cudaMemcpyAsync(need.data() + d0, d_need + d0, sizeof(int32_t) * nd, cudaMemcpyDeviceToHost, st));
       RRHD_CUDA(cudaStreamSynchronize(st));
@@ -1330,12 +1492,9 @@ rrhd_status build_plan(rrhd_ctx *c) {
     most = std::max<int64_t>(most, n);
   }
   const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
-  R.two = R.M > kSweepSMs && R.d_pos && ti * R.G >= 16 && (double)beyond <= kTwoBeyond * (double)all;
+  R.slots = most;
   R.cl = cluster_size(R, most);
-  if (R.cl > 1) R.two = false;
-  const int cap = R.cl > 1 ? 2 : slot_cap(R, R.two);
-  R.nlow = std::min<int64_t>(most, cap);
-  R.nhigh = std::max<int64_t>(0, most - cap);
+  R.two = R.cl == 1 && R.M > kSweepSMs && ti * R.G >= 16 && (double)beyond <= kTwoBeyond * (double)all;
   // rrhd_rad_plan_info: levels and the largest level over batches of R.DB directions
   std::vector<int32_t> off((size_t)entries);
   RRHD_CUDA(cudaMemcpyAsync(off.data(), R.d_lvl, sizeof(int32_t) * entries, cudaMemcpyDeviceToHost, st));
@@ -1422,14 +1581,18 @@ static rrhd_status rad_setup_t(rrhd_ctx *c) {
     return rrhd_fail(RRHD_ERR_OOM, "sweep allocation failed");
   }
   if ((s = build_plan<T>(c))) return s;
-  if (R.nhigh) {
-    const size_t bytes = sizeof(T) * (size_t)R.nhigh * R.G * R.M;
-    if (cudaMalloc(&R.d_slots, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      R.d_slots = nullptr;
+  Shape q = shape_of(R);  // without positions: one CTA an SM
+  int64_t high = q.high;
+  if (R.two) high = std::max<int64_t>(high, R.slots - slot_cap(R, true));
+  if (high) {
+    const size_t bytes = sizeof(T) * (size_t)high * R.G * R.M;
+    if (!take(&R.d_slots, bytes))
       return rrhd_fail(RRHD_ERR_OOM, "sweep slot allocation failed (%lld bytes)", (long long)bytes);
-    }
   }
+  const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
+  const size_t arrays = 2 * ti * (size_t)N * R.M * R.G + 128 * (size_t)N * (R.G + 1);
+  if ((s = fill(c, (int64_t)arrays, true))) return s;
+  RRHD_CUDA(cudaStreamSynchronize(c->stream));
   return RRHD_OK;
 }
 
@@ -1478,6 +1641,41 @@ extern "C" rrhd_status rrhd_rad_plan_info(const rrhd_ctx *c, int64_t *levels, in
   return RRHD_OK;
 }
 
+extern "C" rrhd_status rrhd_rad_plan_form(const rrhd_ctx *c, rrhd_rad_form *form) {
+  RRHD_CHECK_ARG(c && form, "null argument");
+  const RadState &R = c->rad;
+  if (!R.ready) return rrhd_fail(RRHD_ERR_STATE, "rrhd_rad_setup has not run");
+  const Shape q = shape_of(R);
+  form->cluster = R.cl;
+  form->ctas_per_sm = q.two ? 2 : 1;
+  form->wide_slots = R.d_ord_hi ? 1 : 0;
+  form->stream = !R.d_dist ? 0 : R.prec == RRHD_RAD_FP32 || R.d_wgt ? 2 : 1;
+  form->scratch_dirs = R.d_x ? R.xdirs : 0;
+  form->build_dirs = R.build_dirs;
+  form->slots_shared = q.low;
+  form->slots_global = q.high;
+  return RRHD_OK;
+}
+
+extern "C" rrhd_status rrhd_rad_memory(rrhd_ctx *c, int64_t bytes) {
+  RRHD_CHECK_ARG(c, "null context");
+  c->rad_keep = bytes < 0 ? -1 : bytes;
+  RadState &R = c->rad;
+  if (!R.ready) return RRHD_OK;
+  RRHD_CUDA(cudaSetDevice(c->device));
+  R.settled = false;  // a wider bound is used by the next sweep
+  if (R.d_x && R.xdirs < R.M) {
+    RRHD_CUDA(cudaStreamSynchronize(c->stream));
+    drop_scratch(R);
+  }
+  bool freed = true;
+  while (c->rad_keep >= 0 && freed && sizes_of(c).kept > (size_t)c->rad_keep) {
+    const rrhd_status s = give_back(c, freed);
+    if (s) return s;
+  }
+  return RRHD_OK;
+}
+
 extern "C" rrhd_status rrhd_rad_plan_levels(const rrhd_ctx *c, int32_t *levels) {
   RRHD_CHECK_ARG(c && levels, "null argument");
   const RadState &R = c->rad;
@@ -1514,7 +1712,7 @@ extern "C" rrhd_status rrhd_sweep(rrhd_ctx *c, const void *alpha, const void *be
     k_dyn_from_arrays<float, float><<<grid_for(N, 256), 256, 0, c->stream>>>(
         N, R.G, R.SW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q, (float *)R.d_src);
   RRHD_CUDA(cudaGetLastError());
-  return run_sweep(c, S, I, false);
+  return run_sweep_rows(c, S, I);
 }
 
 // ---------------------------------------------------------------- coupled step
@@ -1605,22 +1803,6 @@ rrhd_status move_rows(rrhd_ctx *c, void *array, double *to, const double *from) 
 }  // namespace
 
 namespace {
-// Frees what a sweep can do without: its scratch (a later sweep makes another), then the geometry
-// stream.  False: nothing left.
-rrhd_status give_back(rrhd_ctx *c, bool &freed) {
-  RadState &R = c->rad;
-  freed = R.d_x || R.d_dist;
-  if (!freed) return RRHD_OK;
-  RRHD_CUDA(cudaStreamSynchronize(c->stream));
-  if (R.d_x) {
-    cudaFree(R.d_x);
-    R.d_x = nullptr;
-  } else {
-    drop_stream(R);
-  }
-  return RRHD_OK;
-}
-
 void drop_coupled(RadState &R) {
   for (void **p : {&R.d_I, &R.d_S, (void **)&R.d_G4, (void **)&R.d_mE, (void **)&R.d_mF, (void **)&R.d_mT,
                    (void **)&R.d_mom, (void **)&R.d_cnt}) {
@@ -1652,11 +1834,17 @@ rrhd_status make_coupled(rrhd_ctx *c) {
                {(void **)&R.d_mF, fp64 ? sizeof(double) * 3 * rows : 0},
                {(void **)&R.d_mT, fp64 ? sizeof(double) * 9 * rows : 0},
                {(void **)&R.d_mom, fp64 ? 0 : sizeof(float) * 16 * rows}};
+  // a coupled step sweeps in its own arrays: the scratch is the first of them, or in the way
+  if (R.d_x && R.xdirs == R.M) {
+    std::swap(R.d_I, R.d_x);
+    R.xdirs = 0;
+  } else if (R.d_x) {
+    RRHD_CUDA(cudaStreamSynchronize(c->stream));
+    drop_scratch(R);
+  }
   for (const auto &q : parts) {
     if (!q.bytes) continue;
-    while (cudaMalloc(q.p, q.bytes) != cudaSuccess) {
-      cudaGetLastError();
-      *q.p = nullptr;
+    while (!*q.p && !take(q.p, q.bytes)) {
       bool freed = false;
       const rrhd_status s = give_back(c, freed);
       if (s) return s;
@@ -1666,7 +1854,7 @@ rrhd_status make_coupled(rrhd_ctx *c) {
   }
   for (cudaEvent_t &e : R.ev) RRHD_CUDA(cudaEventCreate(&e));
   RRHD_CUDA(cudaStreamCreateWithFlags(&R.side, cudaStreamNonBlocking));
-  return RRHD_OK;
+  return fill(c, -1, false);  // with the arrays made, what else of the stream fits
 }
 rrhd_status alloc_coupled(rrhd_ctx *c) {
   const rrhd_status s = make_coupled(c);
@@ -1745,9 +1933,7 @@ extern "C" rrhd_status rrhd_coupled_step(rrhd_ctx *c, double tau, const rrhd_cou
   }
   RRHD_CUDA(cudaEventRecord(R.ev[4], ss_st));
   // 3. sweep with the previous scattering integral
-  bool swapped = false;
-  if ((s = run_sweep(c, R.d_S, R.d_I, true, &swapped))) return s;
-  if (swapped) std::swap(R.d_I, R.d_S);
+  if ((s = run_sweep_coupled(c))) return s;
   RRHD_CUDA(cudaEventRecord(R.ev[2], st));
   // the scattering below overwrites the moments the source read, and the next step reads
   // the state the source wrote: join the side stream

@@ -202,7 +202,7 @@ class TransportSweep:
     (float arrays as "fp32", face values and the transport update in double).
     dirs_per_batch: directions whose levels plan_info counts together.  item_geometry
     ("fp32" and "mixed" only): accepted; every sweep keeps its items' geometry in sweep
-    order where device memory holds it."""
+    order where device memory holds it (limit_sweep_memory)."""
 
     def __init__(self, grid, dg: DirectionGrid, groups: int = 1, precision: str = "fp64", dirs_per_batch: int = 0,
                  boundary_value: float = 0.0, item_geometry: bool = False):
@@ -224,6 +224,19 @@ class TransportSweep:
         lv, mx = C.c_int64(), C.c_int64()
         L.check(L.lib.rrhd_rad_plan_info(self.grid.handle, C.byref(lv), C.byref(mx)), "rrhd_rad_plan_info")
         return lv.value, mx.value
+
+    def plan_form(self):
+        """The form a sweep takes now (rrhd_rad_form): CTAs a direction, where its values lie, what of the
+        geometry is kept."""
+        f = L.RadForm()
+        L.check(L.lib.rrhd_rad_plan_form(self.grid.handle, C.byref(f)), "rrhd_rad_plan_form")
+        return {name: getattr(f, name) for name, _ in f._fields_}
+
+
+def limit_sweep_memory(grid, bytes: int = -1):
+    """Most device memory the sweeps of `grid` keep beyond their plan (rrhd_rad_memory); negative: no bound
+    beyond what is left to the caller."""
+    L.check(L.lib.rrhd_rad_memory(grid.handle, bytes), "rrhd_rad_memory")
 
 
 def CalculateIllum(sw: TransportSweep, alpha, betta, Q, S, I=None):

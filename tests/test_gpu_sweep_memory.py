@@ -55,11 +55,12 @@ class Context:
 
 
 def test_coupled_arrays_all_or_none(mesh):
-    """8 groups: arrays of 402 MB.  The intensity fits, the scattering integral does not, not even with the
-    stream's 277 MB given back; the next call finds nothing that this one left behind."""
+    """8 groups: arrays of 402 MB.  The intensity is there (the sweep's scratch), the scattering integral does
+    not fit, not even with the stream's 277 MB given back; the next calls find nothing that this one left behind
+    (the intensity fits, then)."""
     c = Context(mesh, 8)
     S = 10 ** np.random.default_rng(53).uniform(-3, -1, (mesh.n_cells * 8, M))
-    held = leave(500)
+    held = leave(100)
     for _ in range(2):
         assert L.lib.rrhd_rad_set(c.grid.handle, L.RRHD_RAD_S, L.ptr(S)) == L.RRHD_ERR_OOM
         assert L.lib.rrhd_rad_get(c.grid.handle, L.RRHD_RAD_S, L.ptr(np.empty_like(S))) == L.RRHD_ERR_STATE
