@@ -110,9 +110,9 @@ __device__ __forceinline__ void face_cos(const T *g, T wx, T wy, T wz, T *cosf) 
 //                       the face areas sum to zero)
 //   bits 8-11           out-faces (cos > 0)
 //   bit 12              the node at b1's vertex is traced to b2 (else to b1, lam = 2/3)
-//   bit 13              some face is neither (parallel to the direction)
-//   bits 14-15          how the stream holds the weights (item_weights)
-constexpr uint32_t kCodeB2 = 1u << 12, kCodeOdd = 1u << 13;
+//   bit 13              the weights come from the cell: some face is neither (parallel to the
+//                       direction), or the third in-face is small (third_weight)
+constexpr uint32_t kCodeB2 = 1u << 12, kCodeCell = 1u << 13;
 
 // Code word and distances of one (cell, direction) from the cell's normals and heights
 // g[16]: tA = r_b1 / 6, tB = r_b2 / 6 (bit 12; else 0).  b1, b2: the smallest by (t, face
@@ -148,7 +148,7 @@ __device__ __forceinline__ uint32_t item_geometry(const T *g, const T *cosf, T &
   tA = tb1;
   tB = (T)0;
   uint32_t code = out << 8 | (uint32_t)n << 6;
-  if (n + __popc(out) != 4) code |= kCodeOdd;
+  if (n + __popc(out) != 4) code |= kCodeCell;
   if (n >= 1) code |= (uint32_t)b1;
   if (n >= 2) {
     code |= (uint32_t)b2 << 2;
@@ -178,37 +178,14 @@ __device__ __forceinline__ void item_weights(const T (&f)[4], uint32_t code, T (
   for (int j = 0; j < 4; j++) wo += (code >> (8 + j)) & 1u ? f[j] : (T)0;
 }
 
-// The stream keeps three of the four (in double; a sweep in float takes them from the cell's
-// sector).  They sum to one, so the largest, at least a quarter, is found again to a few roundings:
-// bits 14-15 of the code word say whose place (b1, b2, third) holds wo, 3 that wo is left out.
-// With one or two in-faces it is the third's, whose weight nothing is multiplied by.
-constexpr int kLeftBit = 14;
-template <class T>
-__device__ __forceinline__ uint32_t left_out(uint32_t code, const T (&w)[3], T wo) {
-  if (((code >> 6) & 3u) < 3u) return 2u;
-  uint32_t left = 3;
-  T most = wo;
-#pragma unroll
-  for (int q = 0; q < 3; q++)
-    if (w[q] > most) left = (uint32_t)q, most = w[q];
-  return left;
+// In double the stream keeps three of the four, of b1, b2 and the out-faces (a sweep in float takes
+// all from the cell's sector).  The third in-face's is what they leave of one, good to 2^-52 / its
+// size; below 1/16 the item takes its weights from the cell (no item of the jittered Kuhn meshes is).
+// Without a third in-face nothing is multiplied by it.
+__device__ __forceinline__ double third_weight(const double (&w)[3], double wo) {
+  return (1.0 - w[0]) - (w[1] + wo);
 }
-// the three of the stream ...
-template <class T>
-__device__ __forceinline__ void pack_weights(uint32_t left, T (&w)[3], T wo) {
-#pragma unroll
-  for (int q = 0; q < 3; q++)
-    if (left == (uint32_t)q) w[q] = wo;
-}
-// ... and all four again
-template <class T>
-__device__ __forceinline__ void unpack_weights(uint32_t left, T (&w)[3], T &wo) {
-  const T rest = ((T)1 - w[0]) - (w[1] + w[2]);
-  wo = rest;
-#pragma unroll
-  for (int q = 0; q < 3; q++)
-    if (left == (uint32_t)q) wo = w[q], w[q] = rest;
-}
+constexpr double kThirdMin = 1.0 / 16.0;
 
 // 32 bytes of global memory in one access (32-byte aligned)
 __device__ __forceinline__ void ld_32(const double *p, double &a, double &b, double &c, double &d) {
@@ -436,13 +413,13 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
       }
       const uint64_t c = now.o.x;
       const uint32_t code = now.o.y;
-      T w[3], cw[4];  // cw: the cell's weights, where there is no stream of them
+      T w[3], wo, cw[4];  // cw: the cell's weights, where there is no stream of them
       TI sv[GR];
       if constexpr (GT > 0) ld_groups<true>(S + (uint64_t)iq * (uint32_t)GT, sv);
       if constexpr (WGT) {
         const double2 u = __ldcs(reinterpret_cast<const double2 *>(wgt) + at_i);
         w[0] = u.x, w[1] = u.y;
-        w[2] = __ldcs(wgt3 + at_i);
+        wo = __ldcs(wgt3 + at_i);
       } else {
         ld_cell_weights(a.wt + 4 * c, cw);
       }
@@ -467,15 +444,10 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
       const T EA = ex(-k * tA);
       const T E2 = EA * EA, EX = ex(-k * tB);  // formed in any case: the two chains overlap
       const T EB = two ? EX : E2 * E2;
-      T wo;
       if constexpr (!WGT) item_weights(cw, code, w, wo);
-      if constexpr (sizeof(T) == 8) {  // the same bits with and without the stream
-        const uint32_t left = (code >> kLeftBit) & 3u;
-        if constexpr (!WGT) pack_weights(left, w, wo);
-        unpack_weights(left, w, wo);
-      }
+      if constexpr (sizeof(T) == 8) w[2] = third_weight(w, wo);  // the same bits with and without the stream
       T par = (T)0;  // a face parallel to the direction holds the boundary value
-      if (code & kCodeOdd) {
+      if (code & kCodeCell) {
         const int nin = (int)(code >> 6) & 3;
         uint32_t seen = (code >> 8) & 15u;
         if (nin > 0) seen |= 1u << (code & 3);
@@ -784,7 +756,7 @@ __global__ void __launch_bounds__(kPlanThreads)
         T f[4], wq[3], wo;
         ld_cell_weights(wt + 4 * c, f);
         item_weights(f, code, wq, wo);
-        code |= left_out(code, wq, wo) << kLeftBit;
+        if (((code >> 6) & 3u) == 3u && !(wq[2] >= kThirdMin)) code |= kCodeCell;
       }
       ord[i] = make_uint4((uint32_t)c, code, (own & 0xffffu) | s[0] << 16, (s[1] & 0xffffu) | s[2] << 16);
       if (hi16) hi16[i] = make_uint2(own >> 16 | (s[0] & 0xffff0000u), s[1] >> 16 | (s[2] & 0xffff0000u));
@@ -844,10 +816,9 @@ __global__ void k_fill_stream(int64_t N, int64_t total, const uint4 *ord, const 
     T f[4], wq[3], wo;
     ld_cell_weights(wt + 4 * c, f);
     item_weights(f, o.y, wq, wo);
-    pack_weights((o.y >> kLeftBit) & 3u, wq, wo);
     wgt[2 * at] = wq[0];
     wgt[2 * at + 1] = wq[1];
-    wgt3[at] = wq[2];
+    wgt3[at] = wo;
   }
 }
 

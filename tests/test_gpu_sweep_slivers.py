@@ -54,14 +54,36 @@ def directions(tilt):
     return Directions(np.ascontiguousarray(w), np.full(len(w), 4 * np.pi / len(w)), 4 * np.pi)
 
 
+def slim(n, width, seed):
+    """Tetrahedra over a tip below the middle of a base with one short side: the third in-face is small."""
+    rng = np.random.default_rng(seed)
+    a, b = rng.uniform(0.5, 1, (n, 2)), -rng.uniform(0.5, 1, (n, 2))
+    c = b + width * rng.uniform(-1, 1, (n, 2))
+    mid = (a + b + c) / 3
+    z = np.ones((n, 1))
+    corners = np.stack([np.hstack([x, y * z]) for x, y in ((a, 1), (b, 1), (c, 1), (mid, 0))], 1)
+    return np.stack([q[rng.permutation(4)] for q in corners])
+
+
 @pytest.mark.parametrize("bc", [0.0, 0.25])
 @pytest.mark.parametrize("precision,width,bar", [("fp64", 1e-6, 1e-12), ("mixed", 1e-6, 1e-7), ("fp32", 1e-3, 1e-5)])
 def test_small_out_faces(precision, width, bar, bc):
-    n, G = 240, 2
-    corners = needles(n, width, 1.0, 61)
-    corners[::4] = needles(n, 1.0, 0.2, 62)[::4]  # flat cells: the out-face is the largest
+    corners = needles(240, width, 1.0, 61)
+    corners[::4] = needles(240, 1.0, 0.2, 62)[::4]  # flat cells: the out-face is the largest
+    check(corners, directions(0.02 * width), precision, bar, bc)
+
+
+@pytest.mark.parametrize("bc", [0.0, 0.25])
+@pytest.mark.parametrize("precision,bar", [("fp64", 1e-12), ("mixed", 1e-7), ("fp32", 1e-5)])
+def test_small_third_in_face(precision, bar, bc):
+    """Weights of 0.001 to 0.3, on either side of the 1/16 below which they are taken from the cell."""
+    corners = np.concatenate([slim(120, 0.05, 64), slim(120, 0.5, 65)])
+    check(corners, directions(0.01), precision, bar, bc)
+
+
+def check(corners, d, precision, bar, bc):
+    n, G = len(corners), 2
     m = single_cells(corners)
-    d = directions(0.02 * width)
     real = np.float64 if precision == "fp64" else np.float32
     rng = np.random.default_rng(63)
     alpha = 10 ** rng.uniform(0.5, 1.5, n)  # no thin cells: 1 - exp(-k t) has its digits as well
