@@ -64,8 +64,17 @@ struct Rec {
   static constexpr int RW = 16 + 16 / (int)sizeof(T);  // words: 144 B in double, 80 B in float
 };
 // Per-cell source record (SW words): {k, betta/k, alpha Q_g/k}, one Q for all groups where
-// they share it (the coupled step).
-constexpr int kSrcQ = 2;
+// they share it (the coupled step).  In float with one or two groups the cell's weights follow at
+// word kSrcW: an item's record and weights are one 32-byte access.
+constexpr int kSrcQ = 2, kSrcW = 4;
+template <class T>
+constexpr bool weights_in_record(int G) {
+  return sizeof(T) == 4 && (G == 1 || G == 2);
+}
+template <class T>
+constexpr int source_words(int G, bool one_q) {
+  return weights_in_record<T>(G) ? 8 : one_q ? 4 : (kSrcQ + G + 3) / 4 * 4;
+}
 
 template <class T>
 __device__ __forceinline__ void load_vec(const T *r, T *g, int n) {
@@ -191,6 +200,12 @@ constexpr double kThirdMin = 1.0 / 16.0;
 __device__ __forceinline__ void ld_32(const double *p, double &a, double &b, double &c, double &d) {
   asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p) : "memory");
 }
+__device__ __forceinline__ void ld_32(const float *p, float &a, float &b, float &c, float &d, float (&e)[4]) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a), "=f"(b), "=f"(c), "=f"(d), "=f"(e[0]), "=f"(e[1]), "=f"(e[2]), "=f"(e[3])
+               : "l"(p)
+               : "memory");
+}
 __device__ __forceinline__ void st_32(double *p, double a, double b, double c, double d) {
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
@@ -292,11 +307,16 @@ __device__ __forceinline__ void bulk_prefetch(const P *p, uint32_t n) {
 // CLUSTER: a.cl CTAs of a cluster share a direction's levels (few directions with long fronts);
 // slots 2 and up are in global memory, where a level's values pass from CTA to CTA over the
 // cluster barrier.
+// A sweep in float with one group: 64 registers let two CTAs of 512 threads share an SM (14^3 x 6 cells
+// x 256 x 1 0.30 ms, 0.50 with the 72 it would take; 36^3 x 128 x 1 1.42 and 1.53).
+template <class T, int GT, bool HIGH, int NB>
+constexpr int kResident = sizeof(T) == 4 && GT == 1 && !HIGH ? 2 : NB;
 template <class T, class TI, int GT, bool HIGH, bool WIDE, int GEO, int NT, int NB, bool CLUSTER>
-__global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
+__global__ void __launch_bounds__(NT, (kResident<T, GT, HIGH, NB>)) k_sweep(const SweepArgs<T, TI> a) {
   extern __shared__ __align__(16) uint8_t sweep_smem[];
   constexpr int GR = GT > 0 ? GT : 1;
   constexpr bool WGT = GEO == 2;
+  constexpr bool AHEAD = sizeof(T) == 4;  // the cell's weights an item ahead, where they take few registers
   const int cl = CLUSTER ? a.cl : 1, x = (int)blockIdx.x / cl, d = a.d0 + x;
   const int first = CLUSTER ? ((int)blockIdx.x - x * cl) * NT + (int)threadIdx.x : (int)threadIdx.x;  // in a level
   const int step = cl * NT, kAhead = 4 * step;
@@ -333,6 +353,7 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
     uint2 hi;
     T tA, tB;
     T k, bk, q0, q1;  // q1: of the second group where each has its own
+    T cw[AHEAD ? 4 : 1];
   };
   auto load_record = [&](int i, Item &it) {
     it.o = __ldcs(ord + i);
@@ -351,9 +372,12 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
     const T *sr = reinterpret_cast<const T *>(src + (uint64_t)it.o.x * src_bytes);
     if constexpr (sizeof(T) == 8) {
       ld_32(sr, it.k, it.bk, it.q0, it.q1);
+    } else if constexpr (weights_in_record<T>(GT)) {
+      ld_32(sr, it.k, it.bk, it.q0, it.q1, it.cw);
     } else {
       const float4 t = __ldg(reinterpret_cast<const float4 *>(sr));
       it.k = t.x, it.bk = t.y, it.q0 = t.z, it.q1 = t.w;
+      ld_cell_weights(a.wt + 4 * (uint64_t)it.o.x, it.cw);
     }
   };
   // one thread asks L2 for the streams' lines some levels ahead
@@ -420,6 +444,9 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
         const double2 u = __ldcs(reinterpret_cast<const double2 *>(wgt) + at_i);
         w[0] = u.x, w[1] = u.y;
         wo = __ldcs(wgt3 + at_i);
+      } else if constexpr (AHEAD) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) cw[q] = now.cw[q];
       } else {
         ld_cell_weights(a.wt + 4 * c, cw);
       }
@@ -444,6 +471,12 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
       const T EA = ex(-k * tA);
       const T E2 = EA * EA, EX = ex(-k * tB);  // formed in any case: the two chains overlap
       const T EB = two ? EX : E2 * E2;
+      T v0[GR], v1[GR], v2[GR];
+      if constexpr (GT > 0) {  // asked for before the branch below
+        get_slot(s0, v0);
+        get_slot(s1, v1);
+        get_slot(s2, v2);
+      }
       if constexpr (!WGT) item_weights(cw, code, w, wo);
       if constexpr (sizeof(T) == 8) w[2] = third_weight(w, wo);  // the same bits with and without the stream
       T par = (T)0;  // a face parallel to the direction holds the boundary value
@@ -469,10 +502,7 @@ __global__ void __launch_bounds__(NT, NB) k_sweep(const SweepArgs<T, TI> a) {
       };
       if constexpr (GT > 0) {
         TI iv[GT];
-        T v0[GT], v1[GT], v2[GT], o[GT];
-        get_slot(s0, v0);
-        get_slot(s1, v1);
-        get_slot(s2, v2);
+        T o[GT];
 #pragma unroll
         for (int g = 0; g < GT; g++) {
           T q = now.q0, cell;
@@ -827,7 +857,7 @@ __global__ void k_fill_stream(int64_t N, int64_t total, const uint4 *ord, const 
 // distributed) from caller arrays (caller numbering) ...
 template <class T, class TA>
 __global__ void k_dyn_from_arrays(int64_t N, int G, int SW, const int32_t *perm, const TA *alpha, const TA *betta,
-                                  const TA *Q, T *src) {
+                                  const TA *Q, const T *wt, T *src) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= N) return;
   const int64_t p = perm[c];
@@ -837,12 +867,14 @@ __global__ void k_dyn_from_arrays(int64_t N, int G, int SW, const int32_t *perm,
   o[0] = k;
   o[1] = be / k;
   for (int g = 0; g < G; g++) o[kSrcQ + g] = (al * (T)Q[p * G + g]) / k;
+  if (weights_in_record<T>(G))
+    for (int j = 0; j < 4; j++) o[kSrcW + j] = wt[4 * c + j];
 }
 
 // ... or from the solver state: alpha = a rho, betta = b rho, Q_g = B(T) / kRadiation / G.
 template <class T>
 __global__ void k_dyn_from_state(int64_t N, int G, int SW, const double *state, double a_coef, double b_coef,
-                                 Emission em, T *src) {
+                                 Emission em, const T *wt, T *src) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= N) return;
   const double rho = state[10 * c + 5], prs = state[10 * c + 9];
@@ -853,6 +885,8 @@ __global__ void k_dyn_from_state(int64_t N, int G, int SW, const double *state, 
   o[0] = k;
   o[1] = be / k;
   o[kSrcQ] = (al * q) / k;
+  if (weights_in_record<T>(G))
+    for (int j = 0; j < 4; j++) o[kSrcW + j] = wt[4 * c + j];
 }
 
 // ---------------------------------------------------------------- coupled step
@@ -1043,6 +1077,13 @@ cudaError_t launch_sweep_groups(const SweepArgs<T, TI> &a, int64_t low, bool two
     if (a.nhigh) return launch_sweep_geo<T, TI, GT, true, false, 256, 2>(a, nd, smem, st);
     return launch_sweep_geo<T, TI, GT, false, false, 256, 2>(a, nd, smem, st);
   }
+  if constexpr (sizeof(T) == 4 && GT == 2) {
+    // The same with two groups, at a cost (64 registers of 77), so where it fills SMs twice and L2 holds
+    // the lines of twice as many fronts: 14^3 x 256 x 2 0.49 -> 0.33 ms, 36^3 3.05 -> 2.6, but 48^3 6.5 ->
+    // 10.6, 24^3 x 100 0.78 -> 0.82.
+    if (!a.nhigh && nd > kSweepSMs && 2 * smem <= kSmemOne && low * 128 * std::min(nd, 2 * kSweepSMs) <= (int64_t)320 << 20)
+      return launch_sweep_geo<T, TI, GT, false, false, 512, 2>(a, nd, smem, st);
+  }
   if (a.ord_hi) return launch_sweep_geo<T, TI, GT, true, true, 512, 1>(a, nd, smem, st);
   if (a.nhigh) return launch_sweep_geo<T, TI, GT, true, false, 512, 1>(a, nd, smem, st);
   return launch_sweep_geo<T, TI, GT, false, false, 512, 1>(a, nd, smem, st);
@@ -1064,7 +1105,7 @@ rrhd_status launch_sweep(rrhd_ctx *c, int d0, int nd, const void *S, void *I, in
   a.wgt = (const T *)R.d_wgt;
   a.wgt3 = (const T *)R.d_wgt3;
   a.qs = one_q ? 0 : 1;
-  a.SW = one_q ? 4 : R.SW;
+  a.SW = source_words<T>(R.G, one_q);
   a.wt = (const T *)R.d_wt;
   a.rec = (const T *)R.d_rec;
   a.w = (const T *)R.d_w;
@@ -1455,6 +1496,9 @@ rrhd_status build_plan(rrhd_ctx *c) {
       if ((s = items())) return s;
     }
   }
+  std::vector<int32_t> off((size_t)entries);
+  RRHD_CUDA(cudaMemcpyAsync(off.data(), R.d_lvl, sizeof(int32_t) * entries, cudaMemcpyDeviceToHost, st));
+  RRHD_CUDA(cudaStreamSynchronize(st));
   const int cap2 = slot_cap(R, true);
   int64_t all = 0, beyond = 0, most = 0;
   for (int32_t n : need) {
@@ -1467,9 +1511,6 @@ rrhd_status build_plan(rrhd_ctx *c) {
   R.cl = cluster_size(R, most);
   R.two = R.cl == 1 && R.M > kSweepSMs && ti * R.G >= 16 && (double)beyond <= kTwoBeyond * (double)all;
   // rrhd_rad_plan_info: levels and the largest level over batches of R.DB directions
-  std::vector<int32_t> off((size_t)entries);
-  RRHD_CUDA(cudaMemcpyAsync(off.data(), R.d_lvl, sizeof(int32_t) * entries, cudaMemcpyDeviceToHost, st));
-  RRHD_CUDA(cudaStreamSynchronize(st));
   R.levels = R.max_level = 0;
   for (int d0 = 0; d0 < R.M; d0 += R.DB) {
     std::vector<int64_t> items;
@@ -1505,7 +1546,7 @@ static rrhd_status rad_setup_t(rrhd_ctx *c) {
   RadState &R = c->rad;
   const int64_t N = c->N;
   constexpr int W = Rec<T>::RW;
-  R.SW = (kSrcQ + R.G + 3) / 4 * 4;
+  R.SW = source_words<T>(R.G, false);
   std::vector<T> rec((size_t)W * N, (T)0), wt((size_t)4 * N), w(3 * R.M);
   std::vector<int32_t> iperm(N);
   for (int64_t i = 0; i < N; i++) iperm[c->h_perm[i]] = (int32_t)i;
@@ -1675,13 +1716,16 @@ extern "C" rrhd_status rrhd_sweep(rrhd_ctx *c, const void *alpha, const void *be
   const int64_t N = c->N;
   if (R.prec == RRHD_RAD_FP64)
     k_dyn_from_arrays<double, double><<<grid_for(N, 256), 256, 0, c->stream>>>(
-        N, R.G, R.SW, c->d_perm, (const double *)alpha, (const double *)betta, (const double *)Q, (double *)R.d_src);
+        N, R.G, R.SW, c->d_perm, (const double *)alpha, (const double *)betta, (const double *)Q,
+        (const double *)R.d_wt, (double *)R.d_src);
   else if (R.prec == RRHD_RAD_MIXED)  // float arrays, double records
     k_dyn_from_arrays<double, float><<<grid_for(N, 256), 256, 0, c->stream>>>(
-        N, R.G, R.SW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q, (double *)R.d_src);
+        N, R.G, R.SW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q,
+        (const double *)R.d_wt, (double *)R.d_src);
   else
     k_dyn_from_arrays<float, float><<<grid_for(N, 256), 256, 0, c->stream>>>(
-        N, R.G, R.SW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q, (float *)R.d_src);
+        N, R.G, R.SW, c->d_perm, (const float *)alpha, (const float *)betta, (const float *)Q,
+        (const float *)R.d_wt, (float *)R.d_src);
   RRHD_CUDA(cudaGetLastError());
   return run_sweep_rows(c, S, I);
 }
@@ -1878,11 +1922,13 @@ extern "C" rrhd_status rrhd_coupled_step(rrhd_ctx *c, double tau, const rrhd_cou
   const Emission em{o->emission.temp_coef, o->emission.sigma_sb, o->emission.pi, o->emission.rad_unit};
   // 2. opacities and emission from the new primitives
   if (rec64)
-    k_dyn_from_state<double><<<grid_for(N, 256), 256, 0, st>>>(N, R.G, 4, state, o->absorption, o->scattering,
-                                                                em, (double *)R.d_src);
+    k_dyn_from_state<double><<<grid_for(N, 256), 256, 0, st>>>(N, R.G, source_words<double>(R.G, true), state,
+                                                                o->absorption, o->scattering, em,
+                                                                (const double *)R.d_wt, (double *)R.d_src);
   else
-    k_dyn_from_state<float><<<grid_for(N, 256), 256, 0, st>>>(N, R.G, 4, state, o->absorption, o->scattering, em,
-                                                               (float *)R.d_src);
+    k_dyn_from_state<float><<<grid_for(N, 256), 256, 0, st>>>(N, R.G, source_words<float>(R.G, true), state,
+                                                               o->absorption, o->scattering, em,
+                                                               (const float *)R.d_wt, (float *)R.d_src);
   RRHD_CUDA(cudaGetLastError());
   // 4. 4-force from the previous intensity's moments and the source con2prim, on the side
   // stream beside the sweep: they read the state after the opacities were taken from it and
