@@ -533,10 +533,12 @@ __global__ void __launch_bounds__(NT, (kResident<T, GT, HIGH, NB>)) k_sweep(cons
     }
     hi = hi2;
     hi2 = lvl[min(L + 3, depth)];
-    if constexpr (CLUSTER)
+    if constexpr (CLUSTER) {
+      __syncwarp();  // the barrier wants whole warps, whose lanes have left the loop one by one
       asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    else
+    } else {
       __syncthreads();
+    }
   }
 }
 
@@ -1008,16 +1010,40 @@ int slot_cap(const RadState &R, bool two) {  // slots a CTA's shared memory can 
   return (int)((two ? kSmemTwo : kSmemOne) / (tv * R.G));
 }
 
-// CTAs that share a direction.  Where a direction's slots fit one CTA's shared memory, one: the
-// values stay there (48^3 x 6 cells x 8, 32 and 74 directions, one group FP64: 2.1, 2.4 and 2.9
-// ms; 3.1, 3.7 and 4.6 with 8, 4 and 2 CTAs).  Where they do not, they are all in global memory
-// and few directions take as many CTAs as there are SMs for, at most the portable eight: four
-// groups 3.9, 4.8 and 6.7 ms, 5.9, 6.5 and 8.6 with one; 96^3 x 8 and 32 directions x 4 groups 13.5
-// and 23 ms, 67 and 82 with one.
-int cluster_size(const RadState &R, int64_t slots) {
+// CTAs that share a direction: a power of two up to the portable eight.
+// One where its slots take no more than half of an SM's shared memory: the values stay there (48^3 x
+// 6 cells x 8 and 16 directions, one group FP64: 2.1 and 2.2 ms; 2.5 and 2.3 with two CTAs).
+// At least two where they take more than kRoomy of it: what does not fit is read back from L2 (48^3 x 8,
+// four groups: 6.0; 3.6, 3.7 and 3.9 with 2, 4 and 8), and where it just fits, the L1 that is left holds
+// hardly a load in flight (80^3 x 4, 206 KB: 20.3; 8.0, 6.1 and 6.0; 48^3 x 1 x 4, 197 KB: 6.9, 4.7 with two;
+// 36^3 x 24 x 4, 194 KB: 2.3, 2.7 with two).
+// All slots are in global memory then and a level's barrier costs more, so each CTA gets about a
+// round of the level that the average item is in: 640 items, or 460 for four where one is not open
+// (36^3 x 8 x 3, 1,050 items: 2.2 ms with one, 2.8 with two; 64^3 x 8 x 4, 3,300: 6.9, 5.8 and 6.5 with 2, 4
+// and 8; 64^3 x 1 x 4, 1,900: 8.1, 7.5 and 7.5; 96^3 x 8, 7,000: 12.4, 8.9 and 7.8).  Near all SMs they take
+// bandwidth from one another: where one is open up to 64 of them (64^3 x 16 5.5 -> 3.7 ms with four each,
+// 64^3 x 36 6.6 -> 6.7 with two), and eight each only where that leaves half (80^3 x 18: 9.3, 6.8 with four).
+constexpr int kRoomy = 196 * 1024;
+// off: the level offsets of all directions.
+int cluster_size(const RadState &R, int64_t slots, const std::vector<int32_t> &off) {
+  if (slots <= slot_cap(R, true)) return 1;
+  const int64_t bytes = (R.prec == RRHD_RAD_FP32 ? sizeof(float) : sizeof(double)) * R.G * slots;
+  const bool roomy = bytes <= kRoomy;
+  double items = 0, squares = 0;
+  for (int d = 0; d < R.M; d++)
+    for (int L = 0; L < R.depth[d]; L++) {
+      const double n = off[R.lvl_base[d] + L + 1] - off[R.lvl_base[d] + L];
+      items += n;
+      squares += n * n;
+    }
+  const double width = squares / items;
   int cl = 1;
-  if (slots > slot_cap(R, false))
-    while (cl < 8 && 2 * cl * R.M <= kSweepSMs) cl *= 2;
+  for (int next = 2; next <= 8; next *= 2) {
+    const int most = roomy ? kSweepSMs * 7 / 16 : next == 8 ? kSweepSMs / 2 : kSweepSMs;
+    const int each = roomy || next == 8 ? 640 : next == 4 ? 460 : 0;
+    if (next * R.M > most || width < next * each) break;
+    cl = next;
+  }
   return cl;
 }
 
@@ -1508,7 +1534,7 @@ rrhd_status build_plan(rrhd_ctx *c) {
   }
   const size_t ti = R.prec == RRHD_RAD_FP64 ? sizeof(double) : sizeof(float);
   R.slots = most;
-  R.cl = cluster_size(R, most);
+  R.cl = cluster_size(R, most, off);
   R.two = R.cl == 1 && R.M > kSweepSMs && ti * R.G >= 16 && (double)beyond <= kTwoBeyond * (double)all;
   // rrhd_rad_plan_info: levels and the largest level over batches of R.DB directions
   R.levels = R.max_level = 0;

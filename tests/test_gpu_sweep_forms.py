@@ -80,6 +80,33 @@ def test_wide_slots_with_and_without_a_cluster():
     assert np.max(np.abs(few - want) / np.abs(want)) <= 1e-12
 
 
+@pytest.mark.parametrize("shape,M,G,precision,cluster", [((10, 9, 10), 8, 64, "fp64", 2), ((90, 90, 1), 2, 2, "fp64", 2),
+                                                         ((210, 210, 1), 2, 1, "fp64", 8)])
+def test_clusters_of_every_size(shape, M, G, precision, cluster):
+    m = box(*shape) if shape[2] > 1 else kuhn_box(*shape, lo=(-1, -1, 0), hi=(1, 1, 0.01), jitter=0.1, seed=33)
+    d = fibonacci_directions(M)
+    if shape[2] == 1:
+        w = np.array([[0.02, 0.01, 1.0], [0.01, -0.03, -1.0]])
+        d = Directions(w / np.linalg.norm(w, axis=1, keepdims=True), np.full(2, 2 * np.pi), 4 * np.pi)
+    inputs = inputs_of(m, M, G, precision)
+    got, form, _ = sweep(m, d, G, precision, inputs, bc=0.2)
+    assert form["cluster"] == cluster
+    want, missing = oracle.port_sweep(m, d.dirs, *inputs, bc=0.2)
+    assert missing == 0
+    assert np.max(np.abs(got - want) / np.abs(want)) <= 1e-12
+
+
+def test_cluster_of_four():
+    """Against one CTA a direction: the first directions of a larger set give the same bits alone."""
+    m, d = box(64, 64, 64), fibonacci_directions(75)
+    inputs = inputs_of(m, 75, 1, "fp64")
+    many, form, _ = sweep(m, d, 1, "fp64", inputs)
+    assert form["cluster"] == 1
+    few, form, _ = sweep(m, d.subset(0, 8), 1, "fp64", inputs[:3] + [np.ascontiguousarray(inputs[3][:, :8])])
+    assert form["cluster"] == 4
+    assert np.array_equal(many[:, :8], few)
+
+
 SPILLED = ((11, 11, 11), 75, 64)   # beyond one CTA's shared memory
 SHARED_SM = ((7, 7, 7), 149, 64)   # ... of two CTAs an SM
 CLUSTER = ((10, 9, 10), 8, 64)     # several CTAs a direction
