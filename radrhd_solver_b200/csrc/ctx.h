@@ -66,7 +66,7 @@ struct RadState {
   // the plan: per direction its N items in level order and the level offsets
   uint4 *d_ord = nullptr;     // [M][N] {cell, code word, own and upwind slots (16 bits each)}
   uint2 *d_ord_hi = nullptr;  // [M][N] upper halves of the slots, where 16 bits do not hold them
-  // geometry stream, where memory allows: [M][N][2] distances; double: [M][N][2] weights of b1 and b2, [M][N] of the out-faces
+  // geometry stream, where memory allows: [M][N][2] distances; double: [M][N][2] and [M][N] weights of the in-faces
   void *d_dist = nullptr, *d_wgt = nullptr, *d_wgt3 = nullptr;
   uint32_t *d_pos = nullptr;  // [M][N] each cell's position in sweep order, with the distances
   int32_t *d_lvl = nullptr, *d_depth = nullptr;  // level offsets of all directions; levels per direction

@@ -2,9 +2,8 @@
 
 A needle with its base up, seen from below, has three in-faces and one out-face of some 1e-6 of the
 surface; where nothing enters, the cell's value is that face's alone, and its weight has to hold all
-its digits: one minus the others' would be off by 2^-53 / 1e-6 = 1e-10.  Base triangles of all shapes, local
-face orders of all kinds and flat cells (whose out-face is the largest) go through every way of
-keeping the weights.  Bars: 1e-12 relative in double, 1e-7 (one float rounding of I) in mixed
+its digits: one minus the others' would be off by 2^-53 / 1e-6 = 1e-10.  Among the cells: base triangles of
+all shapes, local face orders of all kinds, and flat ones, whose out-face is the largest.  Bars: 1e-12 relative in double, 1e-7 (one float rounding of I) in mixed
 precision and 1e-5 in float, as in test_gpu_sweep.py."""
 import numpy as np
 import pytest
@@ -76,7 +75,7 @@ def test_small_out_faces(precision, width, bar, bc):
 @pytest.mark.parametrize("bc", [0.0, 0.25])
 @pytest.mark.parametrize("precision,bar", [("fp64", 1e-12), ("mixed", 1e-7), ("fp32", 1e-5)])
 def test_small_third_in_face(precision, bar, bc):
-    """Weights of 0.001 to 0.3, on either side of the 1/16 below which they are taken from the cell."""
+    """Weights of 0.001 to 0.3 among the in-faces."""
     corners = np.concatenate([slim(120, 0.05, 64), slim(120, 0.5, 65)])
     check(corners, directions(0.01), precision, bar, bc)
 
