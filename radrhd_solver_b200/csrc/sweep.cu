@@ -6,8 +6,8 @@
 // Here the order is built on the device once per mesh and direction set as
 // levels per direction: level 0 holds the cells whose in-faces are all on the
 // boundary, level L+1 those whose last upwind neighbour is in level L.  A sweep
-// is one kernel with one CTA per direction that walks its direction's levels,
-// one thread per cell and a CTA barrier between levels.
+// is one kernel: a CTA per direction, or a cluster of them where directions are few and their
+// fronts wide, walks its direction's levels, one thread per cell and a barrier between levels.
 //
 // One value per cell.  The reference gives every out-face the mean over its three
 // interpolation nodes of the intensity traced back from the node to the in-face it
@@ -26,12 +26,12 @@
 // A cell's outgoing value lives from its level to the last level of its downwind
 // neighbours; the plan gives it a slot for that time (a free list per direction), so a
 // direction needs about as many slots as its front is wide (9,400 on the 48^3 x 6 mesh)
-// and no face-value array exists.  Slots sit in shared memory when they fit, else in a
-// per-direction array that stays in L2.
+// and no face-value array exists.  Slots sit in shared memory when they fit, else (or where
+// a cluster shares them) in a per-direction array that stays in L2.
 //
 // What a thread reads of its item comes in sweep order: a 16-byte record (cell, face
-// choice, slots) and the two distances; by cell index it reads the source record of the
-// step and the scattering integral.
+// choice, slots) and, where memory holds them, the two distances and the weights; by cell index
+// it reads the source record of the step and the scattering integral.
 // Compiled with --fmad=false: in double precision every value is the oracle's operation
 // for operation, but for exp, exp(-4x) = exp(-x)^4 and the order of the face sums.
 #include <cuda_runtime.h>
@@ -284,7 +284,7 @@ __device__ __forceinline__ void bulk_prefetch(const P *p, uint32_t n) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b - skip), "r"((n + skip) & ~15u) : "memory");
 }
 
-// One CTA per direction.  GT: compile-time group count (1, 2 or 4; S and I in the sweep's own
+// One CTA (or cluster) per direction.  GT: compile-time group count (1, 2 or 4; S and I in the sweep's own
 // layout), 0 for any other.  HIGH: slots from a.cap on are in global memory (the others in
 // shared memory).  GEO: from the stream come 0 nothing (distances and weights from the cell's
 // records), 1 the distances (weights from the cell's sector), 2 the weights as well (double).
@@ -297,8 +297,8 @@ __device__ __forceinline__ void bulk_prefetch(const P *p, uint32_t n) {
 // uncoalesced accesses (a request every few cycles when each misses L1) decides the rest: per
 // item one 32-byte source record, and by cell also S and I.
 // Measured (whole sweep with its copies; before: one launch per level of all directions, face
-// values in HBM): 48^3 x 6 cells x 256 directions FP64, one group, 28.1 -> 5.5 ms; 12^3 x 6 x
-// 64, 269 -> 80 us; 32^3 x 256 x 4 FP64 12.6 -> 4.0 ms; 48^3 x 256 x 4 mixed 37.0 -> 10.2 ms.
+// values in HBM): 48^3 x 6 cells x 256 directions FP64, one group, 28.1 -> 5.0 ms; 12^3 x 6 x
+// 64, 269 -> 84 us; coupled step's sweep 32^3 x 256 x 4 FP64 12.6 -> 3.9 ms, 48^3 x 256 x 4 mixed 37.0 -> 10.2.
 // With every load from L1 it would take half of that: issue slots and the latency of the FP64
 // chains at 16 warps an SM, and the wait at each level's barrier.
 //
@@ -1011,22 +1011,23 @@ int slot_cap(const RadState &R, bool two) {  // slots a CTA's shared memory can 
 // CTAs that share a direction: a power of two up to the portable eight.
 // One where its slots take no more than half of an SM's shared memory: the values stay there (48^3 x
 // 6 cells x 8 and 16 directions, one group FP64: 2.1 and 2.2 ms; 2.5 and 2.3 with two CTAs).
-// At least two where they take more than kRoomy of it: what does not fit is read back from L2 (48^3 x 8,
+// Two at least where they take more than kRoomy of it: what does not fit is read back from L2 (48^3 x 8,
 // four groups: 6.0; 3.6, 3.7 and 3.9 with 2, 4 and 8), and where it just fits, the L1 that is left holds
 // hardly a load in flight (80^3 x 4, 206 KB: 20.3; 8.0, 6.1 and 6.0; 48^3 x 1 x 4, 197 KB: 6.9, 4.7 with two;
-// 36^3 x 24 x 4, 194 KB: 2.3, 2.7 with two).
+// 36^3 x 24 x 4, 194 KB: 2.3, 2.7 with two), but for levels of a few hundred items (24^3 x 64 x 8: 3.3, 3.7).
 // All slots are in global memory then and a level's barrier costs more, so each CTA gets about a
 // round of the level that the average item is in: 640 items, or 460 for four where one is not open
-// (36^3 x 8 x 3, 1,050 items: 2.2 ms with one, 2.8 with two; 64^3 x 8 x 4, 3,300: 6.9, 5.8 and 6.5 with 2, 4
-// and 8; 64^3 x 1 x 4, 1,900: 8.1, 7.5 and 7.5; 96^3 x 8, 7,000: 12.4, 8.9 and 7.8).  Near all SMs they take
-// bandwidth from one another: where one is open up to 64 of them (64^3 x 16 5.5 -> 3.7 ms with four each,
-// 64^3 x 36 6.6 -> 6.7 with two), and eight each only where that leaves half (80^3 x 18: 9.3, 6.8 with four).
+// (36^3 x 8 x 3, 1,050 items: 2.2 ms with one, 2.8 with two; 64^3 x 8 x 4, 3,300: 6.9, 5.8 and 6.5 with
+// 2, 4 and 8; 64^3 x 1 x 4, 1,900: 8.1, 7.5 and 7.5; 96^3 x 8, 7,000: 12.4, 8.9 and 7.8).  Near all SMs they
+// take bandwidth from one another: where one is open up to 64 of them (64^3 x 16 5.5 -> 3.7 ms with four
+// each, 64^3 x 36 6.6 -> 6.7 with two), and eight each only where that leaves half (80^3 x 18: 9.3, 6.8
+// with four).
 constexpr int kRoomy = 196 * 1024;
 // off: the level offsets of all directions.
 int cluster_size(const RadState &R, int64_t slots, const std::vector<int32_t> &off) {
   if (slots <= slot_cap(R, true)) return 1;
   const int64_t bytes = (R.prec == RRHD_RAD_FP32 ? sizeof(float) : sizeof(double)) * R.G * slots;
-  const bool roomy = bytes <= kRoomy;
+  const bool roomy = bytes <= kRoomy, fits = slots <= slot_cap(R, false);
   double items = 0, squares = 0;
   for (int d = 0; d < R.M; d++)
     for (int L = 0; L < R.depth[d]; L++) {
@@ -1038,7 +1039,7 @@ int cluster_size(const RadState &R, int64_t slots, const std::vector<int32_t> &o
   int cl = 1;
   for (int next = 2; next <= 8; next *= 2) {
     const int most = roomy ? kSweepSMs * 7 / 16 : next == 8 ? kSweepSMs / 2 : kSweepSMs;
-    const int each = roomy || next == 8 ? 640 : next == 4 ? 460 : 0;
+    const int each = roomy || next == 8 ? 640 : next == 4 ? 460 : fits ? 400 : 0;
     if (next * R.M > most || width < next * each) break;
     cl = next;
   }
@@ -1102,10 +1103,11 @@ cudaError_t launch_sweep_groups(const SweepArgs<T, TI> &a, int64_t low, bool two
     return launch_sweep_geo<T, TI, GT, false, false, 256, 2>(a, nd, smem, st);
   }
   if constexpr (sizeof(T) == 4 && GT == 2) {
-    // The same with two groups, at a cost (64 registers of 77), so where it fills SMs twice and L2 holds
-    // the lines of twice as many fronts: 14^3 x 256 x 2 0.49 -> 0.33 ms, 36^3 3.05 -> 2.6, but 48^3 6.5 ->
-    // 10.6, 24^3 x 100 0.78 -> 0.82.
-    if (!a.nhigh && nd > kSweepSMs && 2 * smem <= kSmemOne && low * 128 * std::min(nd, 2 * kSweepSMs) <= (int64_t)320 << 20)
+    // The same with two groups, at a cost (64 registers of 77), so where it fills SMs twice and the
+    // lines of twice as many fronts are few times what L2 holds: 14^3 x 256 x 2 0.49 -> 0.33 ms, 40^3
+    // 4.0 -> 3.7, but 44^3 (360 MB) 5.1 -> 6.9, 48^3 6.5 -> 10.6, and 24^3 x 100 0.78 -> 0.82.
+    if (!a.nhigh && nd > kSweepSMs && 2 * smem <= kSmemOne &&
+        low * 128 * std::min(nd, 2 * kSweepSMs) <= (int64_t)320 << 20)
       return launch_sweep_geo<T, TI, GT, false, false, 512, 2>(a, nd, smem, st);
   }
   if (a.ord_hi) return launch_sweep_geo<T, TI, GT, true, true, 512, 1>(a, nd, smem, st);
@@ -1170,8 +1172,8 @@ bool by_position(const RadState &R) {
 template <class TI, class V, bool IMPORT>
 cudaError_t launch_tile(rrhd_ctx *c, int gw, int d0, int nd, const int32_t *perm, const void *in, void *out) {
   const dim3 tiles((unsigned)((c->N * gw + 31) / 32), (unsigned)((nd + kTileDirs<V> - 1) / kTileDirs<V>));
-  k_tile<V, IMPORT><<<tiles, 256, 0, c->stream>>>(c->N, gw, c->rad.M, d0, nd, perm, by_position<TI>(c->rad) ? c->rad.d_pos : nullptr, (const V *)in,
-                                                  (V *)out);
+  const uint32_t *pos = by_position<TI>(c->rad) ? c->rad.d_pos : nullptr;
+  k_tile<V, IMPORT><<<tiles, 256, 0, c->stream>>>(c->N, gw, c->rad.M, d0, nd, perm, pos, (const V *)in, (V *)out);
   return cudaGetLastError();
 }
 
