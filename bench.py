@@ -523,7 +523,8 @@ def coupled_component(dev, m, W, steps=100, warm=1, M=256, G=4, train_epochs=2, 
         if form == "plain":
             states["plain_dump"] = (Wg, Ug)
         bio = 8 if fp64 else 4  # bytes per intensity / scattering value
-        # S in, I out, an item's 16-byte record; the outgoing values stay on chip
+        # what any such sweep moves: S in, I out and an item's 16-byte record, once each (this one also moves
+        # 44 bytes of geometry an item, S and I twice more between layouts, and the values that do not fit on chip)
         sweep_alg = (2.0 * bio * G + 16.0) * m.n_cells * M + m.n_cells * 32.0
         out[form] = {"dirs_per_batch": batch[0] if fp64 else batch[1], "item_geometry": geo, "ms_per_step": ms, "steps_per_s": 1e3 / ms, "cell_updates_per_s": m.n_cells / (ms / 1e3),
                      "cell_dir_group_per_s": m.n_cells * M * G / (ms / 1e3), "phase_ms_last_step": ph,
@@ -581,7 +582,7 @@ def sweep_component(dev, nhex=32, M=256, G=4, reps=3, precisions=("fp64", "fp32"
         ms = _time(lambda: illum.CalculateIllum(sw, alpha, betta, Q, S, I), reps, stream, warm=1)
         levels, biggest = sw.plan_info()
         bpv = 8 if prec == "fp64" else 4
-        alg = (2.0 * G * bpv + 16.0) * m.n_cells * M + m.n_cells * 32.0
+        alg = (2.0 * G * bpv + 16.0) * m.n_cells * M + m.n_cells * 32.0  # as in coupled_component
         out[prec] = {"ms": ms, "cell_dir_per_s": m.n_cells * M / (ms / 1e3), "levels": levels,
                      "largest_level": biggest, "plan_build_s": t_plan, "alg_gbs": alg / (ms / 1e3) / 1e9}
         del alpha, betta, Q, S, I

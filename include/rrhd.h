@@ -481,15 +481,15 @@ rrhd_status rrhd_rad_source(const rrhd_emission *em, const double *W, const doub
  * (illum_utils.cpp:377-433), area-weighted face mean (plain mean for the last
  * cell).  The upwind order (the reference's sorted_graph, made offline by its
  * graph/ and make_trace/ tools) is built on the device at setup as levels of
- * cells whose upwind neighbours are all done; a sweep is one kernel, one CTA per
- * direction, that walks the levels of its direction. */
+ * cells whose upwind neighbours are all done; a sweep is one kernel in which a CTA,
+ * or a cluster of them, walks the levels of each direction. */
 #define RRHD_RAD_FP64 0  /* sweep arithmetic and storage in double */
 #define RRHD_RAD_FP32 1  /* in float (input of the tensor-core scattering) */
-#define RRHD_RAD_MIXED 2 /* the sweep in double (geometry, records, face values, arithmetic)
+#define RRHD_RAD_MIXED 2 /* the sweep in double (geometry, records, outgoing values, arithmetic)
                             with the scattering integral S read and the intensity I written
                             in float, the tensor-core scattering's input and output: the
                             intensity is the double sweep's rounded once.  Caller arrays
-                            (rrhd_sweep) are float.  Storing the face values in float lets
+                            (rrhd_sweep) are float.  Keeping outgoing values in float lets
                             the rounding accumulate along each characteristic; rounding the
                             geometry to float moves the attenuation of faces at grazing
                             incidence and the choice between nearly equally distant

@@ -338,7 +338,7 @@ __global__ void k_get_state(int64_t N, double *W, int64_t sw, double *U, int64_t
 
 // Both arrays packed ([N][5]): a CTA moves 128 cells through shared memory, so that the caller's
 // side moves whole lines and a cell's 80 bytes are five 16-byte accesses of neighbouring threads
-// (one thread a cell strode 40 and 80 bytes): 1,572,864 cells, set 152 -> 60 us, get 88 -> 60 us.
+// (one thread a cell strode 40 and 80 bytes): 1,572,864 cells, set 152 -> 55 us, get 88 -> 60 us.
 // Bound: HBM (320 B a cell).
 constexpr int kStateCells = 128;
 template <bool SET>

@@ -199,7 +199,7 @@ class TransportSweep:
     upwind order the reference reads from its offline graph/ and make_trace/
     outputs (sorted_graph, vec_x0), built on the GPU as levels.  precision:
     "fp64" or "fp32" (storage and arithmetic of alpha, betta, Q, S, I), or "mixed"
-    (float arrays as "fp32", face values and the transport update in double).
+    (float arrays as "fp32", outgoing values and the transport update in double).
     dirs_per_batch: directions whose levels plan_info counts together.  item_geometry
     ("fp32" and "mixed" only): accepted; every sweep keeps its items' geometry in sweep
     order where device memory holds it (limit_sweep_memory)."""
