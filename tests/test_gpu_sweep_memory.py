@@ -114,3 +114,31 @@ def test_transfers_in_pieces(mesh, precision, G):
     torch.cuda.empty_cache()
     assert np.array_equal(c.step.get("S"), values[1])
     c.close()
+
+
+@pytest.mark.parametrize("G,megabytes,dirs", [(4, 60, M), (8, 20, M // 2)])
+def test_scratch_takes_the_streams_memory(mesh, G, megabytes, dirs):
+    """A sweep after a coupled step, which has taken the scratch: it is made again from the stream's memory, of
+    all directions (4 groups: 201 MB against 60 free and 151 of weights) or of half of them (8 groups: 402 MB,
+    20 free, 277 of weights and stream)."""
+    rows, n = mesh.n_cells * G, mesh.n_cells
+    gen = torch.Generator("cuda").manual_seed(55)
+    rand = lambda *s: torch.rand(*s, generator=gen, device="cuda", dtype=torch.float64)
+    x = [rand(n) + 0.1, rand(n), rand(n, G), rand(rows, M)]
+    torch.cuda.synchronize()
+    fresh = Context(mesh, G)
+    want = illum.CalculateIllum(fresh.sw, *x)
+    fresh.grid.sync()
+    fresh.close()
+    c = Context(mesh, G)
+    c.steps()
+    assert c.sw.plan_form()["scratch_dirs"] == 0 and c.sw.plan_form()["stream"] == 2
+    I = torch.empty_like(x[3])
+    held = leave(megabytes)
+    illum.CalculateIllum(c.sw, *x, I)
+    c.grid.sync()
+    assert c.sw.plan_form()["scratch_dirs"] == dirs and c.sw.plan_form()["stream"] < 2
+    del held
+    torch.cuda.empty_cache()
+    assert torch.equal(I, want)
+    c.close()
