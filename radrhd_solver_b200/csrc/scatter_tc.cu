@@ -623,10 +623,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             float4 v = make_float4(run[4 * j] * inv, run[4 * j + 1] * inv, run[4 * j + 2] * inv,
                                    run[4 * j + 3] * inv);
             if (SCALED && col < nS) {
-              v.x = add_iso(v.x, iso_hi, iso_lo);
-              v.y = add_iso(v.y, iso_hi, iso_lo);
-              v.z = add_iso(v.z, iso_hi, iso_lo);
-              v.w = add_iso(v.w, iso_hi, iso_lo);
+              add_iso2(v.x, v.y, iso_hi, iso_lo);
+              add_iso2(v.z, v.w, iso_hi, iso_lo);
             }
             if (col < nS) {
               if constexpr (NG > 1) {
@@ -1111,7 +1109,7 @@ __global__ void __launch_bounds__(R_THREADS, 1)
             float v[4] = {run[4 * j] * inv, run[4 * j + 1] * inv, run[4 * j + 2] * inv, run[4 * j + 3] * inv};
             if (SCALED && col < nS) {
 #pragma unroll
-              for (int i = 0; i < 4; i++) v[i] = add_iso(v[i], iso_hi, iso_lo);
+              for (int i = 0; i < 4; i += 2) add_iso2(v[i], v[i + 1], iso_hi, iso_lo);
             }
             if (col < nS) {
               if constexpr (NG == 4) {
